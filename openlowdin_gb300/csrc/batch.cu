@@ -243,15 +243,19 @@ struct LowdinGB300_Batch {
       drop_graphs();
       tasks_dirty = false;
     }
-    if (!use_graph || calls++ == 0) return fock_sequence(precision, split, s);
+    if (!use_graph || calls++ == 0) {
+      Lanes lanes(s);
+      return fock_sequence(precision, split, s, lanes);
+    }
     Graph &g = graphs[precision & 3];
     if (!g.exec || g.split != split || g.skip != skip) {
       if (g.exec) cudaGraphExecDestroy(g.exec);
       g = Graph{};
       if (!capture) CK(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking));
       const long long l0 = launch_count();
+      Lanes lanes(capture, true);   // held until the capture has ended
       CK(cudaStreamBeginCapture(capture, cudaStreamCaptureModeThreadLocal));
-      const bool ok = fock_sequence(precision, split, capture);
+      const bool ok = fock_sequence(precision, split, capture, lanes);
       cudaGraph_t graph = nullptr;
       const cudaError_t e = cudaStreamEndCapture(capture, &graph);
       const long long captured = launch_count() - l0;
@@ -356,7 +360,7 @@ struct LowdinGB300_Batch {
   }
 
   // every launch of one build, in stream order
-  bool fock_sequence(int precision, double split, cudaStream_t s) {
+  bool fock_sequence(int precision, double split, cudaStream_t s, Lanes &lanes) {
     CK(cudaMemsetAsync(Dn.p, 0, Dn.n * sizeof(double), s));
     CK(cudaMemsetAsync(Dn32.p, 0, Dn32.n * sizeof(float), s));
     CK(cudaMemsetAsync(cnt.p, 0, 2 * kNQC * sizeof(unsigned long long), s));
@@ -367,10 +371,11 @@ struct LowdinGB300_Batch {
       CK(launch_dn_max_batch(slots.p, nslots, max_nsh, s));
     }
     if (jk_mixed && npslots) CK(launch_pair_gather(pslots.p, npslots, ptotal, s));
-    if (!LibintInterface::launch_jk_groups(jk, jk_mixed, jk_mixed ? split : 0.0, boys, s, skip, rows_choice))
+    if (!LibintInterface::launch_jk_groups(jk, jk_mixed, jk_mixed ? split : 0.0, boys, s, skip, rows_choice,
+                                           -1, false, &lanes))
       return false;
     if (jk_mixed && npslots) CK(launch_pair_scatter(pslots.p, npslots, ptotal, s));
-    if (!launch_cp_groups(cp, (precision & 2) ? 2 : 0, split, boys, s, skip)) return false;
+    if (!launch_cp_groups(cp, (precision & 2) ? 2 : 0, split, boys, s, skip, &lanes)) return false;
     CK(launch_finalize_batch(slots.p, nslots, total, s));
     return true;
   }

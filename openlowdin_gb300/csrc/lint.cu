@@ -26,6 +26,109 @@ void set_error(const char *fmt, ...) {
   if (strict && strict[0] == '1') abort();
 }
 
+// ------------------------------------------------------------------ lanes --
+// Seven side streams and the caller's own: a build has 6 (s, p) to 21 (s, p,
+// d) class launches, and each further lane costs the host a wait, a record and
+// another wait.  Measured, one stream -> lanes: one water (34 functions, 6
+// launches of 6-170 CTAs) 192 -> 116 us; four waters with d (21 launches, the
+// eight cooperative ones of 16-264 CTAs) 3.88 -> 1.43 ms; electron-proton
+// coupling of six waters 504 -> 380 us; a 387-function chain, whose launches
+// fill the GPU by themselves, 41.7 -> 41.6 ms.
+constexpr int kSideLanes = 7;
+constexpr size_t kLanePool = 16;   // sets kept per process; a set above it is destroyed when given back
+
+struct LaneSet {
+  int device = -1;
+  cudaStream_t s[kSideLanes] = {};
+  cudaEvent_t fork = nullptr, done[kSideLanes] = {};
+  bool create() {
+    CK(cudaGetDevice(&device));
+    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    for (int k = 0; k < kSideLanes; ++k) {
+      CK(cudaStreamCreateWithFlags(&s[k], cudaStreamNonBlocking));
+      CK(cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming));
+    }
+    return true;
+  }
+  ~LaneSet() {
+    for (int k = 0; k < kSideLanes; ++k) {
+      if (s[k]) cudaStreamDestroy(s[k]);
+      if (done[k]) cudaEventDestroy(done[k]);
+    }
+    if (fork) cudaEventDestroy(fork);
+  }
+};
+
+namespace {
+std::mutex g_lane_mu;
+std::vector<LaneSet *> g_lane_free;
+}  // namespace
+
+Lanes::Lanes(cudaStream_t s, bool captured) {
+  if (!captured) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+      cudaGetLastError();   // the legacy stream beside another stream's capture: stay on s
+      return;
+    }
+    if (st != cudaStreamCaptureStatusNone) return;
+  }
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  {
+    std::lock_guard<std::mutex> lk(g_lane_mu);
+    for (size_t k = g_lane_free.size(); k-- > 0;)
+      if (g_lane_free[k]->device == dev) {
+        set_ = g_lane_free[k];
+        g_lane_free.erase(g_lane_free.begin() + k);
+        return;
+      }
+  }
+  LaneSet *n = new LaneSet();
+  if (n->create()) set_ = n;
+  else delete n;
+}
+
+Lanes::~Lanes() {
+  if (!set_) return;
+  {
+    std::lock_guard<std::mutex> lk(g_lane_mu);
+    if (g_lane_free.size() < kLanePool) {
+      g_lane_free.push_back(set_);
+      return;
+    }
+  }
+  delete set_;
+}
+
+bool Lanes::run(std::vector<Job> &jobs, cudaStream_t s) {
+  std::stable_sort(jobs.begin(), jobs.end(), [](const Job &a, const Job &b) { return a.cost > b.cost; });
+  const int lanes = set_ ? (int)std::min<size_t>(jobs.size(), kSideLanes + 1) : 1;
+  if (lanes > 1) CK(cudaEventRecord(set_->fork, s));
+  double load[kSideLanes + 1] = {};
+  bool used[kSideLanes + 1] = {};
+  cudaError_t err = cudaSuccess;
+  for (Job &j : jobs) {
+    const int k = (int)(std::min_element(load, load + lanes) - load);   // lane 0 is s itself
+    cudaStream_t q = k ? set_->s[k - 1] : s;
+    if (k && !used[k]) err = cudaStreamWaitEvent(q, set_->fork, 0);
+    used[k] = true;
+    load[k] += j.cost;
+    if (err == cudaSuccess) err = j.launch(q);
+    if (err != cudaSuccess) break;
+  }
+  // the lanes are joined also after a failed launch: s then still ends behind
+  // whatever was queued
+  for (int k = 1; k < lanes; ++k)
+    if (used[k]) {
+      cudaError_t e = cudaEventRecord(set_->done[k - 1], set_->s[k - 1]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(s, set_->done[k - 1], 0);
+      if (err == cudaSuccess) err = e;
+    }
+  CK(err);
+  return true;
+}
+
 // ------------------------------------------------------------- Boys table --
 // F_n(T_i), T_i = i h, from the series F_n(T) = e^{-T} sum_k (2T)^k /
 // ((2n+1)(2n+3)...(2n+2k+1)) in long double.
@@ -327,7 +430,8 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
 
 // mode 0: FP64, 1: FP32 throughout, 2: split at `split` (FP64 above, FP32 below)
 bool launch_cp_groups(const TaskSet<CPTask> &ts, int mode, double split, BoysTables boys, cudaStream_t s,
-                      double skip) {
+                      double skip, Lanes *lanes) {
+  std::vector<Lanes::Job> jobs;
   for (int c = 0; c < kNQC; ++c) {
     if (!ts.cnt[c]) continue;
     TaskLaunch tl{};
@@ -337,22 +441,22 @@ bool launch_cp_groups(const TaskSet<CPTask> &ts, int mode, double split, BoysTab
     tl.cut = 1e-10;
     tl.skip = (float)skip;
     tl.boys = boys;
+    tl.split = mode == 2 ? split : 0.0;
+    set_fp32_copies(tl);
     const int cb = c / kNumPairClasses, ck = c % kNumPairClasses;
-    if (mode == 2) {
-      tl.split = split;
-      set_fp32_copies(tl);
-      tl.lower = 0;
-      CK(launch_cp_tasks(cb, ck, false, ts.d + ts.off[c], tl, s));
-      tl.lower = 1;
-      CK(launch_cp_tasks(cb, ck, true, ts.d + ts.off[c], tl, s));
-    } else {
-      set_fp32_copies(tl);
-      CK(launch_cp_tasks(cb, ck, mode == 1, ts.d + ts.off[c], tl, s));
-    }
+    const CPTask *d = ts.d + ts.off[c];
+    auto add = [&](bool fp32) {
+      if (!lanes) return launch_cp_tasks(cb, ck, fp32, d, tl, s);
+      jobs.push_back({launch_cost(cb, ck, tl.nblocks), [=](cudaStream_t q) { return launch_cp_tasks(cb, ck, fp32, d, tl, q); }});
+      return cudaSuccess;
+    };
+    tl.lower = 0;
+    CK(add(mode == 1));
+    tl.lower = 1;
+    if (mode == 2) CK(add(true));
   }
-  return true;
+  return !lanes || lanes->run(jobs, s);
 }
-
 
 bool coupling(LibintInterface *A, LibintInterface *B, const double *dDa, const double *dDb, double *dJa,
               double *dJb, bool fp32, cudaStream_t s) {
@@ -379,7 +483,10 @@ bool coupling(LibintInterface *A, LibintInterface *B, const double *dDa, const d
   SpeciesBufs bb{B->dDsC.p, B->dDsC32.p, nullptr, nullptr, B->dJacc.p, B->dJacc32.p};
   if (!add_cp_tasks(A->cp, A, B, ba, bb, dJa != nullptr, dJb != nullptr, 1.0)) return false;
   if (!A->cp.upload(s)) return false;
-  if (!launch_cp_groups(A->cp, fp32 ? 1 : 0, 0.0, A->boys, s)) return false;
+  {
+    Lanes lanes(s);
+    if (!launch_cp_groups(A->cp, fp32 ? 1 : 0, 0.0, A->boys, s, 0.0, &lanes)) return false;
+  }
   if (dJa) CK(launch_coupling_extract(A->dJacc.p, A->dJacc32.p, A->d_norma, nA, 1.0, 0, dJa, s));
   if (dJb) CK(launch_coupling_extract(B->dJacc.p, B->dJacc32.p, B->d_norma, nB, 1.0, 0, dJb, s));
   return true;
@@ -413,6 +520,11 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
   q.cut = 1e-10;
   q.eps = DBL_EPSILON;
   q.nsh = nsh;
+  std::vector<Lanes::Job> jobs;
+  auto add = [&](int cb, int ck) {
+    const ITParams p = q;
+    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), [=](cudaStream_t z) { return launch_it(cb, ck, p, z); }});
+  };
   if (intra) {
     if (!A->dD.ensure((size_t)nA * nA) || !A->dDs.ensure((size_t)nA * nA) || !A->dDn.ensure((size_t)nsh * nsh))
       return false;
@@ -435,7 +547,7 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
         q.ket0 = A->sig.start[ck];
         q.nket = A->sig.count(ck);
         q.triangle = cb == ck;
-        CK(launch_it(cb, ck, q, s));
+        add(cb, ck);
       }
   } else {
     q.screen = 0;
@@ -455,8 +567,12 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
         q.ket0 = B->all.start[ck];
         q.nket = B->all.count(ck);
         q.triangle = 0;
-        CK(launch_it(cb, ck, q, s));
+        add(cb, ck);
       }
+  }
+  {
+    Lanes lanes(s);
+    if (!lanes.run(jobs, s)) return false;
   }
   CK(launch_scale_cube(A->dA.p, A->d_norma, K->d_norma, nA, nB, s));
   CK(cudaMemcpyAsync(hOut, A->dA.p, cube * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -500,6 +616,11 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
   G12Params P{};
   P.gem = A->dGem.p;
   P.n = n;
+  std::vector<Lanes::Job> jobs;
+  auto add = [&](int cb, int ck) {
+    const G12Params p = P;
+    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket), [=](cudaStream_t z) { return launch_g12(cb, ck, p, z); }});
+  };
   if (!B) {
     CK(launch_scale_density(dD, A->d_norma, n, A->dDs.p, A->dDs32.p, s));
     CK(cudaMemsetAsync(A->dGacc.p, 0, sizeof(double) * n * n, s));
@@ -517,8 +638,12 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
         P.ket0 = A->sig.start[ck];
         P.nket = A->sig.count(ck);
         P.triangle = cb == ck;
-        CK(launch_g12(cb, ck, P, s));
+        add(cb, ck);
       }
+    {
+      Lanes lanes(s);
+      if (!lanes.run(jobs, s)) return false;
+    }
     CK(launch_symmetrize(A->dGacc.p, nullptr, A->d_norma, n, 0.25, dOut, s));
     return true;
   }
@@ -541,8 +666,12 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
       P.nbra = A->all.count(cb);
       P.ket0 = B->all.start[ck];
       P.nket = B->all.count(ck);
-      CK(launch_g12(cb, ck, P, s));
+      add(cb, ck);
     }
+  {
+    Lanes lanes(s);
+    if (!lanes.run(jobs, s)) return false;
+  }
   CK(launch_coupling_extract(A->dJacc.p, nullptr, A->d_norma, n, 1.0, 1, dOut, s));
   return true;
 }

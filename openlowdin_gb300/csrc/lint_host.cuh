@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -162,6 +163,42 @@ struct DevBuf {
 };
 
 constexpr int kNQC = kNumPairClasses * kNumPairClasses;
+
+// Relative cost of a class launch: its blocks times the integrals and
+// recursion nodes of a quartet.  Only the order of launches depends on it.
+inline double launch_cost(int cb, int ck, double blocks) {
+  const int L = pc_L(cb) + pc_L(ck);
+  return (blocks + 300.0) * ncart(pc_la(cb)) * ncart(pc_lb(cb)) * ncart(pc_la(ck)) * ncart(pc_lb(ck)) * (L + 1);
+}
+// Streams for the quartet-class launches of one build.  The classes of a build
+// only add into the same accumulators, so they need no order among
+// themselves; on one stream each of them waits for the last block of the one
+// before.  A lease takes a set of side streams from a bounded per-device pool
+// and gives it back when it goes out of scope; a set is only ever used by one
+// lease at a time, and work left on its streams merely orders the next user's
+// launches behind it.
+struct LaneSet;
+class Lanes {
+ public:
+  // side streams for launches forked from `s`.  None when s is being captured
+  // (a set given back before the capture ends would carry another caller's
+  // launches into the graph), unless `captured`: the caller holds the lease
+  // until its own capture has ended.
+  explicit Lanes(cudaStream_t s, bool captured = false);
+  ~Lanes();
+  Lanes(const Lanes &) = delete;
+  Lanes &operator=(const Lanes &) = delete;
+  // runs the queued launches: costliest first, each on the lane with the
+  // least work so far, every lane ordered behind `s` and s behind every lane
+  struct Job {
+    double cost;
+    std::function<cudaError_t(cudaStream_t)> launch;
+  };
+  bool run(std::vector<Job> &jobs, cudaStream_t s);
+
+ private:
+  LaneSet *set_ = nullptr;
+};
 
 // device buffers of one species in one build: scaled density (FP64 + FP32),
 // shell-block norms (FP64 + FP32) and the output accumulators (FP64 + FP32)
@@ -541,7 +578,10 @@ struct LibintInterface {
     CK(cudaMemsetAsync(dGacc32.p, 0, sizeof(float) * n * n, s));
     CK(cudaMemsetAsync(dcount.p, 0, sizeof(unsigned long long) * kNQC, s));
     if (precision != 0) CK(launch_pair_gather(dpslot.p, 1, (long long)sig.h.size(), s));
-    if (!launch_jk_groups(jk, precision, split, boys, s)) return false;
+    {
+      Lanes lanes(s);
+      if (!launch_jk_groups(jk, precision, split, boys, s, 0.0, nullptr, -1, false, &lanes)) return false;
+    }
     if (precision != 0) CK(launch_pair_scatter(dpslot.p, 1, (long long)sig.h.size(), s));
     CK(launch_symmetrize(dGacc.p, dGacc32.p, d_norma, n, 0.25, dGout, s));
     // the quartet counts travel with the result; they are summed when asked for
@@ -616,10 +656,12 @@ struct LibintInterface {
 
   // rows: per quartet class the FP32 kernel of mixed launches (-1 size rule,
   // 0 jk_tasks_kernel, 1 bra-row kernel; null: size rule); only: a single
-  // class (-1: all) and, with lower_only, only its FP32 launch (autotuning)
+  // class (-1: all) and, with lower_only, only its FP32 launch (autotuning);
+  // lanes: side streams for the launches (null: all on s, in class order)
   static bool launch_jk_groups(const TaskSet<JKTask> &ts, int precision, double split, BoysTables boys,
                                cudaStream_t s, double skip = 0.0, const signed char *rows = nullptr,
-                               int only = -1, bool lower_only = false) {
+                               int only = -1, bool lower_only = false, Lanes *lanes = nullptr) {
+    std::vector<Lanes::Job> jobs;
     for (int c = 0; c < kNQC; ++c) {
       if (!ts.cnt[c] || (only >= 0 && c != only)) continue;
       TaskLaunch tl{};
@@ -634,20 +676,22 @@ struct LibintInterface {
       tl.skip = (float)skip;
       tl.boys = boys;
       const int cb = c / kNumPairClasses, ck = c % kNumPairClasses;
-      if (precision == 0) {
-        tl.split = 0.0;
-        set_fp32_copies(tl);
-        CK(launch_jk_tasks(cb, ck, false, ts.d + ts.off[c], tl, s));
-      } else {
-        tl.split = split;
-        set_fp32_copies(tl);
-        tl.lower = 0;
-        if (!lower_only) CK(launch_jk_tasks(cb, ck, false, ts.d + ts.off[c], tl, s));
-        tl.lower = 1;
-        CK(launch_jk_tasks(cb, ck, true, ts.d + ts.off[c], tl, s));
-      }
+      const JKTask *d = ts.d + ts.off[c];
+      tl.split = precision == 0 ? 0.0 : split;
+      set_fp32_copies(tl);
+      auto add = [&](bool fp32) {
+        if (lanes)
+          jobs.push_back({launch_cost(cb, ck, tl.nblocks), [=](cudaStream_t q) { return launch_jk_tasks(cb, ck, fp32, d, tl, q); }});
+        else
+          return launch_jk_tasks(cb, ck, fp32, d, tl, s);
+        return cudaSuccess;
+      };
+      tl.lower = 0;
+      if (!lower_only) CK(add(false));
+      tl.lower = 1;
+      if (precision != 0) CK(add(true));
     }
-    return true;
+    return !lanes || lanes->run(jobs, s);
   }
 };
 
@@ -659,7 +703,7 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
                   unsigned long long *counters = nullptr);
 // mode 0: FP64, 1: FP32 throughout, 2: split at `split` (FP64 above, FP32 below)
 bool launch_cp_groups(const TaskSet<CPTask> &ts, int mode, double split, BoysTables boys, cudaStream_t s,
-                      double skip = 0.0);
+                      double skip = 0.0, Lanes *lanes = nullptr);
 bool coupling(LibintInterface *A, LibintInterface *B, const double *dDa, const double *dDb, double *dJa,
               double *dJb, bool fp32, cudaStream_t s);
 bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, const double *hC, int p,

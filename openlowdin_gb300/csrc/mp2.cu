@@ -98,6 +98,7 @@ void mp2_columns(const PairList &P, long long colB, MP2Columns &mc) {
 
 // integrals of every bra pair of PA against the ket pairs [k0, k1) of PB
 bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, int k1, cudaStream_t s) {
+  std::vector<Lanes::Job> jobs;
   for (int ck = 0; ck < kNumPairClasses; ++ck) {
     const int ka = std::max(k0, PB.start[ck]), kb = std::min(k1, PB.start[ck + 1]);
     if (ka >= kb) continue;
@@ -107,10 +108,13 @@ bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, 
         q.nbra = std::min(PA.start[cb + 1] - b0, 65535 * kWarpsPerBlock);
         q.ket0 = ka;
         q.nket = kb - ka;
-        CK(launch_mp2x(cb, ck, q, s));
+        const MXParams p = q;
+        jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128),
+                        [=](cudaStream_t z) { return launch_mp2x(cb, ck, p, z); }});
       }
   }
-  return true;
+  Lanes lanes(s);
+  return lanes.run(jobs, s);
 }
 
 // Writer of the reference's transformed-integral file `<species>moint.dat`
