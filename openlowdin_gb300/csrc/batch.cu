@@ -28,6 +28,7 @@ struct LowdinGB300_Batch {
   bool finalized = false;
   DevBuf<double> Ds, Dn, Gacc, Jacc;
   DevBuf<float> Ds32, Dn32, Gacc32, Jacc32;
+  DevBuf<float2> Dd;
   DevBuf<unsigned long long> cnt;
   DevBuf<SpeciesSlot> slots;
   // pair-indexed arrays of the FP32 row kernels, one PairSlot per two-body species
@@ -77,6 +78,7 @@ struct LowdinGB300_Batch {
     Ds.release(); Dn.release(); Gacc.release(); Jacc.release(); cnt.release(); slots.release();
     Dp32.release(); Jp32.release(); DnP32.release(); pslots.release();
     Ds32.release(); Dn32.release(); Gacc32.release(); Jacc32.release();
+    Dd.release();
     active.release();
     jk.release(); cp.release();
   }
@@ -115,7 +117,8 @@ struct LowdinGB300_Batch {
     total = tot;
     const long long dsz = dtot > 0 ? dtot : 1;
     if (!Ds.ensure(tot) || !Gacc.ensure(tot) || !Jacc.ensure(tot) || !Dn.ensure(dsz) || !Ds32.ensure(tot) ||
-        !Gacc32.ensure(tot) || !Jacc32.ensure(tot) || !Dn32.ensure(dsz) || !cnt.ensure(2 * kNQC))
+        !Gacc32.ensure(tot) || !Jacc32.ensure(tot) || !Dn32.ensure(dsz) || !cnt.ensure(2 * kNQC) ||
+        !Dd.ensure(tot))
       return false;
     // pair-indexed arenas of the two-body species
     std::vector<long long> peoff(sp.size(), -1), pairoff(sp.size(), -1);
@@ -162,6 +165,7 @@ struct LowdinGB300_Batch {
       S.P = x.P;
       S.Ds = Ds.p + off[k];
       S.Ds32 = Ds32.p + off[k];
+      S.Dd = Dd.p + off[k];
       S.Dn = dnoff[k] >= 0 ? Dn.p + dnoff[k] : nullptr;
       S.Dn32 = dnoff[k] >= 0 ? Dn32.p + dnoff[k] : nullptr;
       S.norma = x.h->d_norma;
@@ -182,7 +186,7 @@ struct LowdinGB300_Batch {
       if (x.two_body) {
         // non-electron species are not screened: their norm pointers are never read
         SpeciesBufs b{S.Ds, S.Ds32, S.Dn ? S.Dn : Dn.p, S.Dn32 ? S.Dn32 : Dn32.p, S.Gacc, S.Gacc32,
-                      Dp32.p + peoff[k], Jp32.p + peoff[k], DnP32.p + pairoff[k], S.Dnmax32};
+                      Dp32.p + peoff[k], Jp32.p + peoff[k], DnP32.p + pairoff[k], S.Dnmax32, S.Dd};
         const auto before = sizes(jk);
         if (!x.h->add_jk_tasks(jk, b, 0.5 * x.factor, cnt.p)) return false;
         mark(jk, before, x.sys);
@@ -366,10 +370,8 @@ struct LowdinGB300_Batch {
     CK(cudaMemsetAsync(cnt.p, 0, 2 * kNQC * sizeof(unsigned long long), s));
     CK(launch_prepare_batch(slots.p, nslots, total, s));
     const int jk_mixed = precision & 1;
-    if (jk_mixed) {
-      CK(cudaMemsetAsync(Dnmax32.p, 0, Dnmax32.n * sizeof(float), s));
-      CK(launch_dn_max_batch(slots.p, nslots, max_nsh, s));
-    }
+    CK(cudaMemsetAsync(Dnmax32.p, 0, Dnmax32.n * sizeof(float), s));
+    CK(launch_dn_max_batch(slots.p, nslots, max_nsh, s));
     if (jk_mixed && npslots) CK(launch_pair_gather(pslots.p, npslots, ptotal, s));
     if (!LibintInterface::launch_jk_groups(jk, jk_mixed, jk_mixed ? split : 0.0, boys, s, skip, rows_choice,
                                            -1, false, &lanes))

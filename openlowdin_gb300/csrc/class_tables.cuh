@@ -12,29 +12,34 @@ namespace lgb {
 // the pair classes of s, p and d shells with total angular momentum up to
 // kTemplatedMaxL; classes with an f shell run on the cooperative kernels
 constexpr int kTemplatedPairClasses = 6;
-template <int B, int K>
+template <int B, int K, int MAXL = kTemplatedMaxL>
 constexpr bool templated_class() {
-  return B < kTemplatedPairClasses && K < kTemplatedPairClasses && pc_L(B) + pc_L(K) <= kTemplatedMaxL;
+  return B < kTemplatedPairClasses && K < kTemplatedPairClasses && pc_L(B) + pc_L(K) <= MAXL;
+}
+// FP32 and double-float kernels stop at kTemplatedMaxL4
+template <typename R>
+constexpr int max_l() {
+  return std::is_same<R, double>::value ? kTemplatedMaxL : kTemplatedMaxL4;
 }
 
 template <typename R, int B, int K>
 constexpr JKFn jk_entry() {
-  if constexpr (templated_class<B, K>() && B >= K) return &jk_tasks_kernel<R, pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
+  if constexpr (templated_class<B, K, max_l<R>()>() && B >= K) return &jk_tasks_kernel<R, pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
   else return nullptr;
 }
 template <int B, int K>
 constexpr JKFn jkr_entry() {
-  if constexpr (templated_class<B, K>() && B >= K) return &jk32_row_kernel<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
+  if constexpr (templated_class<B, K, kTemplatedMaxL4>() && B >= K) return &jk32_row_kernel<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
   else return nullptr;
 }
 template <typename R, int B, int K>
 constexpr CPFn cp_entry() {
-  if constexpr (templated_class<B, K>()) return &cp_tasks_kernel<R, pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
+  if constexpr (templated_class<B, K, max_l<R>()>()) return &cp_tasks_kernel<R, pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
   else return nullptr;
 }
 template <int B, int K>
 constexpr ITFn it_entry() {
-  if constexpr (templated_class<B, K>()) return &it_kernel<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
+  if constexpr (templated_class<B, K, kTemplatedMaxL4>()) return &it_kernel<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
   else return nullptr;
 }
 
@@ -56,6 +61,25 @@ static_assert(kNumPairClasses == 10, "launch-table rows list every pair class");
   const JKFn kJK64_##B[kNumPairClasses] = LGB_ROW(jk_entry, double, B); \
   const JKFn kJK32_##B[kNumPairClasses] = LGB_ROW(jk_entry, float, B);  \
   const JKFn kJKR_##B[kNumPairClasses] = LGB_ROW(jkr_entry, B);
+
+// Classes with double-float J/K kernels: those where they beat FP64.  ns per
+// quartet on the whole GPU, FP64 / double-float (12 waters with d shells, 480
+// functions): (ss|ss) .121/.064, (ps|ss) .253/.109, (ps|ps) .429/.216, (pp|ss)
+// .479/.193, (pp|ps) .954/.580, (ds|ss) .400/.177, (ds|ps) .740/.500, (dp|ss)
+// .847/.567.  Above 27 integrals the code (some 27,000 instructions for (pp|pp))
+// outgrows the instruction cache and little is left: (pp|pp) 2.64/2.38, (ds|pp)
+// 1.86/1.52, (dp|ps) 1.78/1.57, (ds|ds) 1.87/1.78, (dd|ss) 1.85/2.05.
+template <int B, int K>
+constexpr JKFn jkd_entry() {
+  if constexpr (templated_class<B, K, kTemplatedMaxL4>() && B >= K &&
+                QClass<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>::NINT <= 27)
+    return &jk_tasks_kernel<dd32, pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
+  else return nullptr;
+}
+
+#define LGB_JKD_TABLE(B)                                   \
+  extern const JKFn kJKD_##B[kNumPairClasses];                           \
+  const JKFn kJKD_##B[kNumPairClasses] = LGB_ROW(jkd_entry, B);
 
 #define LGB_CP_TABLES(B)                                   \
   extern const CPFn kCP64_##B[kNumPairClasses];                          \

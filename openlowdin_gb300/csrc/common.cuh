@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <type_traits>
 
+#include "dd32.cuh"
+
 namespace lgb {
 
 constexpr int kMaxL = 3;               // per-shell angular momentum handled by the kernels (f)
@@ -71,6 +73,7 @@ struct alignas(16) PairT {
 };
 using PairRec = PairT<double>;
 using PairRec32 = PairT<float>;
+using PairRecD = PairT<dd32>;   // double-float
 
 // One primitive pair: exponent sum p, its reciprocal, the Gaussian-product
 // centre P, P - A, and Kt = sqrt(2 pi^{5/2}) exp(-ab/p |AB|^2) c_a N_a c_b N_b / p
@@ -84,6 +87,33 @@ struct alignas(16) PrimT {
 };
 using PrimRec = PrimT<double>;
 using PrimRec32 = PrimT<float>;
+// In double-float the product centre has three terms: P - Q of two pairs on
+// one atom loses its leading digits, times sqrt(rho) of tight functions.
+template <>
+struct alignas(16) PrimT<dd32> {
+  dd32 p, inv_p, Kt, pad;
+  dd32 PA[3];
+  float P[3][3];
+  float pad2;
+};
+using PrimRecD = PrimT<dd32>;
+template <typename R>
+__device__ __forceinline__ R centre_diff(const PrimT<R> &a, const PrimT<R> &b, int d) {
+  if constexpr (std::is_same<R, dd32>::value) return diff3(a.P[d], b.P[d]);
+  else return a.P[d] - b.P[d];
+}
+template <typename R>
+__device__ __forceinline__ R halved(R x) {
+  if constexpr (std::is_same<R, dd32>::value) return scaled(x, 0.5f);
+  else return R(0.5) * x;
+}
+// K x of a small whole number
+template <int K, typename R>
+__device__ __forceinline__ R times(R x) {
+  if constexpr (K == 1) return x;
+  else if constexpr (std::is_same<R, dd32>::value) return K == 2 ? scaled(x, 2.f) : x * float(K);
+  else return R(K) * x;
+}
 
 constexpr double kSqrt2Pi52 = 5.914967172795612;  // sqrt(2 pi^{5/2})
 
@@ -203,8 +233,81 @@ __device__ __forceinline__ void boys_f32(float T, float (&F)[L + 1], const float
   }
 }
 
+// Boys function in double-float.  T < kBoysTMax: Taylor series of F_L about
+// T_i = i / 32 (|x| <= 1/64: seven terms leave 5e-17), whose coefficients carry
+// two FP32 terms up to k = 3 and one beyond (x^4 c_4 < 3e-9, so its FP32
+// rounding is below 2e-16); F_{L-1}.. by the downward recursion, for L = 1 by a
+// second series, which is cheaper than e^{-T}.  T >= kBoysTMax as in FP64, where
+// e^{-T} (< 3e-16) is an FP32 term.
+// Row i of order L (kDDRow floats): c_0..c_3 as (hi, lo), c_4, c_5, c_6, e^{-T_i} (hi, lo).
+constexpr int kDDMaxL = 4;
+constexpr int kDDPoints = 36 * 32 + 1;
+constexpr int kDDRow = 16;
+constexpr size_t kBoysDDSize = (size_t)(kDDMaxL + 1) * kDDPoints * kDDRow;
+
+__device__ __forceinline__ dd32 boys_dd_series(const float4 &a, const float4 &b, const float4 &c, dd32 x) {
+  const float t = ffma(x.hi, ffma(x.hi, c.z, c.y), c.x);
+  dd32 s = fast_two_sum(b.z, ffma(x.hi, t, b.w));
+  s = mad(s, x, dd32(b.x, b.y));
+  s = mad(s, x, dd32(a.z, a.w));
+  return mad(s, x, dd32(a.x, a.y));
+}
+// e^x, |x| <= 1/64
+__device__ __forceinline__ dd32 exp_small_dd(dd32 x) {
+  const float t = ffma(x.hi, ffma(x.hi, 1.f / 720, 1.f / 120), 1.f / 24);
+  dd32 s = fast_two_sum(1.f / 6, ffma(x.hi, t, (float)(1.0 / 6 - (double)(1.f / 6))));
+  s = mad(s, x, dd32(0.5f));
+  s = mad(s, x, dd32(1.f));
+  return mad(s, x, dd32(1.f));
+}
+
+template <int L>
+__device__ __forceinline__ void boys_dd(dd32 T, dd32 (&F)[L + 1], const float *__restrict__ tab) {
+  if (T.hi < (float)kBoysTMax) {
+    const int i = __float2int_rn(fmul(T.hi, 32.f));
+    const dd32 x = two_sum(fsub(fmul((float)i, 0.03125f), T.hi), -T.lo);
+    const float4 *r = reinterpret_cast<const float4 *>(tab + ((size_t)L * kDDPoints + i) * kDDRow);
+    const float4 c = __ldg(r + 2);
+    F[L] = boys_dd_series(__ldg(r), __ldg(r + 1), c, x);
+    if constexpr (L == 1) {
+      const float4 *q = reinterpret_cast<const float4 *>(tab + (size_t)i * kDDRow);
+      F[0] = boys_dd_series(__ldg(q), __ldg(q + 1), __ldg(q + 2), x);
+    } else if constexpr (L > 1) {
+      const dd32 e = dd32(c.w, __ldg(reinterpret_cast<const float *>(r + 3))) * exp_small_dd(x);
+      const dd32 twoT = scaled(T, 2.f);
+#pragma unroll
+      for (int m = L - 1; m >= 0; --m) {
+        const dd32 o((float)(1.0 / (2 * m + 1)), (float)(1.0 / (2 * m + 1) - (double)(float)(1.0 / (2 * m + 1))));
+        F[m] = mad(twoT, F[m + 1], e);
+        if (m) F[m] = F[m] * o;
+      }
+    }
+  } else {
+    const dd32 r = rsqrt_r(T);
+    F[0] = r * dd32((float)0.88622692545275801365,
+                    (float)(0.88622692545275801365 - (double)(float)0.88622692545275801365));
+    if constexpr (L > 0) {
+      const float e = __expf(-T.hi);
+      const dd32 o2T = scaled(r * r, 0.5f);
+#pragma unroll
+      for (int m = 0; m < L; ++m) {
+        dd32 v = m ? F[m] * float(2 * m + 1) : F[0];
+        v.lo = fsub(v.lo, e);
+        F[m + 1] = v * o2T;
+      }
+    }
+  }
+}
+
 template <typename R>
 struct BoysTab;
+template <>
+struct BoysTab<dd32> {
+  template <int L>
+  __device__ __forceinline__ static void eval(dd32 T, dd32 (&F)[L + 1], const double *, const float *tdd) {
+    boys_dd<L>(T, F, tdd);
+  }
+};
 template <>
 struct BoysTab<double> {
   template <int L>

@@ -22,6 +22,13 @@
 
 namespace lgb {
 
+template <typename R>
+__device__ __forceinline__ R shfl_xor(R v, int o) {
+  if constexpr (std::is_same<R, dd32>::value)
+    return dd32(__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o));
+  else return __shfl_xor_sync(0xffffffffu, v, o);
+}
+
 template <int LA, int LB, int LC, int LD>
 struct QClass {
   static constexpr int L1 = LA + LB, L2 = LC + LD, L = L1 + L2;
@@ -46,21 +53,21 @@ __device__ __forceinline__ void vrr_prim(R (&X)[QClass<LA, LB, LC, LD>::nE * QCl
   const R rp = q * opq;          // rho / p
   const R rq = p * opq;          // rho / q
   const R rho = p * rp;          // p q / (p + q)
-  R PQ2 = 0, PA[3], WP[3], QCv[3], WQ[3];
+  R PQ2 = R(0), PA[3], WP[3], QCv[3], WQ[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const R PQ = pb.P[d] - pk.P[d];
+    const R PQ = centre_diff(pb, pk, d);
     PA[d] = pb.PA[d];
     QCv[d] = pk.PA[d];
     WP[d] = -rp * PQ;            // W - P = q (Q - P) / (p + q)
     WQ[d] = rq * PQ;             // W - Q = p (P - Q) / (p + q)
-    PQ2 += PQ * PQ;
+    PQ2 = mad(PQ, PQ, PQ2);
   }
   R F[L + 1];
   BoysTab<R>::template eval<L>(rho * PQ2, F, boys64, boys32);
   // 2 pi^{5/2} K_ab K_cd / (p q sqrt(p + q)) with the constants folded into Kt
   const R pref = pb.Kt * pk.Kt * rs;
-  const R o2p = R(0.5) * pb.inv_p, o2q = R(0.5) * pk.inv_p, o2pq = R(0.5) * opq;
+  const R o2p = halved(pb.inv_p), o2q = halved(pk.inv_p), o2pq = halved(opq);
 
   // bra nodes Vb[e][m], m <= L - |e|
   R Vb[NE][L + 1];
@@ -73,8 +80,8 @@ __device__ __forceinline__ void vrr_prim(R (&X)[QClass<LA, LB, LC, LD>::nE * QCl
     constexpr int mmax = L - clevel(e);
 #pragma unroll
     for (int m = 0; m <= mmax; ++m) {
-      R v = PA[d] * Vb[em][m] + WP[d] * Vb[em][m + 1];
-      if constexpr (ei > 0) v += R(ei) * o2p * (Vb[emm][m] - rp * Vb[emm][m + 1]);
+      R v = mad2(PA[d], Vb[em][m], WP[d], Vb[em][m + 1]);
+      if constexpr (ei > 0) v = mad(times<ei>(o2p), mad(-rp, Vb[emm][m + 1], Vb[emm][m]), v);
       Vb[e][m] = v;
     }
   });
@@ -102,13 +109,16 @@ __device__ __forceinline__ void vrr_prim(R (&X)[QClass<LA, LB, LC, LD>::nE * QCl
         constexpr int em = ed > 0 ? cminus(e, d) : 0;
 #pragma unroll
         for (int m = 0; m <= mmax; ++m) {
-          R v = QCv[d] * get(ec, std::integral_constant<int, fm>{}, m) +
-                WQ[d] * get(ec, std::integral_constant<int, fm>{}, m + 1);
+          R v = mad2(QCv[d], get(ec, std::integral_constant<int, fm>{}, m), WQ[d],
+                     get(ec, std::integral_constant<int, fm>{}, m + 1));
           if constexpr (fi > 0)
-            v += R(fi) * o2q *
-                 (get(ec, std::integral_constant<int, fmm>{}, m) - rq * get(ec, std::integral_constant<int, fmm>{}, m + 1));
+            v = mad(times<fi>(o2q),
+                    mad(-rq, get(ec, std::integral_constant<int, fmm>{}, m + 1),
+                        get(ec, std::integral_constant<int, fmm>{}, m)),
+                    v);
           if constexpr (ed > 0)
-            v += R(ed) * o2pq * get(std::integral_constant<int, em>{}, std::integral_constant<int, fm>{}, m + 1);
+            v = mad(times<ed>(o2pq), get(std::integral_constant<int, em>{}, std::integral_constant<int, fm>{}, m + 1),
+                    v);
           Vk[e][f][m] = v;
         }
       });
@@ -152,7 +162,7 @@ __device__ __forceinline__ void hrr(const R *in, const R (&AB)[3], R *out) {
           constexpr int ar = decltype(ac)::value;
           constexpr int apr = cplus(A0 + ar, d) - A0;
 #pragma unroll
-          for (int k = 0; k < NK; ++k) H[j][ar][bi][k] = H[j - 1][apr][bm][k] + AB[d] * H[j - 1][ar][bm][k];
+          for (int k = 0; k < NK; ++k) H[j][ar][bi][k] = mad(AB[d], H[j - 1][ar][bm][k], H[j - 1][apr][bm][k]);
         });
       });
     });
@@ -191,7 +201,7 @@ __device__ __forceinline__ void hrr_ket(const R *in, const R (&CD)[3], R *out) {
           constexpr int cr = decltype(cc)::value;
           constexpr int cpr = cplus(C0 + cr, d) - C0;
 #pragma unroll
-          for (int r = 0; r < NROW; ++r) H[j][r][cr][di] = H[j - 1][r][cpr][dm] + CD[d] * H[j - 1][r][cr][dm];
+          for (int r = 0; r < NROW; ++r) H[j][r][cr][di] = mad(CD[d], H[j - 1][r][cr][dm], H[j - 1][r][cpr][dm]);
         });
       });
     });
@@ -207,22 +217,38 @@ __device__ __forceinline__ void hrr_ket(const R *in, const R (&CD)[3], R *out) {
 // Full contracted quartet: out[NA*NB*NC*ND] row-major (a, b, c, d).  pbra and
 // pket point at the first primitive pair of the bra and of the ket pair (they
 // may come from different species, and from global or shared memory).
+// parts > 1 (a power of two, uniform in the warp): the primitive quartets are
+// dealt to `parts` lanes, 32 / parts apart, and their contracted [e0|f0] added
+// by shuffles, so every lane of the warp must call and ends with the whole
+// quartet; lanes with live = false add nothing.  slice / slices: only every
+// slices-th round of `parts` primitive quartets, from round `slice` on.
 template <typename R, int LA, int LB, int LC, int LD>
 __device__ __forceinline__ void eri_quartet(const PairT<R> &bra, const PrimT<R> *pbra, const PairT<R> &ket,
                                             const PrimT<R> *pket,
                                             const double *boys64, const float *boys32,
-                                            R (&out)[QClass<LA, LB, LC, LD>::NINT]) {
+                                            R (&out)[QClass<LA, LB, LC, LD>::NINT], int part = 0, int parts = 1,
+                                            bool live = true, int slice = 0, int slices = 1) {
   using QC_ = QClass<LA, LB, LC, LD>;
   R X[QC_::nE * QC_::nF];
 #pragma unroll
   for (int i = 0; i < QC_::nE * QC_::nF; ++i) X[i] = R(0);
-  for (int ib = 0; ib < bra.nprim; ++ib) {
-    const PrimT<R> pb = pbra[ib];
-    for (int ik = 0; ik < ket.nprim; ++ik) {
-      const PrimT<R> pk = pket[ik];
-      vrr_prim<R, LA, LB, LC, LD>(X, pb, pk, boys64, boys32);
+  const int nk = ket.nprim, np = live ? bra.nprim * nk : 0;
+  const int first = slice * parts + part, step = slices * parts;
+  int ib = 0, ik = first;
+  for (int k = first; k < np; k += step) {
+    while (ik >= nk) {
+      ik -= nk;
+      ++ib;
     }
+    const PrimT<R> pb = pbra[ib];
+    const PrimT<R> pk = pket[ik];
+    vrr_prim<R, LA, LB, LC, LD>(X, pb, pk, boys64, boys32);
+    ik += step;
   }
+  if (parts > 1)
+    for (int o = 32 / parts; o < 32; o <<= 1)
+#pragma unroll
+      for (int i = 0; i < QC_::nE * QC_::nF; ++i) X[i] += shfl_xor(X[i], o);
   const R AB[3] = {bra.AB[0], bra.AB[1], bra.AB[2]};
   const R CD[3] = {ket.AB[0], ket.AB[1], ket.AB[2]};
   R Y[QC_::NA * QC_::NB * QC_::nF];

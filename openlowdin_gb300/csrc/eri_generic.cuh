@@ -57,7 +57,9 @@ __device__ __forceinline__ const CartInfo *cart_shared(CartInfo *dst) {
 struct CoLayout {
   int vb, vk, x, h0, h1, y, out, misc, kb, total;
 };
-constexpr int kCoMiscN = 32;
+constexpr int kCoBatch = 8;                  // primitive quartets whose scalars are prepared together
+constexpr int kCoScalars = 17 + kGenMaxL + 1;  // PA WP QC WQ rp rq o2p o2q o2pq, then [00|00]^(m)
+constexpr int kCoMiscN = kCoBatch * kCoScalars;
 constexpr int kCoKbN = (kCartN + 2) / 2;   // doubles holding kCartN + 1 ints
 
 __host__ __device__ inline CoLayout co_layout(int la, int lb, int lc, int ld) {
@@ -143,18 +145,22 @@ __device__ inline void geminal_aux(int L, double rho, double T, const double *__
 // row-major (a, b, c, d).  Every thread of the group must call it (it
 // synchronises the group); the result is valid after the call returns.
 // GEM: the operator is the geminal `gem` (geminal_aux) instead of 1/r12.
+// slice / slices: only the primitive quartets slice, slice + slices, ... are
+// contracted (a share of the integrals; the shares add up to the quartet).
+// The scalars and auxiliary functions of up to kCoBatch primitive quartets are
+// prepared at once, one lane each: on one lane that serial chain of FP64
+// operations held up the other 31 for every primitive quartet.
 template <typename G, bool GEM = false>
 __device__ inline void eri_coop(G g, const CartInfo *__restrict__ ct, const CoLayout &Lo, int la, int lb, int lc,
                                 int ld, const PairRec &bra, const PrimRec *__restrict__ pbra, const PairRec &ket,
                                 const PrimRec *__restrict__ pket, const double *boys64, double *sm,
-                                const double *gem = nullptr) {
+                                const double *gem = nullptr, int slice = 0, int slices = 1) {
   const int tid = g.tid(), nt = g.nt();
   const int L1 = la + lb, L2 = lc + ld, L = L1 + L2, M = L + 1;
   const int NE = coff(L1 + 1), NF = coff(L2 + 1), E0 = coff(la), F0 = coff(lc);
   const int nE = NE - E0, nF = NF - F0;
   double *Vb = sm + Lo.vb, *Vk = sm + Lo.vk, *X = sm + Lo.x, *Y = sm + Lo.y, *out = sm + Lo.out;
   double *Hb[2] = {sm + Lo.h0, sm + Lo.h1};
-  double *misc = sm + Lo.misc;
   int *kb = reinterpret_cast<int *>(sm + Lo.kb);
   g.sync();   // the previous quartet's readers of the work arrays are done
   for (int i = tid; i < nE * nF; i += nt) X[i] = 0.0;
@@ -166,35 +172,42 @@ __device__ inline void eri_coop(G g, const CartInfo *__restrict__ ct, const CoLa
       off += NE * (L2 - ct[f].lev + 1);
     }
   }
-  for (int ib = 0; ib < bra.nprim; ++ib)
-    for (int ik = 0; ik < ket.nprim; ++ik) {
-      g.sync();
-      if (tid == 0) {
-        const PrimRec pb = pbra[bra.prim0 + ib];
-        const PrimRec pk = pket[ket.prim0 + ik];
-        const double p = pb.p, q = pk.p;
-        const double opq = 1.0 / (p + q);
-        const double rp = q * opq, rq = p * opq, rho = p * rp;
-        double PQ2 = 0;
-        for (int d = 0; d < 3; ++d) {
-          const double PQ = pb.P[d] - pk.P[d];
-          misc[d] = pb.PA[d];          // PA
-          misc[3 + d] = -rp * PQ;      // WP
-          misc[6 + d] = pk.PA[d];      // QC
-          misc[9 + d] = rq * PQ;       // WQ
-          PQ2 += PQ * PQ;
-        }
-        misc[12] = rp;
-        misc[13] = rq;
-        misc[14] = 0.5 * pb.inv_p;
-        misc[15] = 0.5 * pk.inv_p;
-        misc[16] = 0.5 * opq;
-        double F[kGenMaxL + 1];
-        if constexpr (GEM) geminal_aux(L, rho, rho * PQ2, gem, F);
-        else boys_f64_rt(L, rho * PQ2, F, boys64);
-        const double pref = pb.Kt * pk.Kt * sqrt(opq);
-        for (int m = 0; m <= L; ++m) Vb[m] = pref * F[m];
+  const int nk = ket.nprim, np = bra.nprim * nk;
+  for (int k0 = slice; k0 < np; k0 += slices * kCoBatch) {
+    g.sync();
+    const int batch = min(kCoBatch, (np - k0 + slices - 1) / slices);
+    if (tid < batch) {
+      const int k = k0 + tid * slices;
+      double *misc = sm + Lo.misc + tid * kCoScalars;
+      const PrimRec pb = pbra[bra.prim0 + k / nk];
+      const PrimRec pk = pket[ket.prim0 + k % nk];
+      const double p = pb.p, q = pk.p;
+      const double opq = 1.0 / (p + q);
+      const double rp = q * opq, rq = p * opq, rho = p * rp;
+      double PQ2 = 0;
+      for (int d = 0; d < 3; ++d) {
+        const double PQ = pb.P[d] - pk.P[d];
+        misc[d] = pb.PA[d];          // PA
+        misc[3 + d] = -rp * PQ;      // WP
+        misc[6 + d] = pk.PA[d];      // QC
+        misc[9 + d] = rq * PQ;       // WQ
+        PQ2 += PQ * PQ;
       }
+      misc[12] = rp;
+      misc[13] = rq;
+      misc[14] = 0.5 * pb.inv_p;
+      misc[15] = 0.5 * pk.inv_p;
+      misc[16] = 0.5 * opq;
+      double F[kGenMaxL + 1];
+      if constexpr (GEM) geminal_aux(L, rho, rho * PQ2, gem, F);
+      else boys_f64_rt(L, rho * PQ2, F, boys64);
+      const double pref = pb.Kt * pk.Kt * sqrt(opq);
+      for (int m = 0; m <= L; ++m) misc[17 + m] = pref * F[m];
+    }
+    for (int j = 0; j < batch; ++j) {
+      const double *misc = sm + Lo.misc + j * kCoScalars;
+      g.sync();
+      if (tid <= L) Vb[tid] = misc[17 + tid];
       g.sync();
       const double rp = misc[12], rq = misc[13], o2p = misc[14], o2q = misc[15], o2pq = misc[16];
       // bra vertical recursion, one angular-momentum level at a time
@@ -246,6 +259,7 @@ __device__ inline void eri_coop(G g, const CartInfo *__restrict__ ct, const CoLa
         X[i] += Vk[kb[f] + e * (L2 - ct[f].lev + 1)];
       }
     }
+  }
   g.sync();
   // bra transfer: X [a over totals la..la+lb][nF] -> Y [NA][NB][nF]
   const int NA = ncart(la), NB = ncart(lb), NC = ncart(lc), ND = ncart(ld);

@@ -12,7 +12,7 @@ namespace lgb {
 template <typename R>
 __device__ __forceinline__ R warp_sum(R v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 16; o > 0; o >>= 1) v += shfl_xor(v, o);
   return v;
 }
 
@@ -31,32 +31,26 @@ template <typename R>
 __device__ __forceinline__ bool abs_above(R v, R t) { return abs_bits(v) > abs_bits(t); }
 // 2^k, k = 0..3 (quartet degeneracies), from the exponent field alone
 template <typename R>
-__device__ __forceinline__ R pow2(int k) {
+__device__ __forceinline__ auto pow2(int k) {
   if constexpr (std::is_same<R, double>::value) return __longlong_as_double((long long)(1023 + k) << 52);
   else return __int_as_float((127 + k) << 23);
 }
 
-// largest shell-block maximum |D| over the six index pairs of a quartet
+// largest shell-block maximum |D| over the six index pairs of a quartet, by bit
+// patterns: the norms are >= 0, and a NaN orders above every number, so that no
+// quartet that meets one is screened
 template <typename T>
 __device__ __forceinline__ T dnorm6(const T *__restrict__ Dn, int nsh, int a, int b, int c, int d) {
-  T m = __ldg(Dn + a * nsh + b);
-  m = max(m, __ldg(Dn + a * nsh + c));
-  m = max(m, __ldg(Dn + b * nsh + c));
-  m = max(m, __ldg(Dn + a * nsh + d));
-  m = max(m, __ldg(Dn + b * nsh + d));
-  m = max(m, __ldg(Dn + c * nsh + d));
-  return m;
-}
-template <>
-__device__ __forceinline__ double dnorm6(const double *__restrict__ Dn, int nsh, int a, int b, int c, int d) {
-  const unsigned long long *u = reinterpret_cast<const unsigned long long *>(Dn);   // entries are >= 0
-  unsigned long long m = __ldg(u + a * nsh + b);
+  using U = std::conditional_t<std::is_same<T, double>::value, unsigned long long, unsigned>;
+  const U *u = reinterpret_cast<const U *>(Dn);
+  U m = __ldg(u + a * nsh + b);
   m = max(m, __ldg(u + a * nsh + c));
   m = max(m, __ldg(u + b * nsh + c));
   m = max(m, __ldg(u + a * nsh + d));
   m = max(m, __ldg(u + b * nsh + d));
   m = max(m, __ldg(u + c * nsh + d));
-  return __longlong_as_double((long long)m);
+  if constexpr (std::is_same<T, double>::value) return __longlong_as_double((long long)m);
+  else return __uint_as_float(m);
 }
 
 // Per-system build flag of a batch (LowdinGB300_batch_set_active): off
@@ -77,10 +71,37 @@ __device__ __forceinline__ int find_task(const T *__restrict__ tasks, int ntasks
   return lo;
 }
 
+__device__ __forceinline__ double scaled(double a, double f) { return a * f; }
+__device__ __forceinline__ float scaled(float a, float f) { return a * f; }
+
 template <typename R>
 __device__ __forceinline__ void atomic_acc(double *g64, float *g32, size_t i, R v) {
   if constexpr (std::is_same<R, double>::value) atomicAdd(g64 + i, v);
+  else if constexpr (std::is_same<R, dd32>::value) atomicAdd(g64 + i, to_double(v));
   else atomicAdd(g32 + i, v);
+}
+
+// element i of a matrix kept in FP64, FP32 and double-float
+template <typename R>
+__device__ __forceinline__ R elem(const double *m64, const float *m32, const float2 *md, int i) {
+  if constexpr (std::is_same<R, double>::value) return __ldg(m64 + i);
+  else if constexpr (std::is_same<R, dd32>::value) {
+    const float2 v = __ldg(md + i);
+    return dd32(v.x, v.y);
+  } else return __ldg(m32 + i);
+}
+
+// FP32 Schwarz factor of a record of any precision (that of its FP32 copy)
+__device__ __forceinline__ float schwarz32(const PairRec &p) { return (float)p.Q; }
+__device__ __forceinline__ float schwarz32(const PairRec32 &p) { return p.Q; }
+__device__ __forceinline__ float schwarz32(const PairRecD &p) { return p.Q.hi; }
+
+// Bound of the double-float quartets of a species: `tier` (kTierBound times
+// its largest product of Schwarz factors) times the largest density element.
+// Zero, so that everything stays in FP64, for densities whose products could
+// leave the FP32 exponent range, infinities and NaN.
+__device__ __forceinline__ float tier_bound(float tier, float d) {
+  return d > 1e-12f && d < 1e20f ? tier * d : 0.f;
 }
 
 // ----------------------------------------------------------------- Schwarz --
@@ -91,7 +112,7 @@ __global__ void __launch_bounds__(128) schwarz_kernel(SchwarzParams P) {
   const PairRec pr = P.pairs[P.p0 + t];
   constexpr int N = ncart(LA) * ncart(LB);
   double I[N * N];
-  eri_quartet<double, LA, LB, LA, LB>(pr, P.prims + pr.prim0, pr, P.prims + pr.prim0, P.boys.f64, P.boys.f32, I);
+  eri_quartet<double, LA, LB, LA, LB>(pr, P.prims + pr.prim0, pr, P.prims + pr.prim0, P.boys.f64, P.boys.dd, I);
   double m = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i) m = fmax(m, fabs(I[i * N + i]));
@@ -99,8 +120,10 @@ __global__ void __launch_bounds__(128) schwarz_kernel(SchwarzParams P) {
 }
 
 // --------------------------------------------------------------------- J/K --
-// Lane x of warp y in a block evaluates quartet (bra = tile_y*4 + y, ket =
-// tile_x*32 + x) of its task.  The 32 lanes of a warp share the bra pair, so the
+// Warp y of a block takes bra pair tile_y * bras + y of its task and the ket
+// pairs tile_x * kets + (lane mod kets): one quartet per lane, or, for
+// contracted classes (kets < 32), 32 / kets lanes per quartet, of which the
+// first digests it.  The 32 lanes of a warp share the bra pair, so the
 // bra-block Coulomb term is reduced across the warp before its atomics.
 // Digestion follows the six updates of a permutation-unique quartet
 // (g12 += D34 v, g34 += D12 v, g13/g24/g14/g23 += 0.5 f D v, all x degeneracy);
@@ -109,180 +132,269 @@ __global__ void __launch_bounds__(128) schwarz_kernel(SchwarzParams P) {
 // Q_ab Q_cd max|D| as the reference does; mixed launches compute it in FP32
 // from the FP32 records in both kernels, so each quartet lands in exactly one
 // of the FP64 (bound >= split) and FP32 (bound < split) launches.
+// Tier: the FP64 and the double-float launch of a class compute the same FP32
+// bound and divide the quartets at tier_bound; the screening decision itself is
+// the FP64 one in both (taken from FP32 only where that cannot differ).
+// Blocks per SM the registers are cut for.  The light double-float classes wait
+// on loads (L1 hits half of the scattered density and norm reads), so more warps
+// pay until spills outweigh them: 387-function chain, (ps|ss) 5.5 ms at 4
+// blocks, 4.6 at 5, 5.3 at 6; (ss|ss) 2.2 -> 1.85 at 8; (ps|ps) 3.8 -> 3.6 and
+// (pp|ss) 2.1 -> 1.6 at 4.
 template <typename R, int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(128) jk_tasks_kernel(const JKTask *__restrict__ tasks, TaskLaunch TL) {
+constexpr int jk_min_blocks() {
+  if (!std::is_same<R, dd32>::value) return 1;
+  constexpr int N = QClass<LA, LB, LC, LD>::NINT;
+  return N == 1 ? 8 : N <= 3 ? 5 : N <= 9 ? 4 : 1;
+}
+template <typename R, int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) jk_tasks_kernel(const JKTask *__restrict__ tasks, TaskLaunch TL) {
   using Q = QClass<LA, LB, LC, LD>;
-  constexpr bool F64 = std::is_same<R, double>::value;
+  constexpr bool F64 = std::is_same<R, double>::value, DD = std::is_same<R, dd32>::value;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
-  const int t = find_task(tasks, TL.ntasks, blockIdx.x);
-  const JKTask &T = tasks[t];
-  const int act = system_flag(T.active);
-  if (act == kSysOff) return;   // converged system: nothing to build
-  if (act == kSysFP64 && TL.mixed && TL.lower) return;   // system held in FP64: the FP64 launch takes it all
-  const int local = blockIdx.x - T.blk0;
-  const int tx = local % T.nbx, ty = local / T.nbx;
-  if (T.triangle && tx * 32 > ty * kWarpsPerBlock + kWarpsPerBlock - 1) return;
-  if (TL.mixed && act != kSysFP64 && ty * kWarpsPerBlock < T.nbra && (T.Dnmax32 || !T.screen)) {
-    // The tile's first bra and first ket carry its largest Schwarz factors and
-    // Dnmax32 bounds the six norms, so in FP32 (rounding is monotonic, same
-    // order of products) ub >= every quartet bound b of the tile: a tile the
-    // launch cannot take leaves before staging its records.
-    float ub = T.pairs32[T.bra0 + ty * kWarpsPerBlock].Q * T.pairs32[T.ket0 + tx * 32].Q;
-    if (T.screen) ub *= __ldg(T.Dnmax32);
-    if (TL.lower ? (T.screen && ub < fmaxf(TL.eps32, TL.skip)) : ub < TL.split32) return;
-  }
-  const PairT<R> *pairs;
-  const PrimT<R> *prims;
-  const R *D;
-  if constexpr (F64) {
-    pairs = T.pairs; prims = T.prims; D = T.Ds;
-  } else {
-    pairs = T.pairs32; prims = T.prims32; D = T.Ds32;
-  }
-  // The block's 32 ket pairs (shared by its bra warps) and the first primitive
-  // pair of each, staged once in shared memory by coalesced 16-byte copies.
-  // Strides 80 / 112 B (pairs) and 48 / 80 B (primitives) keep the per-lane
-  // 16-byte reads free of bank conflicts.
+  // The tile's ket pairs (shared by its bra warps) and the first primitive
+  // pair of each, staged in shared memory by coalesced 16-byte copies.
+  // Strides 80 / 112 B (pairs) and 48 / 80 / 96 B (primitives) keep the per-lane
+  // 16-byte reads nearly free of bank conflicts.
   struct alignas(16) SPair {
     PairT<R> p;
     int4 pad;
   };
   __shared__ SPair sk[32];
   __shared__ PrimT<R> skp[32];
-  {
-    constexpr int WP = sizeof(PairT<R>) / 16, WQ = sizeof(PrimT<R>) / 16;
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    for (int w = tid; w < 32 * WP; w += 32 * kWarpsPerBlock) {
-      const int r = w / WP, k = w % WP;
-      const int kr = T.ket0 + min(tx * 32 + r, T.nket - 1);
-      reinterpret_cast<int4 *>(&sk[r].p)[k] = __ldg(reinterpret_cast<const int4 *>(pairs + kr) + k);
-    }
-    __syncthreads();
-    for (int w = tid; w < 32 * WQ; w += 32 * kWarpsPerBlock) {
-      const int r = w / WQ, k = w % WQ;
-      reinterpret_cast<int4 *>(skp + r)[k] = __ldg(reinterpret_cast<const int4 *>(prims + sk[r].p.prim0) + k);
-    }
-    __syncthreads();
+  const int slices = TL.tile.slices;
+  int blk = blockIdx.x, slice = 0;
+  if (slices > 1) {
+    blk = blockIdx.x / slices;
+    slice = blockIdx.x - blk * slices;
   }
-  const int kpos = tx * 32 + threadIdx.x;
-  const int bpos = ty * kWarpsPerBlock + threadIdx.y;
-  if (bpos >= T.nbra) return;  // warp-uniform
-  bool active = kpos < T.nket && (!T.triangle || kpos <= bpos);
-  const int bi = T.bra0 + bpos;
-  const int ki = T.ket0 + min(kpos, T.nket - 1);
-  const PairT<R> &bra = pairs[bi];
-  const PairT<R> &ket = sk[threadIdx.x].p;
+  const int t = find_task(tasks, TL.ntasks, blk);
+  const JKTask &T = tasks[t];
+  const int act = system_flag(T.active);
+  if (act == kSysOff) return;   // converged system: nothing to build
+  const bool all64 = act == kSysFP64;   // system held in FP64: the launches above the split take it all
+  if (all64 && TL.mixed && TL.lower) return;
+  const int local = blk - T.blk0;
+  const int kets = TL.tile.kets, parts = 32 / kets, bras = blockDim.y;
+  const int ty = local / T.nbx, b0 = ty * bras;
+  int k0 = (local - ty * T.nbx) * TL.tile.chunk * kets;
+  int kend = min(T.nket, k0 + TL.tile.chunk * kets);
+  if (T.triangle) kend = min(kend, b0 + bras);
+  if (k0 >= kend) return;
+  // The quartets of this launch have lo <= b (b < split in the FP32 half), b the
+  // FP32 bound: Q_ab Q_cd times, for screened species, the largest of the six
+  // shell-block norms,
+  float lo = 0.f;
   if (TL.mixed) {
-    // FP32 bound from the FP32 Schwarz factors (the FP64 records hold the
-    // same values before rounding), identical in both launches
-    float b = T.pairs32[bi].Q * (float)ket.Q;
-    if (T.screen) {
-      b *= dnorm6(T.Dn32, T.nsh, bra.sa, bra.sb, ket.sa, ket.sb);
-      if (b < fmaxf(TL.eps32, act == kSysFP64 ? 0.f : TL.skip)) active = false;   // no skip in an FP64 check
-    }
-    if (act != kSysFP64 && (TL.lower ? !(b < TL.split32) : (b < TL.split32))) active = false;
-  } else if (T.screen) {
-    const double b = T.pairs[bi].Q * (F64 ? (double)ket.Q : T.pairs[ki].Q) *
-                     dnorm6(T.Dn, T.nsh, bra.sa, bra.sb, ket.sa, ket.sb);
-    if (abs_below(b, TL.eps)) active = false;
+    const float cutoff = T.screen ? fmaxf(TL.eps32, all64 ? 0.f : TL.skip) : 0.f;
+    lo = TL.lower || all64 ? cutoff : fmaxf(cutoff, TL.split32);
   }
-  if (__all_sync(0xffffffffu, !active)) return;
-  if (T.count) {
-    const unsigned cnt = __popc(__ballot_sync(0xffffffffu, active));
-    if (threadIdx.x == 0) atomicAdd(T.count, (unsigned long long)cnt);
-  }
-  R I[Q::NINT];
-  if (active) {
-    const PrimT<R> *kp = ket.nprim == 1 ? skp + threadIdx.x : prims + ket.prim0;
-    eri_quartet<R, LA, LB, LC, LD>(bra, prims + bra.prim0, ket, kp, TL.boys.f64, TL.boys.f32, I);
+  // and, w being that bound (for species without screening, Q_ab Q_cd times the
+  // largest norm of all), w >= tb in the FP64 launch, w < tb in the
+  // double-float one
+  const float dmax = T.Dnmax32 ? __ldg(T.Dnmax32) : -1.f;
+  const float tb = TL.tier == Tier::all ? 0.f : tier_bound(T.tier, dmax);
+  if (TL.tier == Tier::lower && (tb == 0.f || (T.screen && !(lo < tb)))) return;
+  // Pairs are sorted by decreasing Schwarz factor inside a class and Dnmax32
+  // bounds the six norms, so the first bra and the first ket of a range bound
+  // every quartet after them (FP32 rounding is monotonic, same order of
+  // products; plain builds screen in FP64, with room for that rounding): the
+  // block leaves, before staging records, a range that cannot reach lo.
+  const float qb0 = T.pairs32[T.bra0 + b0].Q;
+  const float reach = TL.mixed ? lo : (T.screen ? TL.eps32 * 0.99999f : 0.f);
+  const float tier_reach = TL.tier == Tier::upper ? tb : 0.f;
+  auto out_of_reach = [&](int k) {
+    const float qq = qb0 * T.pairs32[T.ket0 + k].Q;
+    if (T.screen) return dmax >= 0.f && qq * dmax < fmaxf(reach, tier_reach);
+    return qq < reach || (TL.tier == Tier::upper && qq * dmax < tier_reach);
+  };
+  if (out_of_reach(k0)) return;
+  const PairT<R> *pairs;
+  const PrimT<R> *prims;
+  if constexpr (F64) {
+    pairs = T.pairs; prims = T.prims;
+  } else if constexpr (DD) {
+    pairs = T.pairsd; prims = T.primsd;
   } else {
-#pragma unroll
-    for (int x = 0; x < Q::NINT; ++x) I[x] = R(0);
+    pairs = T.pairs32; prims = T.prims32;
   }
-  const R deg = active ? pow2<R>((bra.sa != bra.sb) + (ket.sa != ket.sb) + (bi != ki)) : R(0);
-  R hf;
-  if constexpr (F64) hf = T.hf;
-  else hf = T.hf32;
-  const R hdeg = deg * hf;
+  auto D = [&](int i) { return elem<R>(T.Ds, T.Ds32, T.Dd, i); };
   const int n = T.n;
   double *G = T.Gacc;
   float *G32 = T.Gacc32;
-  const int fa = bra.fa, fb = bra.fb, fc = ket.fa, fd = ket.fb;
-  auto Iat = [&](int a, int b, int c, int d) -> R { return I[((a * NB + b) * NC + c) * ND + d]; };
-  // J12: bra block, warp-reduced
+  const int kl = threadIdx.x & (kets - 1), part = parts == 1 ? 0 : threadIdx.x / kets;
+  const int bpos = b0 + threadIdx.y;
+  const int bi = T.bra0 + min(bpos, T.nbra - 1);
+  const PairT<R> &bra = pairs[bi];
+  const int fa = bra.fa, fb = bra.fb;
+  const float qbra = T.pairs32[bi].Q;
+  R hf;
+  if constexpr (F64) hf = T.hf;
+  else if constexpr (DD) hf = dd32(T.hfd.x, T.hfd.y);
+  else hf = T.hf32;
+  R j12[NA * NB];
 #pragma unroll
-  for (int a = 0; a < NA; ++a)
+  for (int x = 0; x < NA * NB; ++x) j12[x] = R(0);
+  unsigned cnt = 0;
+  bool worked = false;
+  for (bool first = true; k0 < kend; k0 += kets, first = false) {
+    if (!first && out_of_reach(k0)) break;   // every later ket is out of reach too
+    __syncwarp();
+    __syncthreads();                         // the previous tile has been read
+    {
+      constexpr int WP = sizeof(PairT<R>) / 16, WQ = sizeof(PrimT<R>) / 16;
+      const int tid = threadIdx.y * 32 + threadIdx.x;
+      for (int w = tid; w < kets * WP; w += 32 * bras) {
+        const int r = w / WP, k = w % WP;
+        const int kr = T.ket0 + min(k0 + r, T.nket - 1);
+        reinterpret_cast<int4 *>(&sk[r].p)[k] = __ldg(reinterpret_cast<const int4 *>(pairs + kr) + k);
+      }
+      __syncthreads();
+      for (int w = tid; w < kets * WQ; w += 32 * bras) {
+        const int r = w / WQ, k = w % WQ;
+        reinterpret_cast<int4 *>(skp + r)[k] = __ldg(reinterpret_cast<const int4 *>(prims + sk[r].p.prim0) + k);
+      }
+      __syncthreads();
+    }
+    const int kpos = k0 + kl;
+    if (bpos >= T.nbra) continue;  // warp-uniform
+    bool active = kpos < T.nket && (!T.triangle || kpos <= bpos);
+    const int ki = T.ket0 + min(kpos, T.nket - 1);
+    const PairT<R> &ket = sk[kl].p;
+    if (TL.mixed || TL.tier != Tier::all) {
+      // FP32 bound from the FP32 Schwarz factors and norms, identical in every
+      // launch of the class
+      float b = qbra * schwarz32(ket);
+      const float qq = b;
+      if (T.screen) b *= dnorm6(T.Dn32, T.nsh, bra.sa, bra.sb, ket.sa, ket.sb);
+      const float w = T.screen ? b : qq * dmax;
+      if (TL.mixed) {
+        if (T.screen && b < fmaxf(TL.eps32, all64 ? 0.f : TL.skip)) active = false;   // no skip in an FP64 check
+        if (!all64 && (TL.lower ? !(b < TL.split32) : (b < TL.split32))) active = false;
+      } else if (T.screen && b < 1.00001f * TL.eps32) {
+        if (b < 0.99999f * TL.eps32) active = false;
+        else if (active) {
+          // too near the threshold for FP32 to decide
+          const double b64 = T.pairs[bi].Q * T.pairs[ki].Q * dnorm6(T.Dn, T.nsh, bra.sa, bra.sb, ket.sa, ket.sb);
+          if (abs_below(b64, TL.eps)) active = false;
+        }
+      }
+      if (TL.tier != Tier::all) {
+        if (TL.tier == Tier::upper ? w < tb : !(w < tb)) active = false;
+      }
+    } else if (T.screen) {
+      const double b = T.pairs[bi].Q * T.pairs[ki].Q * dnorm6(T.Dn, T.nsh, bra.sa, bra.sb, ket.sa, ket.sb);
+      if (abs_below(b, TL.eps)) active = false;
+    }
+    const unsigned live = __ballot_sync(0xffffffffu, active && part == 0);
+    if (!__any_sync(0xffffffffu, active)) continue;
+    if (slice == 0) cnt += __popc(live);
+    else {   // quartets without a primitive quartet in this slice
+      if (slice * parts >= bra.nprim * ket.nprim) active = false;
+      if (!__any_sync(0xffffffffu, active)) continue;
+    }
+    worked = true;
+    const int fc = ket.fa, fd = ket.fb;
+    R I[Q::NINT];
+    if (active || parts > 1) {
+      const PrimT<R> *kp = ket.nprim == 1 ? skp + kl : prims + ket.prim0;
+      eri_quartet<R, LA, LB, LC, LD>(bra, prims + bra.prim0, ket, kp, TL.boys.f64, TL.boys.dd, I, part, parts, active,
+                                     slice, slices);
+      if (part) active = false;   // the quartet is digested by its first lane
+    }
+    if (!active) continue;   // no warp-wide step follows inside the loop
+    // density blocks of the quartet, all asked for at once: one at a time behind
+    // the atomics before them they would cost a trip to L2 each
+    R dcd[NC][ND], dac[NA][NC], dad[NA][ND], dbc[NB][NC], dbd[NB][ND];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int d = 0; d < ND; ++d) dcd[c][d] = D((fc + c) * n + fd + d);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) dac[a][c] = D((fa + a) * n + fc + c);
+#pragma unroll
+      for (int d = 0; d < ND; ++d) dad[a][d] = D((fa + a) * n + fd + d);
+    }
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      R s = 0;
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
+      for (int c = 0; c < NC; ++c) dbc[b][c] = D((fb + b) * n + fc + c);
 #pragma unroll
-        for (int d = 0; d < ND; ++d) s += __ldg(D + (fc + c) * n + fd + d) * Iat(a, b, c, d);
-      s = warp_sum(s * deg);
-      if (threadIdx.x == 0) atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fb + b, s);
+      for (int d = 0; d < ND; ++d) dbd[b][d] = D((fb + b) * n + fd + d);
     }
-  if (!active) return;
-  // J34
+    const auto deg = pow2<R>((bra.sa != bra.sb) + (ket.sa != ket.sb) + (bi != ki));
+    const R hdeg = scaled(hf, deg);
+    auto Iat = [&](int a, int b, int c, int d) -> R { return I[((a * NB + b) * NC + c) * ND + d]; };
+    // J12: bra block, summed over this block's kets; J34
 #pragma unroll
-  for (int c = 0; c < NC; ++c)
+    for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      R s = 0;
+      for (int d = 0; d < ND; ++d) {
+        const R w = scaled(dcd[c][d], deg);
+        R s = R(0);
 #pragma unroll
-      for (int a = 0; a < NA; ++a)
+        for (int a = 0; a < NA; ++a)
 #pragma unroll
-        for (int b = 0; b < NB; ++b) s += __ldg(D + (fa + a) * n + fb + b) * Iat(a, b, c, d);
-      atomic_acc<R>(G, G32, (size_t)(fc + c) * n + fd + d, s * deg);
+          for (int b = 0; b < NB; ++b) {
+            j12[a * NB + b] = mad(w, Iat(a, b, c, d), j12[a * NB + b]);
+            s = mad(D((fa + a) * n + fb + b), Iat(a, b, c, d), s);
+          }
+        atomic_acc<R>(G, G32, (size_t)(fc + c) * n + fd + d, scaled(s, deg));
+      }
+    // K13 (i,k) += D(j,l), K14 (i,l) += D(j,k)
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        R s = R(0);
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int d = 0; d < ND; ++d) s = mad(dbd[b][d], Iat(a, b, c, d), s);
+        atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fc + c, s * hdeg);
+      }
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {
+        R s = R(0);
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int c = 0; c < NC; ++c) s = mad(dbc[b][c], Iat(a, b, c, d), s);
+        atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fd + d, s * hdeg);
+      }
     }
-  // K13 (i,k) += D(j,l)
+    // K24 (j,l) += D(i,k), K23 (j,k) += D(i,l)
 #pragma unroll
-  for (int a = 0; a < NA; ++a)
+    for (int b = 0; b < NB; ++b) {
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      R s = 0;
+      for (int d = 0; d < ND; ++d) {
+        R s = R(0);
 #pragma unroll
-      for (int b = 0; b < NB; ++b)
+        for (int a = 0; a < NA; ++a)
 #pragma unroll
-        for (int d = 0; d < ND; ++d) s += __ldg(D + (fb + b) * n + fd + d) * Iat(a, b, c, d);
-      atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fc + c, s * hdeg);
+          for (int c = 0; c < NC; ++c) s = mad(dac[a][c], Iat(a, b, c, d), s);
+        atomic_acc<R>(G, G32, (size_t)(fb + b) * n + fd + d, s * hdeg);
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        R s = R(0);
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+#pragma unroll
+          for (int d = 0; d < ND; ++d) s = mad(dad[a][d], Iat(a, b, c, d), s);
+        atomic_acc<R>(G, G32, (size_t)(fb + b) * n + fc + c, s * hdeg);
+      }
     }
-  // K24 (j,l) += D(i,k)
+  }
+  if (!worked) return;   // warp-uniform
+  __syncwarp();
 #pragma unroll
-  for (int b = 0; b < NB; ++b)
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      R s = 0;
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int c = 0; c < NC; ++c) s += __ldg(D + (fa + a) * n + fc + c) * Iat(a, b, c, d);
-      atomic_acc<R>(G, G32, (size_t)(fb + b) * n + fd + d, s * hdeg);
-    }
-  // K14 (i,l) += D(j,k)
-#pragma unroll
-  for (int a = 0; a < NA; ++a)
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      R s = 0;
-#pragma unroll
-      for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int c = 0; c < NC; ++c) s += __ldg(D + (fb + b) * n + fc + c) * Iat(a, b, c, d);
-      atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fd + d, s * hdeg);
-    }
-  // K23 (j,k) += D(i,l)
-#pragma unroll
-  for (int b = 0; b < NB; ++b)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      R s = 0;
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int d = 0; d < ND; ++d) s += __ldg(D + (fa + a) * n + fd + d) * Iat(a, b, c, d);
-      atomic_acc<R>(G, G32, (size_t)(fb + b) * n + fc + c, s * hdeg);
-    }
+  for (int x = 0; x < NA * NB; ++x) {
+    const R v = warp_sum(j12[x]);
+    if (threadIdx.x == 0) atomic_acc<R>(G, G32, (size_t)(fa + x / NB) * n + fb + x % NB, v);
+  }
+  if (T.count && cnt && threadIdx.x == 0) atomicAdd(T.count, (unsigned long long)cnt);
 }
 
 // ------------------------------------------------------- J/K, FP32 bra rows --
@@ -422,10 +534,10 @@ __global__ void __launch_bounds__(32 * kRowWarps) jk32_row_kernel(const JKTask *
     float I[Q::NINT];
     if (active) {
       if (soa)
-        eri_quartet_k1<float, LA, LB, LC, LD>(bra, prims + bra.prim0, ket, kprim, TL.boys.f64, TL.boys.f32, I);
+        eri_quartet_k1<float, LA, LB, LC, LD>(bra, prims + bra.prim0, ket, kprim, TL.boys.f64, TL.boys.dd, I);
       else
         eri_quartet<float, LA, LB, LC, LD>(bra, prims + bra.prim0, ket, prims + ket.prim0, TL.boys.f64,
-                                           TL.boys.f32, I);
+                                           TL.boys.dd, I);
     } else {
 #pragma unroll
       for (int x = 0; x < Q::NINT; ++x) I[x] = 0.f;
@@ -547,9 +659,14 @@ __global__ void __launch_bounds__(128) cp_tasks_kernel(const CPTask *__restrict_
   if (act == kSysFP64 && TL.mixed && TL.lower) return;   // system held in FP64: the FP64 launch takes it all
   const int local = blockIdx.x - T.blk0;
   const int tx = local % T.nbx, ty = local / T.nbx;
-  const int kpos = tx * 32 + threadIdx.x;
-  const int bpos = ty * kWarpsPerBlock + threadIdx.y;
+  const int kets = TL.tile.kets, parts = 32 / kets;
+  const int kl = threadIdx.x & (kets - 1), part = threadIdx.x / kets;
+  const int kpos = tx * kets + kl;
+  const int bpos = ty * blockDim.y + threadIdx.y;
   if (bpos >= T.nbra) return;
+  // pairs are sorted by decreasing Schwarz factor: the warp's first ket has its
+  // largest bound (with room for the FP32 rounding of the factors)
+  if (T.pa32[T.bra0 + bpos].Q * T.pb32[T.ket0 + tx * kets].Q * 1.00001f < TL.cut32) return;
   bool active = kpos < T.nket;
   {
     // |(ij|kl)| <= Q_ab Q_cd for every component (Schwarz), and raw values
@@ -575,7 +692,7 @@ __global__ void __launch_bounds__(128) cp_tasks_kernel(const CPTask *__restrict_
   }
   if (__all_sync(0xffffffffu, !active)) return;
   if (T.count) {
-    const unsigned cnt = __popc(__ballot_sync(0xffffffffu, active));
+    const unsigned cnt = __popc(__ballot_sync(0xffffffffu, active && part == 0));
     if (threadIdx.x == 0) atomicAdd(T.count, (unsigned long long)cnt);
   }
   const PairT<R> *pa, *pb;
@@ -589,8 +706,10 @@ __global__ void __launch_bounds__(128) cp_tasks_kernel(const CPTask *__restrict_
   const PairT<R> &bra = pa[T.bra0 + bpos];
   const PairT<R> ket = pb[T.ket0 + min(kpos, T.nket - 1)];
   R I[Q::NINT];
-  if (active) {
-    eri_quartet<R, LA, LB, LC, LD>(bra, pra + bra.prim0, ket, prb + ket.prim0, TL.boys.f64, TL.boys.f32, I);
+  if (active || parts > 1) {
+    eri_quartet<R, LA, LB, LC, LD>(bra, pra + bra.prim0, ket, prb + ket.prim0, TL.boys.f64, TL.boys.dd, I, part,
+                                   parts, active);
+    if (part) active = false;   // the quartet is digested by its first lane
   } else {
 #pragma unroll
     for (int x = 0; x < Q::NINT; ++x) I[x] = R(0);
@@ -671,22 +790,26 @@ template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128) it_kernel(ITParams P) {
   using Q = QClass<LA, LB, LC, LD>;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
-  if (P.triangle && blockIdx.x * 32 > blockIdx.y * kWarpsPerBlock + kWarpsPerBlock - 1) return;
-  const int kpos = blockIdx.x * 32 + threadIdx.x;
-  const int bpos = blockIdx.y * kWarpsPerBlock + threadIdx.y;
-  if (bpos >= P.nbra || kpos >= P.nket) return;
-  if (P.triangle && kpos > bpos) return;
-  const int bi = P.bra0 + bpos, ki = P.ket0 + kpos;
+  const int kets = P.kets, parts = 32 / kets, bras = blockDim.y;
+  if (P.triangle && blockIdx.x * kets > blockIdx.y * bras + bras - 1) return;
+  const int part = threadIdx.x / kets;
+  const int kpos = blockIdx.x * kets + (threadIdx.x & (kets - 1));
+  const int bpos = blockIdx.y * bras + threadIdx.y;
+  if (bpos >= P.nbra) return;   // warp-uniform
+  const int bi = P.bra0 + bpos, ki = P.ket0 + min(kpos, P.nket - 1);
   const PairRec bra = P.pa[bi];
   const PairRec ket = P.pb[ki];
   // every raw integral is bounded by Q_ab Q_cd (Schwarz) and only |v| > cut is used
-  if (!abs_above(bra.Q * ket.Q * (1.0 - 1e-9), P.cut)) return;
-  if (P.screen) {
+  bool active = kpos < P.nket && !(P.triangle && kpos > bpos) && abs_above(bra.Q * ket.Q * (1.0 - 1e-9), P.cut);
+  if (P.screen && active) {
     const double b = bra.Q * ket.Q * dnorm6(P.Dn, P.nsh, bra.sa, bra.sb, ket.sa, ket.sb);
-    if (abs_below(b, P.eps)) return;
+    if (abs_below(b, P.eps)) active = false;
   }
+  if (parts == 1 ? !active : __all_sync(0xffffffffu, !active)) return;
   double I[Q::NINT];
-  eri_quartet<double, LA, LB, LC, LD>(bra, P.pra + bra.prim0, ket, P.prb + ket.prim0, P.boys.f64, P.boys.f32, I);
+  eri_quartet<double, LA, LB, LC, LD>(bra, P.pra + bra.prim0, ket, P.prb + ket.prim0, P.boys.f64, P.boys.dd, I, part,
+                                      parts, active);
+  if (part || !active) return;
 #pragma unroll
   for (int x = 0; x < Q::NINT; ++x)
     if (!abs_above(I[x], P.cut)) I[x] = 0.0;
@@ -715,22 +838,27 @@ __global__ void __launch_bounds__(128) it_kernel(ITParams P) {
 }
 
 // ------------------------------------------------------ MP2 transform input --
-// Lane x of warp y: bra pair tile_y*4 + y, ket pair tile_x*32 + x of the batch.
+// Warp y: bra pair tile_y * bras + y; its lanes: ket pairs tile_x * kets + (lane
+// mod kets) of the batch, 32 / kets lanes each.
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128) mp2x_kernel(MXParams P) {
   using Q = QClass<LA, LB, LC, LD>;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
-  const int kpos = blockIdx.x * 32 + threadIdx.x;
-  const int bpos = blockIdx.y * kWarpsPerBlock + threadIdx.y;
-  if (bpos >= P.nbra || kpos >= P.nket) return;
-  const int bi = P.bra0 + bpos, ki = P.ket0 + kpos;
+  const int kets = P.kets, parts = 32 / kets, part = threadIdx.x / kets;
+  const int kpos = blockIdx.x * kets + (threadIdx.x & (kets - 1));
+  const int bpos = blockIdx.y * blockDim.y + threadIdx.y;
+  if (bpos >= P.nbra) return;   // warp-uniform
+  const int bi = P.bra0 + bpos, ki = P.ket0 + min(kpos, P.nket - 1);
   const PairRec bra = P.pairs[bi];
   const PairRec ket = P.kpairs[ki];
-  if (!abs_above(bra.Q * ket.Q * (1.0 - 1e-9), P.cut)) return;
-  if (P.screen && abs_below(bra.Q * ket.Q * dnorm6(P.Dn, P.nsh, bra.sa, bra.sb, ket.sa, ket.sb), P.eps)) return;
+  bool active = kpos < P.nket && abs_above(bra.Q * ket.Q * (1.0 - 1e-9), P.cut);
+  if (active && P.screen && abs_below(bra.Q * ket.Q * dnorm6(P.Dn, P.nsh, bra.sa, bra.sb, ket.sa, ket.sb), P.eps))
+    active = false;
+  if (parts == 1 ? !active : __all_sync(0xffffffffu, !active)) return;
   double I[Q::NINT];
-  eri_quartet<double, LA, LB, LC, LD>(bra, P.prims + bra.prim0, ket, P.kprims + ket.prim0, P.boys.f64, P.boys.f32,
-                                      I);
+  eri_quartet<double, LA, LB, LC, LD>(bra, P.prims + bra.prim0, ket, P.kprims + ket.prim0, P.boys.f64, P.boys.dd,
+                                      I, part, parts, active);
+  if (part || !active) return;
   const int col0 = __ldg(P.colbase + ki) - P.col_first;
   const bool two = bra.sa != bra.sb;
   const size_t n = P.n, ncol = P.ncol;

@@ -22,6 +22,7 @@ namespace lgb {
 constexpr int NPC = kNumPairClasses;
 extern const JKFn kJK64_0[NPC], kJK64_1[NPC], kJK64_2[NPC], kJK64_3[NPC], kJK64_4[NPC], kJK64_5[NPC];
 extern const JKFn kJK32_0[NPC], kJK32_1[NPC], kJK32_2[NPC], kJK32_3[NPC], kJK32_4[NPC], kJK32_5[NPC];
+extern const JKFn kJKD_0[NPC], kJKD_1[NPC], kJKD_2[NPC], kJKD_3[NPC], kJKD_4[NPC], kJKD_5[NPC];
 extern const JKFn kJKR_0[NPC], kJKR_1[NPC], kJKR_2[NPC], kJKR_3[NPC], kJKR_4[NPC], kJKR_5[NPC];
 extern const CPFn kCP64_0[NPC], kCP64_1[NPC], kCP64_2[NPC], kCP64_3[NPC], kCP64_4[NPC], kCP64_5[NPC];
 extern const CPFn kCP32_0[NPC], kCP32_1[NPC], kCP32_2[NPC], kCP32_3[NPC], kCP32_4[NPC], kCP32_5[NPC];
@@ -38,6 +39,7 @@ const MXFn kMXnone[NPC] = {};
 #define LGB_F_ROWS(X) X, X, X, X
 const JKFn *const kJK64[NPC] = {kJK64_0, kJK64_1, kJK64_2, kJK64_3, kJK64_4, kJK64_5, LGB_F_ROWS(kJKnone)};
 const JKFn *const kJK32[NPC] = {kJK32_0, kJK32_1, kJK32_2, kJK32_3, kJK32_4, kJK32_5, LGB_F_ROWS(kJKnone)};
+const JKFn *const kJKD[NPC] = {kJKD_0, kJKD_1, kJKD_2, kJKD_3, kJKD_4, kJKD_5, LGB_F_ROWS(kJKnone)};
 const JKFn *const kJKR[NPC] = {kJKR_0, kJKR_1, kJKR_2, kJKR_3, kJKR_4, kJKR_5, LGB_F_ROWS(kJKnone)};
 const CPFn *const kCP64[NPC] = {kCP64_0, kCP64_1, kCP64_2, kCP64_3, kCP64_4, kCP64_5, LGB_F_ROWS(kCPnone)};
 const CPFn *const kCP32[NPC] = {kCP32_0, kCP32_1, kCP32_2, kCP32_3, kCP32_4, kCP32_5, LGB_F_ROWS(kCPnone)};
@@ -45,29 +47,29 @@ const ITFn *const kIT[NPC] = {kIT_0, kIT_1, kIT_2, kIT_3, kIT_4, kIT_5, LGB_F_RO
 const MXFn *const kMX[NPC] = {kMX_0, kMX_1, kMX_2, kMX_3, kMX_4, kMX_5, LGB_F_ROWS(kMXnone)};
 #undef LGB_F_ROWS
 
-const dim3 kBlock(32, kWarpsPerBlock);
 // LOWDIN_GB300_ROWS=0 keeps the FP32 half of mixed builds on jk_tasks_kernel
 // (read at every launch, so a process can compare both kernels)
 bool row_rows_off() {
   const char *e = std::getenv("LOWDIN_GB300_ROWS");
   return e && e[0] == '0';
 }
-constexpr int kCoUnitsPerTile = kWarpsPerBlock * 4;   // (bra row, group of 8 kets)
 constexpr int kCoMaxSmem = 200 * 1024;                 // dynamic shared memory of a cooperative CTA
 
 struct GenClass {
   int la, lb, lc, ld;
 };
 
-// work unit u of a task-tiled launch -> task, bra position, first ket position
+// work unit u of a task-tiled launch -> task, bra position, ket positions
+// [kpos0, kpos0 + kets) and the slice of the primitive quartets
 template <typename Task>
-__device__ __forceinline__ const Task &coop_unit(const Task *tasks, int ntasks, int u, int *bpos, int *kpos0) {
-  const int blk = u / kCoUnitsPerTile, sub = u % kCoUnitsPerTile;
-  const Task &T = tasks[find_task(tasks, ntasks, blk)];
+__device__ __forceinline__ const Task &coop_unit(const Task *tasks, const TaskLaunch &TL, int u, int *bpos,
+                                                 int *kpos0, int *slice) {
+  const int blk = u / TL.tile.slices;
+  *slice = u - blk * TL.tile.slices;
+  const Task &T = tasks[find_task(tasks, TL.ntasks, blk)];
   const int local = blk - T.blk0;
-  const int tx = local % T.nbx, ty = local / T.nbx;
-  *bpos = ty * kWarpsPerBlock + sub / 4;
-  *kpos0 = tx * 32 + (sub % 4) * 8;
+  *bpos = local / T.nbx;
+  *kpos0 = (local - *bpos * T.nbx) * TL.tile.kets;
   return T;
 }
 
@@ -92,12 +94,12 @@ __device__ __forceinline__ const Task &coop_unit(const Task *tasks, int ntasks, 
 __global__ void __launch_bounds__(128) jk_coop_kernel(const JKTask *__restrict__ tasks, TaskLaunch TL, GenClass K, double *gscr) {
   LGB_COOP_PROLOGUE(K)
   const int NA = ncart(K.la), NB = ncart(K.lb), NC = ncart(K.lc), ND = ncart(K.ld);
-  for (long long u = w0; u < (long long)TL.nblocks * kCoUnitsPerTile; u += wstep) {
-    int bpos, kpos0;
-    const JKTask &T = coop_unit(tasks, TL.ntasks, (int)u, &bpos, &kpos0);
+  for (long long u = w0; u < (long long)TL.nblocks * TL.tile.slices; u += wstep) {
+    int bpos, kpos0, slice;
+    const JKTask &T = coop_unit(tasks, TL, (int)u, &bpos, &kpos0, &slice);
     const int act = system_flag(T.active);
     if (bpos >= T.nbra || act == kSysOff || (act == kSysFP64 && TL.mixed && TL.lower)) continue;
-    for (int kpos = kpos0; kpos < kpos0 + 8 && kpos < T.nket; ++kpos) {
+    for (int kpos = kpos0; kpos < kpos0 + TL.tile.kets && kpos < T.nket; ++kpos) {
       if (T.triangle && kpos > bpos) break;
       const int bi = T.bra0 + bpos, ki = T.ket0 + kpos;
       const PairRec &bra = T.pairs[bi];
@@ -111,11 +113,16 @@ __global__ void __launch_bounds__(128) jk_coop_kernel(const JKTask *__restrict__
         }
         if (act != kSysFP64 && (TL.lower ? !(b < TL.split32) : (b < TL.split32))) active = false;
       } else if (T.screen) {
+        if (T.Dnmax32 && T.pairs32[bi].Q * T.pairs32[ki].Q * __ldg(T.Dnmax32) * 1.00001f < TL.eps32) break;   // kets sorted by Q
         if (abs_below(bra.Q * ket.Q * dnorm6(T.Dn, T.nsh, bra.sa, bra.sb, ket.sa, ket.sb), TL.eps)) active = false;
       }
       if (!active) continue;   // uniform across the warp
-      if (T.count && lane == 0) atomicAdd(T.count, 1ull);
-      eri_coop(g, ct, Lo, K.la, K.lb, K.lc, K.ld, bra, T.prims, ket, T.prims, TL.boys.f64, sm);
+      if (T.count && lane == 0 && slice == 0) atomicAdd(T.count, 1ull);
+      // a slice's share of the integrals is digested by itself (the updates
+      // are linear in them)
+      if (slice >= bra.nprim * ket.nprim) continue;
+      eri_coop(g, ct, Lo, K.la, K.lb, K.lc, K.ld, bra, T.prims, ket, T.prims, TL.boys.f64, sm, nullptr, slice,
+               TL.tile.slices);
       const double deg = (bra.sa == bra.sb ? 1 : 2) * (ket.sa == ket.sb ? 1 : 2) * (bi == ki ? 1 : 2);
       const double hdeg = deg * T.hf;
       const double *__restrict__ D = T.Ds;
@@ -181,12 +188,12 @@ __global__ void __launch_bounds__(128) jk_coop_kernel(const JKTask *__restrict__
 __global__ void __launch_bounds__(128) cp_coop_kernel(const CPTask *__restrict__ tasks, TaskLaunch TL, GenClass K, double *gscr) {
   LGB_COOP_PROLOGUE(K)
   const int NA = ncart(K.la), NB = ncart(K.lb), NC = ncart(K.lc), ND = ncart(K.ld);
-  for (long long u = w0; u < (long long)TL.nblocks * kCoUnitsPerTile; u += wstep) {
-    int bpos, kpos0;
-    const CPTask &T = coop_unit(tasks, TL.ntasks, (int)u, &bpos, &kpos0);
+  for (long long u = w0; u < (long long)TL.nblocks * TL.tile.slices; u += wstep) {
+    int bpos, kpos0, slice;
+    const CPTask &T = coop_unit(tasks, TL, (int)u, &bpos, &kpos0, &slice);
     const int act = system_flag(T.active);
     if (bpos >= T.nbra || act == kSysOff || (act == kSysFP64 && TL.mixed && TL.lower)) continue;
-    for (int kpos = kpos0; kpos < kpos0 + 8 && kpos < T.nket; ++kpos) {
+    for (int kpos = kpos0; kpos < kpos0 + TL.tile.kets && kpos < T.nket; ++kpos) {
       const int bi = T.bra0 + bpos, ki = T.ket0 + kpos;
       const bool tiny = TL.mixed ? T.pa32[bi].Q * T.pb32[ki].Q * 0.999f < TL.cut32
                                        : T.pa[bi].Q * T.pb[ki].Q * (1.0 - 1e-9) < TL.cut;
@@ -518,10 +525,13 @@ bool jk_rows_used(int pcb, int pck, int n, int nsh) {
   return row_smem_bytes(ncart(pc_la(pcb)) + ncart(pc_lb(pcb)), n, nsh) <= (size_t)kRowMaxSmem;
 }
 
-cudaError_t launch_jk_tasks(int pcb, int pck, bool fp32, const JKTask *dtasks, const TaskLaunch &tl,
+bool jk_dd_class(int pcb, int pck) { return class_supported(pcb, pck) && kJKD[pcb][pck]; }
+
+cudaError_t launch_jk_tasks(int pcb, int pck, Arith arith, const JKTask *dtasks, const TaskLaunch &tl,
                             cudaStream_t s) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (tl.ntasks <= 0 || tl.nblocks <= 0) return cudaSuccess;
+  const bool fp32 = arith == Arith::f32;
   if (fp32 && tl.mixed && tl.lower && tl.rows_pref != 0 && jk_rows_used(pcb, pck, tl.rows_n, tl.rows_nsh)) {
     // the FP32 half of a mixed build: bra-row kernel
     const JKFn r = kJKR[pcb][pck];
@@ -537,13 +547,16 @@ cudaError_t launch_jk_tasks(int pcb, int pck, bool fp32, const JKTask *dtasks, c
     count_launches(1);
     return cudaGetLastError();
   }
-  const JKFn f = fp32 ? kJK32[pcb][pck] : kJK64[pcb][pck];
+  // a class without an FP32 kernel is evaluated in FP64 in the FP32 half too
+  const JKFn f = arith == Arith::dd ? kJKD[pcb][pck]
+                 : fp32 && kJK32[pcb][pck] ? kJK32[pcb][pck]
+                                           : kJK64[pcb][pck];
   if (f) {
-    f<<<tl.nblocks, kBlock, 0, s>>>(dtasks, tl);
+    f<<<tl.nblocks * tl.tile.slices, dim3(32, tl.tile.bras), 0, s>>>(dtasks, tl);
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K = gen_class(pcb, pck);
-    const CoopShape c = coop_shape(K, (long long)tl.nblocks * kCoUnitsPerTile);
+    const CoopShape c = coop_shape(K, (long long)tl.nblocks * tl.tile.slices);
     const cudaError_t e = coop_launch(jk_coop_kernel, c, s, dtasks, tl, K);
     if (e != cudaSuccess) return e;
   }
@@ -555,13 +568,13 @@ cudaError_t launch_cp_tasks(int pcb, int pck, bool fp32, const CPTask *dtasks, c
                             cudaStream_t s) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (tl.ntasks <= 0 || tl.nblocks <= 0) return cudaSuccess;
-  const CPFn f = fp32 ? kCP32[pcb][pck] : kCP64[pcb][pck];
+  const CPFn f = fp32 && kCP32[pcb][pck] ? kCP32[pcb][pck] : kCP64[pcb][pck];
   if (f) {
-    f<<<tl.nblocks, kBlock, 0, s>>>(dtasks, tl);
+    f<<<tl.nblocks, dim3(32, tl.tile.bras), 0, s>>>(dtasks, tl);
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K = gen_class(pcb, pck);
-    const CoopShape c = coop_shape(K, (long long)tl.nblocks * kCoUnitsPerTile);
+    const CoopShape c = coop_shape(K, (long long)tl.nblocks * tl.tile.slices);
     const cudaError_t e = coop_launch(cp_coop_kernel, c, s, dtasks, tl, K);
     if (e != cudaSuccess) return e;
   }
@@ -569,13 +582,15 @@ cudaError_t launch_cp_tasks(int pcb, int pck, bool fp32, const CPTask *dtasks, c
   return cudaGetLastError();
 }
 
-cudaError_t launch_it(int pcb, int pck, const ITParams &p, cudaStream_t s) {
+cudaError_t launch_it(int pcb, int pck, ITParams p, cudaStream_t s) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (p.nbra <= 0 || p.nket <= 0) return cudaSuccess;
   const ITFn f = kIT[pcb][pck];
   if (f) {
-    const dim3 grid((unsigned)((p.nket + 31) / 32), (unsigned)((p.nbra + kWarpsPerBlock - 1) / kWarpsPerBlock));
-    f<<<grid, kBlock, 0, s>>>(p);
+    const TileShape t = tile_shape({(double)p.nbra * p.nket, p.mean_prims, p.mean_prims, p.nbra, false});
+    p.kets = t.kets;
+    f<<<dim3((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras)), dim3(32, t.bras),
+        0, s>>>(p);
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K = gen_class(pcb, pck);
@@ -587,13 +602,15 @@ cudaError_t launch_it(int pcb, int pck, const ITParams &p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_mp2x(int pcb, int pck, const MXParams &p, cudaStream_t s) {
+cudaError_t launch_mp2x(int pcb, int pck, MXParams p, cudaStream_t s) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (p.nbra <= 0 || p.nket <= 0) return cudaSuccess;
   const MXFn f = kMX[pcb][pck];
   if (f) {
-    const dim3 grid((unsigned)((p.nket + 31) / 32), (unsigned)((p.nbra + kWarpsPerBlock - 1) / kWarpsPerBlock));
-    f<<<grid, kBlock, 0, s>>>(p);
+    const TileShape t = tile_shape({(double)p.nbra * p.nket, p.mean_prims, p.mean_prims, p.nbra, false});
+    p.kets = t.kets;
+    f<<<dim3((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras)), dim3(32, t.bras),
+        0, s>>>(p);
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K = gen_class(pcb, pck);
@@ -620,7 +637,7 @@ cudaError_t launch_g12(int pcb, int pck, const G12Params &p, cudaStream_t s) {
 cudaError_t launch_schwarz(int pc, const SchwarzParams &p, cudaStream_t s) {
   if (pc < 0 || pc >= kNumPairClasses) return cudaErrorNotSupported;
   if (p.np <= 0) return cudaSuccess;
-  if (2 * pc_L(pc) <= kTemplatedMaxL) {
+  if (2 * pc_L(pc) <= kTemplatedMaxL4) {
     kSZ[pc]<<<(p.np + 127) / 128, 128, 0, s>>>(p);
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;

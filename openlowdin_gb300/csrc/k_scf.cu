@@ -131,7 +131,7 @@ __global__ void boys_eval_kernel(int fp32, const double *T, int n, double *out, 
   if (i >= n) return;
   if (fp32) {
     float F[L + 1];
-    boys_f32<L>((float)T[i], F, tabs.f32);
+    boys_f32<L>((float)T[i], F, tabs.dd);
     for (int m = 0; m <= L; ++m) out[(size_t)i * (L + 1) + m] = F[m];
   } else {
     double F[L + 1];

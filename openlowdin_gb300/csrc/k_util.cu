@@ -23,11 +23,17 @@ __device__ __forceinline__ void atomic_max_nonneg(float *p, float v) {
   atomicMax(reinterpret_cast<unsigned int *>(p), (unsigned int)__float_as_int(v));
 }
 
+__device__ __forceinline__ float2 split2(double s) {
+  const float h = (float)s;
+  return make_float2(h, (float)(s - (double)h));
+}
+
 // Ds = N D N (FP64 and FP32 copies) and Dn[s1][s2] = max |D| over the shell
 // block (unscaled D)
 __global__ void prepare_density_kernel(const double *__restrict__ D, const double *__restrict__ norma,
                                        const int *__restrict__ shell_of, int n, int nsh, double *__restrict__ Ds,
-                                       float *__restrict__ Ds32, double *__restrict__ Dn, float *__restrict__ Dn32) {
+                                       float *__restrict__ Ds32, float2 *__restrict__ Dd, double *__restrict__ Dn,
+                                       float *__restrict__ Dn32) {
   const size_t nn = (size_t)n * n;
   for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < nn; x += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(x / n), j = (int)(x % n);
@@ -35,6 +41,7 @@ __global__ void prepare_density_kernel(const double *__restrict__ D, const doubl
     const double s = d * norma[i] * norma[j];
     Ds[x] = s;
     if (Ds32) Ds32[x] = (float)s;
+    if (Dd) Dd[x] = split2(s);
     const int b = shell_of[i] * nsh + shell_of[j];
     atomic_max_nonneg(Dn + b, fabs(d));
     if (Dn32) atomic_max_nonneg(Dn32 + b, (float)fabs(d));
@@ -129,6 +136,7 @@ __global__ void prepare_batch_kernel(const SpeciesSlot *__restrict__ slots, int 
     const double s = p * S.norma[i] * S.norma[j];
     S.Ds[e] = s;
     S.Ds32[e] = (float)s;
+    S.Dd[e] = split2(s);
     if (S.Gacc) {
       S.Gacc[e] = 0.0;
       S.Gacc32[e] = 0.0f;
@@ -143,34 +151,22 @@ __global__ void prepare_batch_kernel(const SpeciesSlot *__restrict__ slots, int 
   }
 }
 
-// maximum over the block (valid in thread 0)
-__device__ __forceinline__ float block_max(float m) {
-  __shared__ float part[32];
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    m = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.f;
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  }
-  return m;   // valid in thread 0
-}
-
-// largest of Dn32: block x takes columns [256 x, 256 x + 256) of the nsh x nsh
-// norms (a thread walks its column, coalesced across the block), its maximum
-// goes to *out (non-negative floats order as their bit patterns)
+// largest of Dn32 by the norms' bit patterns (non-negative floats order as
+// integers; a NaN orders above all and so keeps every tile): block x takes
+// every gridDim.x-th run of 256 norms, its maximum goes to *out.  One block
+// walking whole columns took 34 us for 512 shells, a chain of 512 loads.
 __device__ __forceinline__ void dn_max_block(const float *__restrict__ Dn32, int nsh, float *__restrict__ out) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  float m = 0.f;
-  if (s < nsh)
-    for (int t = 0; t < nsh; ++t) m = fmaxf(m, Dn32[(size_t)t * nsh + s]);
-  m = block_max(m);
-  if (threadIdx.x == 0) atomicMax(reinterpret_cast<int *>(out), __float_as_int(m));
+  const size_t nn = (size_t)nsh * nsh, step = (size_t)gridDim.x * blockDim.x;
+  int m = 0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nn; i += step)
+    m = max(m, __float_as_int(Dn32[i]));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(reinterpret_cast<int *>(out), m);
 }
 
 __global__ void dn_max_batch_kernel(const SpeciesSlot *__restrict__ slots) {
   const SpeciesSlot &S = slots[blockIdx.y];
-  if (!S.Dn32 || !S.Dnmax32 || blockIdx.x * blockDim.x >= (unsigned)S.nsh) return;
+  if (!S.Dn32 || !S.Dnmax32 || (size_t)blockIdx.x * blockDim.x >= (size_t)S.nsh * S.nsh) return;
   if (S.active && __ldg(S.active) == 0) return;
   dn_max_block(S.Dn32, S.nsh, S.Dnmax32);
 }
@@ -297,9 +293,15 @@ cudaError_t launch_prepare_batch(const SpeciesSlot *slots, int nslots, long long
   return cudaGetLastError();
 }
 
+// about four norms per thread, one block per SM at most
+static int dn_max_grid(int nsh) {
+  const long long b = ((long long)nsh * nsh + 1023) / 1024;
+  return (int)(b > 152 ? 152 : b);
+}
+
 cudaError_t launch_dn_max_batch(const SpeciesSlot *slots, int nslots, int max_nsh, cudaStream_t s) {
   if (nslots <= 0 || max_nsh <= 0) return cudaSuccess;
-  dn_max_batch_kernel<<<dim3((unsigned)((max_nsh + 255) / 256), (unsigned)nslots), 256, 0, s>>>(slots);
+  dn_max_batch_kernel<<<dim3((unsigned)dn_max_grid(max_nsh), (unsigned)nslots), 256, 0, s>>>(slots);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -307,7 +309,7 @@ cudaError_t launch_dn_max_batch(const SpeciesSlot *slots, int nslots, int max_ns
 cudaError_t launch_dn_max(const float *Dn32, int nsh, float *out, cudaStream_t s) {
   const cudaError_t e = cudaMemsetAsync(out, 0, sizeof(float), s);
   if (e != cudaSuccess) return e;
-  dn_max_kernel<<<(nsh + 255) / 256, 256, 0, s>>>(Dn32, nsh, out);
+  dn_max_kernel<<<dn_max_grid(nsh), 256, 0, s>>>(Dn32, nsh, out);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -354,15 +356,15 @@ cudaError_t measure_fma_tflops(bool fp64, double *tflops) {
 }
 
 cudaError_t launch_prepare_density(const double *D, const double *norma, const int *shell_of, int n, int nsh,
-                                   double *Ds, float *Ds32, double *Dn, float *Dn32, cudaStream_t s) {
+                                   double *Ds, float *Ds32, float2 *Dd, double *Dn, float *Dn32, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(Dn, 0, sizeof(double) * nsh * nsh, s);
   if (e != cudaSuccess) return e;
   if (Dn32) {
     e = cudaMemsetAsync(Dn32, 0, sizeof(float) * nsh * nsh, s);
     if (e != cudaSuccess) return e;
   }
-  prepare_density_kernel<<<grid_for((size_t)n * n, 256), 256, 0, s>>>(D, norma, shell_of, n, nsh, Ds, Ds32, Dn,
-                                                                      Dn32);
+  prepare_density_kernel<<<grid_for((size_t)n * n, 256), 256, 0, s>>>(D, norma, shell_of, n, nsh, Ds, Ds32, Dd,
+                                                                      Dn, Dn32);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -54,11 +54,64 @@ constexpr int kNumPairClasses = (kMaxL + 1) * (kMaxL + 2) / 2;
 __host__ __device__ constexpr int pc_la(int pc) { return pc >= 6 ? 3 : (pc >= 3 ? 2 : (pc >= 1 ? 1 : 0)); }
 __host__ __device__ constexpr int pc_lb(int pc) { return pc - pc_la(pc) * (pc_la(pc) + 1) / 2; }
 
-constexpr int kWarpsPerBlock = 4;  // bra pairs per block (one per warp); 32 kets per warp
+constexpr int kWarpsPerBlock = 4;  // most bra pairs per block (one per warp)
+
+// Tile of a class launch: `bras` warps per block, one bra pair each, and
+// `kets` ket pairs per warp.  kets = 32: one quartet per lane.  Below that
+// 32 / kets lanes share a quartet's primitive quartets (eri_quartet).  A J/K
+// launch can also deal them to `slices` blocks, each of which digests its
+// share of the integrals by itself (the updates are linear in them).  For the
+// cooperative classes a unit is one bra pair, `kets` ket pairs and one slice.
+struct TileShape {
+  int kets, bras, slices;
+  int chunk = 1;          // J/K: consecutive ket tiles of one block
+};
+// What a launch has to do: candidate quartets, their mean and largest number
+// of primitive quartets, bra pairs on grid y (limit 65535; 0: not used), and
+// whether its digestion can take a share of the integrals.
+struct LaunchLoad {
+  double quartets = 0, mean = 1, most = 1;
+  int grid_y = 0;
+  bool linear = false;
+};
+// A launch below kFillWarps (two warps per scheduler) is as long as its longest
+// quartet, so it splits quartets over as many lanes as they have primitive
+// quartets on average, over slices until no lane has more than two of the
+// longest quartet's, and puts one warp in a block.  A large one gives a lane
+// about four primitive quartets, because one lane digests for all.  Two waters
+// in a contracted basis (s 6/3/1, p 3/1, d; 50 functions): 7.2 ms with one
+// lane per quartet, 1.7 ms with the lanes alone.  Block counts stay within
+// kMaxTiles.
+constexpr double kFillWarps = 152 * 4 * 2, kMaxTiles = 1e9;
+inline int share_slices(double warps, double shares) {
+  const double room = 4 * kFillWarps / (warps > 1 ? warps : 1);
+  const double n = shares < room ? shares : room;
+  return n > 1 ? (int)n : 1;
+}
+inline TileShape tile_shape(const LaunchLoad &w) {
+  int parts = 1;
+  while (parts < 32 && 2 * parts <= (w.quartets / 32 * 2 * parts <= kFillWarps ? w.mean : w.mean / 4) &&
+         w.quartets / 64 * parts < kMaxTiles)
+    parts *= 2;
+  const double warps = w.quartets / 32 * parts;
+  const int slices = w.linear ? share_slices(warps, w.most / (2 * parts)) : 1;
+  // a block that walks ket tiles leaves at the first one its bound cannot
+  // reach and reduces its bra-block Coulomb sums once; where that would leave
+  // fewer than 32 warps per scheduler, tiles are worth more than that
+  int chunk = 1;
+  while (w.linear && chunk < 8 && warps * slices / (2 * chunk) >= 16 * kFillWarps) chunk *= 2;
+  return {32 / parts, warps * slices >= 2 * kFillWarps || w.grid_y > 65535 ? kWarpsPerBlock : 1, slices, chunk};
+}
+inline TileShape coop_tile(const LaunchLoad &w) {
+  int kets = 8;
+  while (kets > 1 && w.quartets / kets < 4 * kFillWarps) kets /= 2;
+  while (w.quartets / kets > kMaxTiles) kets *= 2;
+  return {kets, 1, w.linear ? share_slices(w.quartets / kets, w.most / 2) : 1};
+}
 
 struct BoysTables {
   const double *f64;
-  const float *f32;
+  const float *dd;        // double-float rows (boys_dd)
 };
 
 // Fields of the structure-of-arrays copy of a pair list's FP32 records
@@ -100,6 +153,7 @@ struct JKTask {
   int screen;             // Schwarz x density screening (electrons only)
   int blk0;               // first flattened block of the task
   int nbx;                // blocks along the ket axis
+  float mean_prims, most_prims;   // mean and largest number of primitive quartets
   int rblk0;              // first block of the task in a bra-row launch (one block per bra pair)
   const float *soa32;     // structure-of-arrays FP32 pair records (null: use pairs32 / prims32)
   int npairs;             // pairs in the species' list (the field stride of soa32)
@@ -115,6 +169,13 @@ struct JKTask {
   // Dnmax32 bounds every quartet bound of a tile or of a ket range after it:
   // the mixed launches leave ranges that bound cannot reach at once
   const float *Dnmax32;
+  // double-float form (null: FP64 alone): pair and primitive records, density,
+  // and tier: bound below which a quartet is evaluated in it, per unit of *Dnmax32
+  const PairRecD *pairsd;
+  const PrimRecD *primsd;
+  const float2 *Dd;
+  float2 hfd;
+  float tier;
 };
 
 // One coupling task: quartets (A pair | B pair) of two species; accumulates
@@ -146,11 +207,30 @@ struct CPTask {
   int bra0, nbra, ket0, nket;
   int nA, nB;
   int blk0, nbx;
+  float mean_prims, most_prims;   // mean and largest number of primitive quartets
 };
+
+// FP64 builds evaluate a quartet whose density-weighted bound is small against
+// the build's largest one in double-float arithmetic (dd32.cuh), on the FP32
+// pipe, and add its integrals into the same FP64 sums.  Its relative error,
+// some 2^-45, times a bound below kTierBound of the largest stays below the
+// FP64 rounding of the sums that the largest quartets go into.  Error of the
+// two-particle matrix against an 80-bit evaluation (2-norm over 2-norm), FP64
+// alone -> two tiers: 4 waters (136 functions) 3.0e-15 -> 2.8e-15, 176-function
+// chain 6.0e-15 -> 4.8e-15, 3 waters with d 3.9e-15 -> 3.6e-15, 12 protons
+// 1.6e-14 -> 1.6e-14 (the sums of eight ket tiles at a time that came with it
+// round less often).  387-function chain (5 % of the quartets above the bound):
+// 41.7 -> 18.2 ms.
+enum class Tier { all, upper, lower };
+constexpr float kTierBound = 1.f / 4096;
+// candidate quartets of a class below which one FP64 launch is shorter than two
+// launches (one water, 120 to 14,000 a class: 116 us in one, 163 us in two)
+constexpr double kTierMinQuartets = 2e5;
 
 struct TaskLaunch {
   int ntasks;
   int nblocks;            // total flattened blocks
+  TileShape tile;         // the tasks' tile
   int nrblocks;           // bra-row launches: total bra pairs of the tasks
   int rows_n, rows_nsh;   // bra-row launches: largest basis and shell count of the tasks
   int rows_pref;          // FP32 half of a mixed launch: -1 size rule, 0 jk_tasks_kernel, 1 bra-row kernel
@@ -162,6 +242,7 @@ struct TaskLaunch {
   // FP32 copies of the thresholds and the mixed flag (split > 0), so that the
   // kernels issue no FP64 conversion or comparison for them
   int mixed;
+  Tier tier;              // J/K and coupling: the quartets this launch takes
   float eps32, split32, cut32;
   BoysTables boys;
 };
@@ -190,9 +271,13 @@ using CPFn = void (*)(const CPTask *, TaskLaunch);
 struct ITParams;
 using ITFn = void (*)(ITParams);
 __host__ __device__ constexpr int pc_L(int pc) { return pc_la(pc) + pc_lb(pc); }
-// classes above this total angular momentum use the block-cooperative kernels
-// (the fully unrolled one-thread-per-quartet kernels of heavier classes spill)
-constexpr int kTemplatedMaxL = 4;
+// classes above this total angular momentum use the cooperative kernels: the
+// fully unrolled one-thread-per-quartet kernels of total 5 keep up to 1.4 KB of
+// a thread in local memory, those of (dp|dp) and (dd|pp) 10 KB
+constexpr int kTemplatedMaxL = 5;
+// the same for the kernels that have no gain from it: FP32 (heavier classes
+// are evaluated in FP64 in the FP32 half of a mixed launch too) and first quarter
+constexpr int kTemplatedMaxL4 = 4;
 
 // First-quarter transform A[nu][lam][sig] += sum_mu C_p(mu) (mu nu|lam sig).
 struct ITParams {
@@ -213,6 +298,8 @@ struct ITParams {
   double *A;
   BoysTables boys;
   double cut;             // raw values with |v| <= cut are dropped (1e-10)
+  double mean_prims;      // mean primitive quartets of a quartet
+  int kets;               // ket pairs per warp (set by the launcher)
 };
 
 // Geminal (G12) two-particle matrices for the operator sum_k c_k exp(-g_k r12^2):
@@ -268,27 +355,28 @@ struct MXParams {
   int ncol;               // columns of the batch
   double *X;              // FP64 output X[mu][col][nu], or (X null)
   __nv_bfloat16 *Xp[3];   // split-BF16 output Xt[col * Kp + nu][mu] (K-major for the tensor cores)
+  double mean_prims;      // mean primitive quartets of a quartet
+  int kets;               // ket pairs per warp (set by the launcher)
   int np;                 // pieces of the split output
   int Kp;                 // padded function count of the split layout
   BoysTables boys;
 };
 using MXFn = void (*)(MXParams);
 
-// blocks of one task (grid tile of 32 kets x kWarpsPerBlock bras)
-inline int task_nbx(int nket) { return (nket + 31) / 32; }
-inline int task_nby(int nbra) { return (nbra + kWarpsPerBlock - 1) / kWarpsPerBlock; }
-
 // launchers (every class with l <= kMaxL)
-cudaError_t launch_jk_tasks(int pcb, int pck, bool fp32, const JKTask *dtasks, const TaskLaunch &tl,
+enum class Arith { f64, f32, dd };
+cudaError_t launch_jk_tasks(int pcb, int pck, Arith arith, const JKTask *dtasks, const TaskLaunch &tl,
                             cudaStream_t s);
+// whether the class has a double-float J/K kernel
+bool jk_dd_class(int pcb, int pck);
 // whether the FP32 launch of class (pcb, pck) over species of up to n
 // functions / nsh shells runs on the bra-row kernel
 bool jk_rows_used(int pcb, int pck, int n, int nsh);
 cudaError_t launch_cp_tasks(int pcb, int pck, bool fp32, const CPTask *dtasks, const TaskLaunch &tl,
                             cudaStream_t s);
-cudaError_t launch_it(int pcb, int pck, const ITParams &p, cudaStream_t s);
+cudaError_t launch_it(int pcb, int pck, ITParams p, cudaStream_t s);
 cudaError_t launch_schwarz(int pc, const SchwarzParams &p, cudaStream_t s);
-cudaError_t launch_mp2x(int pcb, int pck, const MXParams &p, cudaStream_t s);
+cudaError_t launch_mp2x(int pcb, int pck, MXParams p, cudaStream_t s);
 // MP2 transform helpers (k_mp2.cu).  Coefficients: C[p][mu] rows are
 // orbitals; Co[mu][i] = norma[mu] C[n_frozen + i][mu] (n x o), Cv[mu][a] =
 // norma[mu] C[n_occ + a][mu] (n x v); the *32 outputs may be null.
@@ -321,11 +409,14 @@ template <typename T>
 cudaError_t launch_mp2_energy(const T *M, int o, int v, double ei, const double *eo, const double *ev, double cut,
                               double *e2, cudaStream_t s);
 bool class_supported(int pcb, int pck);
-inline bool class_generic(int pcb, int pck) { return pc_L(pcb) + pc_L(pck) > kTemplatedMaxL; }
+// whether the J/K and coupling launches of the class run on the cooperative kernels
+inline bool class_generic(int pcb, int pck) {
+  return pcb >= 6 || pck >= 6 || pc_L(pcb) + pc_L(pck) > kTemplatedMaxL;
+}
 
 // small kernels (the *32 arguments may be null)
 cudaError_t launch_prepare_density(const double *D, const double *norma, const int *shell_of, int n, int nsh,
-                                   double *Ds, float *Ds32, double *Dn, float *Dn32, cudaStream_t s);
+                                   double *Ds, float *Ds32, float2 *Dd, double *Dn, float *Dn32, cudaStream_t s);
 cudaError_t launch_scale_density(const double *D, const double *norma, int n, double *Ds, float *Ds32,
                                  cudaStream_t s);
 cudaError_t launch_symmetrize(const double *Gacc, const float *Gacc32, const double *norma, int n, double scale,
@@ -351,6 +442,7 @@ struct SpeciesSlot {
   long long off;          // prefix of n*n over the slots
   const int *active;      // the slot's system is built while *active != 0 (null: always)
   float *Dnmax32;         // largest element of Dn32 (null: not computed)
+  float2 *Dd;             // Ds in double-float
 };
 cudaError_t launch_prepare_batch(const SpeciesSlot *slots, int nslots, long long total, cudaStream_t s);
 // Dnmax32 of every slot that has Dn32 (after launch_prepare_batch; the

@@ -102,14 +102,17 @@ Lanes::~Lanes() {
 }
 
 bool Lanes::run(std::vector<Job> &jobs, cudaStream_t s) {
-  std::stable_sort(jobs.begin(), jobs.end(), [](const Job &a, const Job &b) { return a.cost > b.cost; });
+  std::stable_sort(jobs.begin(), jobs.end(), [](const Job &a, const Job &b) {
+    return a.in_order != b.in_order ? a.in_order : !a.in_order && a.cost > b.cost;
+  });
   const int lanes = set_ ? (int)std::min<size_t>(jobs.size(), kSideLanes + 1) : 1;
+  const int first = lanes > 1 && !jobs.empty() && jobs[0].in_order ? 1 : 0;   // lane 0 is s itself
   if (lanes > 1) CK(cudaEventRecord(set_->fork, s));
   double load[kSideLanes + 1] = {};
   bool used[kSideLanes + 1] = {};
   cudaError_t err = cudaSuccess;
   for (Job &j : jobs) {
-    const int k = (int)(std::min_element(load, load + lanes) - load);   // lane 0 is s itself
+    const int k = j.in_order ? 0 : (int)(std::min_element(load + first, load + lanes) - load);
     cudaStream_t q = k ? set_->s[k - 1] : s;
     if (k && !used[k]) err = cudaStreamWaitEvent(q, set_->fork, 0);
     used[k] = true;
@@ -134,22 +137,44 @@ bool Lanes::run(std::vector<Job> &jobs, cudaStream_t s) {
 // ((2n+1)(2n+3)...(2n+2k+1)) in long double.
 struct BoysHost {
   std::vector<double> f64;
-  std::vector<float> f32;
-  BoysHost() : f64((size_t)kBoysF64Size), f32((size_t)kBoysPoints * kBoysStride) {
+  std::vector<float> dd;   // double-float rows (boys_dd)
+  // F_n(T) in long double
+  static long double series(int n, long double T) {
+    long double term = 1.0L / (2 * n + 1), sum = term;
+    for (int k = 1; k < 2000; ++k) {
+      term *= 2.0L * T / (2 * n + 2 * k + 1);
+      sum += term;
+      if (term < 1e-24L * sum) break;
+    }
+    return expl(-T) * sum;
+  }
+  static void put(float *r, long double v) {
+    r[0] = (float)v;
+    r[1] = (float)(v - (long double)r[0]);
+  }
+  BoysHost() : f64((size_t)kBoysF64Size), dd(kBoysDDSize) {
     for (int i = 0; i < kBoysPoints; ++i) {
       const long double T = (long double)i * (long double)kBoysH;
       f64[(size_t)i * kBoysStride + kBoysOrders] = (double)expl(-T);
-      f32[(size_t)i * kBoysStride + kBoysOrders] = (float)expl(-T);
       for (int n = 0; n < kBoysOrders; ++n) {
-        long double term = 1.0L / (2 * n + 1), sum = term;
-        for (int k = 1; k < 2000; ++k) {
-          term *= 2.0L * T / (2 * n + 2 * k + 1);
-          sum += term;
-          if (term < 1e-24L * sum) break;
+        f64[(size_t)i * kBoysStride + n] = (double)series(n, T);
+      }
+    }
+    for (int i = 0; i < kDDPoints; ++i) {
+      const long double T = (long double)i / 32;
+      long double F[kDDMaxL + 7];
+      // the top order by the series, the others by the downward recursion
+      F[kDDMaxL + 6] = series(kDDMaxL + 6, T);
+      for (int n = kDDMaxL + 5; n >= 0; --n) F[n] = (2 * T * F[n + 1] + expl(-T)) / (2 * n + 1);
+      for (int L = 0; L <= kDDMaxL; ++L) {
+        float *row = &dd[((size_t)L * kDDPoints + i) * kDDRow];
+        long double fact = 1.0L;
+        for (int k = 0; k < 7; ++k) {
+          if (k > 0) fact *= k;
+          if (k < 4) put(row + 2 * k, F[L + k] / fact);
+          else row[4 + k] = (float)(F[L + k] / fact);
         }
-        const double v = (double)(expl(-T) * sum);
-        f64[(size_t)i * kBoysStride + n] = v;
-        f32[(size_t)i * kBoysStride + n] = (float)v;
+        put(row + 11, expl(-T));
       }
     }
     // per-order Taylor coefficients F_{L+k}(T_i) / k! and e^{-T_i}
@@ -191,7 +216,7 @@ const BoysHost &boys_host() {
 struct DeviceBoys {
   int device = -1;
   double *f64 = nullptr;
-  float *f32 = nullptr;
+  float *dd = nullptr;
 };
 std::mutex g_boys_mu;
 std::vector<DeviceBoys> g_boys;
@@ -203,19 +228,19 @@ bool device_boys(BoysTables &out) {
   for (auto &b : g_boys)
     if (b.device == dev) {
       out.f64 = b.f64;
-      out.f32 = b.f32;
+      out.dd = b.dd;
       return true;
     }
   const BoysHost &h = boys_host();
   DeviceBoys b;
   b.device = dev;
   CK(cudaMalloc(&b.f64, h.f64.size() * sizeof(double)));
-  CK(cudaMalloc(&b.f32, h.f32.size() * sizeof(float)));
+  CK(cudaMalloc(&b.dd, h.dd.size() * sizeof(float)));
   CK(cudaMemcpy(b.f64, h.f64.data(), h.f64.size() * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b.f32, h.f32.data(), h.f32.size() * sizeof(float), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(b.dd, h.dd.data(), h.dd.size() * sizeof(float), cudaMemcpyHostToDevice));
   g_boys.push_back(b);
   out.f64 = b.f64;
-  out.f32 = b.f32;
+  out.dd = b.dd;
   return true;
 }
 
@@ -385,6 +410,11 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
   // JA (from D_B) accumulates into ba.G / ba.G32, JB (from D_A) into bb.G / bb.G32
   double *JA = want_a ? ba.G : nullptr, *JB = want_b ? bb.G : nullptr;
   if (!A->ensure_all() || !B->ensure_all()) return false;
+  double pa[kNumPairClasses], pb[kNumPairClasses];
+  for (int c = 0; c < kNumPairClasses; ++c) {
+    pa[c] = A->all.prims(c);
+    pb[c] = B->all.prims(c);
+  }
   for (int cb = 0; cb < kNumPairClasses; ++cb)
     for (int ck = 0; ck < kNumPairClasses; ++ck) {
       if (!A->all.count(cb) || !B->all.count(ck)) continue;
@@ -421,6 +451,7 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
       t.nbra = A->all.count(cb);
       t.ket0 = B->all.start[ck];
       t.nket = B->all.count(ck);
+      t.mean_prims = t.most_prims = (float)(pa[cb] * pb[ck]);
       t.nA = A->nbasis;
       t.nB = B->nbasis;
       ts.add(cb, ck, t);
@@ -437,6 +468,7 @@ bool launch_cp_groups(const TaskSet<CPTask> &ts, int mode, double split, BoysTab
     TaskLaunch tl{};
     tl.ntasks = ts.cnt[c];
     tl.nblocks = ts.nblk[c];
+    tl.tile = ts.tile[c];
     tl.eps = DBL_EPSILON;
     tl.cut = 1e-10;
     tl.skip = (float)skip;
@@ -447,7 +479,8 @@ bool launch_cp_groups(const TaskSet<CPTask> &ts, int mode, double split, BoysTab
     const CPTask *d = ts.d + ts.off[c];
     auto add = [&](bool fp32) {
       if (!lanes) return launch_cp_tasks(cb, ck, fp32, d, tl, s);
-      jobs.push_back({launch_cost(cb, ck, tl.nblocks), [=](cudaStream_t q) { return launch_cp_tasks(cb, ck, fp32, d, tl, q); }});
+      jobs.push_back({launch_cost(cb, ck, tl.nblocks), fp32,
+                      [=](cudaStream_t q) { return launch_cp_tasks(cb, ck, fp32, d, tl, q); }});
       return cudaSuccess;
     };
     tl.lower = 0;
@@ -523,14 +556,14 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
   std::vector<Lanes::Job> jobs;
   auto add = [&](int cb, int ck) {
     const ITParams p = q;
-    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), [=](cudaStream_t z) { return launch_it(cb, ck, p, z); }});
+    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), false, [=](cudaStream_t z) { return launch_it(cb, ck, p, z); }});
   };
   if (intra) {
     if (!A->dD.ensure((size_t)nA * nA) || !A->dDs.ensure((size_t)nA * nA) || !A->dDn.ensure((size_t)nsh * nsh))
       return false;
     CK(cudaMemcpyAsync(A->dD.p, hD, sizeof(double) * nA * nA, cudaMemcpyHostToDevice, s));
-    CK(launch_prepare_density(A->dD.p, A->d_norma, A->d_shell_of, nA, nsh, A->dDs.p, nullptr, A->dDn.p, nullptr,
-                              s));
+    CK(launch_prepare_density(A->dD.p, A->d_norma, A->d_shell_of, nA, nsh, A->dDs.p, nullptr, nullptr,
+                              A->dDn.p, nullptr, s));
     q.Dn = A->dDn.p;
     q.screen = A->is_electron ? 1 : 0;
     q.pa = q.pb = A->sig.d;
@@ -547,6 +580,7 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
         q.ket0 = A->sig.start[ck];
         q.nket = A->sig.count(ck);
         q.triangle = cb == ck;
+        q.mean_prims = A->sig.prims(cb) * A->sig.prims(ck);
         add(cb, ck);
       }
   } else {
@@ -567,6 +601,7 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
         q.ket0 = B->all.start[ck];
         q.nket = B->all.count(ck);
         q.triangle = 0;
+        q.mean_prims = A->all.prims(cb) * B->all.prims(ck);
         add(cb, ck);
       }
   }
@@ -619,7 +654,7 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
   std::vector<Lanes::Job> jobs;
   auto add = [&](int cb, int ck) {
     const G12Params p = P;
-    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket), [=](cudaStream_t z) { return launch_g12(cb, ck, p, z); }});
+    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket), false, [=](cudaStream_t z) { return launch_g12(cb, ck, p, z); }});
   };
   if (!B) {
     CK(launch_scale_density(dD, A->d_norma, n, A->dDs.p, A->dDs32.p, s));
@@ -1174,6 +1209,7 @@ int LowdinGB300_twobody_device_noalloc(LibintInterface *lint, const double *dD, 
     ts.off[c] = (int)flat.size();
     ts.cnt[c] = (int)ts.group[c].size();
     int b = 0;
+    ts.shape(c);
     for (JKTask t : ts.group[c]) {
       ts.place(c, t, b);
       flat.push_back(t);
@@ -1191,7 +1227,7 @@ int LowdinGB300_twobody_device_noalloc(LibintInterface *lint, const double *dD, 
   }
   ts.d = dtasks;
   // the array keeps the previous call's contents: clear what accumulates
-  if (launch_prepare_density(dD, lint->d_norma, lint->d_shell_of, n, nsh, Ds, Ds32, Dn, Dn32, s) != cudaSuccess ||
+  if (launch_prepare_density(dD, lint->d_norma, lint->d_shell_of, n, nsh, Ds, Ds32, nullptr, Dn, Dn32, s) != cudaSuccess ||
       cudaMemsetAsync(Gacc, 0, sizeof(double) * n * n, s) != cudaSuccess ||
       cudaMemsetAsync(Gacc32, 0, sizeof(float) * n * n, s) != cudaSuccess ||
       cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * kNQC, s) != cudaSuccess) {

@@ -71,7 +71,13 @@ struct PairList {
   // (kSoaFields arrays of size(); null when a pair has several primitives),
   // read by the FP32 row kernels one coalesced field at a time
   float *soa32 = nullptr;
+  PairRecD *dd = nullptr;     // double-float copies
+  PrimRecD *ddp = nullptr;
   void release() {
+    if (dd) cudaFree(dd);
+    if (ddp) cudaFree(ddp);
+    dd = nullptr;
+    ddp = nullptr;
     if (d) cudaFree(d);
     if (dp) cudaFree(dp);
     if (d32) cudaFree(d32);
@@ -84,11 +90,24 @@ struct PairList {
     soa32 = nullptr;
   }
   int count(int pc) const { return start[pc + 1] - start[pc]; }
+  // mean primitive pairs of a class
+  double prims(int pc) const {
+    double n = 0;
+    for (int i = start[pc]; i < start[pc + 1]; ++i) n += h[i].nprim;
+    return count(pc) ? n / count(pc) : 1.0;
+  }
+  double most_prims(int pc) const {
+    int n = 1;
+    for (int i = start[pc]; i < start[pc + 1]; ++i) n = std::max(n, h[i].nprim);
+    return n;
+  }
   // uploads the FP64 records and their FP32 copies
   bool upload() {
     release();
     std::vector<PairRec32> h32(h.size());
     std::vector<PrimRec32> hp32(hp.size());
+    std::vector<PairRecD> hd(h.size());
+    std::vector<PrimRecD> hpd(hp.size());
     for (size_t i = 0; i < h.size(); ++i) {
       const PairRec &a = h[i];
       PairRec32 &b = h32[i];
@@ -100,6 +119,15 @@ struct PairList {
       }
       b.Q = (float)a.Q;
       b.pad = 0.f;
+      PairRecD &c = hd[i];
+      c.sa = a.sa; c.sb = a.sb; c.fa = a.fa; c.fb = a.fb; c.prim0 = a.prim0; c.nprim = a.nprim;
+      c.la = a.la; c.lb = a.lb;
+      for (int k = 0; k < 3; ++k) {
+        c.A[k] = split_double(a.A[k]);
+        c.AB[k] = split_double(a.AB[k]);
+      }
+      c.Q = split_double(a.Q);
+      c.pad = dd32(0.f);
     }
     for (size_t i = 0; i < hp.size(); ++i) {
       const PrimRec &a = hp[i];
@@ -109,8 +137,20 @@ struct PairList {
         b.P[k] = (float)a.P[k];
         b.PA[k] = (float)a.PA[k];
       }
+      PrimRecD &c = hpd[i];
+      c.p = split_double(a.p); c.inv_p = split_double(a.inv_p); c.Kt = split_double(a.Kt);
+      c.pad = dd32(0.f); c.pad2 = 0.f;
+      for (int k = 0; k < 3; ++k) {
+        c.PA[k] = split_double(a.PA[k]);
+        const dd32 h2 = split_double(a.P[k]);
+        c.P[k][0] = h2.hi;
+        c.P[k][1] = h2.lo;
+        c.P[k][2] = (float)(a.P[k] - (double)h2.hi - (double)h2.lo);
+      }
     }
-    if (!(dev_upload(d, h) && dev_upload(dp, hp) && dev_upload(d32, h32) && dev_upload(dp32, hp32))) return false;
+    if (!(dev_upload(d, h) && dev_upload(dp, hp) && dev_upload(d32, h32) && dev_upload(dp32, hp32) &&
+          dev_upload(dd, hd) && dev_upload(ddp, hpd)))
+      return false;
     bool one = !h.empty();
     for (const auto &r : h) one = one && r.nprim == 1;
     if (one) {
@@ -189,9 +229,12 @@ class Lanes {
   Lanes(const Lanes &) = delete;
   Lanes &operator=(const Lanes &) = delete;
   // runs the queued launches: costliest first, each on the lane with the
-  // least work so far, every lane ordered behind `s` and s behind every lane
+  // least work so far, every lane ordered behind `s` and s behind every lane.
+  // Launches that accumulate in FP32, whose sums depend on the order of the
+  // classes in the sixth digit, keep their order, on s
   struct Job {
     double cost;
+    bool in_order;
     std::function<cudaError_t(cudaStream_t)> launch;
   };
   bool run(std::vector<Job> &jobs, cudaStream_t s);
@@ -214,6 +257,7 @@ struct SpeciesBufs {
   float *Jp32 = nullptr;
   float *DnP32 = nullptr;
   const float *Dnmax32 = nullptr;   // largest element of Dn32, or null
+  const float2 *Dd = nullptr;       // Ds in double-float, or null (FP64 alone)
 };
 
 // Tasks grouped by quartet class (bra pair class * 6 + ket pair class); one
@@ -225,11 +269,29 @@ struct TaskSet {
   size_t cap = 0;
   int off[kNQC] = {0}, cnt[kNQC] = {0}, nblk[kNQC] = {0};
   int nrblk[kNQC] = {0}, rn[kNQC] = {0}, rnsh[kNQC] = {0};   // bra-row launches (J/K tasks)
+  TileShape tile[kNQC] = {};
+  // tile of group c from all of its tasks
+  void shape(int c) {
+    LaunchLoad w;
+    w.mean = 0;
+    w.linear = std::is_same<T, JKTask>::value;
+    for (const T &t : group[c]) {
+      double q = (double)t.nbra * t.nket;
+      if constexpr (std::is_same<T, JKTask>::value)
+        if (t.triangle) q *= 0.5;
+      w.quartets += q;
+      w.mean += q * t.mean_prims;
+      w.most = std::max(w.most, (double)t.most_prims);
+    }
+    if (w.quartets > 0) w.mean /= w.quartets;
+    tile[c] = class_generic(c / kNumPairClasses, c % kNumPairClasses) ? coop_tile(w) : tile_shape(w);
+  }
   // block offsets of task t of group c (b: blocks so far in the group)
   void place(int c, T &t, int &b) {
-    t.nbx = task_nbx(t.nket);
+    const int span = tile[c].kets * tile[c].chunk;
+    t.nbx = (t.nket + span - 1) / span;
     t.blk0 = b;
-    b += t.nbx * task_nby(t.nbra);
+    b += t.nbx * ((t.nbra + tile[c].bras - 1) / tile[c].bras);
     if constexpr (std::is_same<T, JKTask>::value) {
       t.rblk0 = nrblk[c];
       nrblk[c] += t.nbra;
@@ -239,6 +301,18 @@ struct TaskSet {
   }
   void clear() {
     for (auto &g : group) g.clear();
+  }
+  // whether every task of group c can run in two tiers
+  bool tiers(int c) const {
+    if constexpr (std::is_same<T, JKTask>::value) {
+      double q = 0;
+      for (const T &t : group[c]) {
+        if (!t.Dd || !t.Dnmax32) return false;
+        q += (double)t.nbra * t.nket;
+      }
+      return q >= kTierMinQuartets && jk_dd_class(c / kNumPairClasses, c % kNumPairClasses);
+    }
+    return false;
   }
   void add(int cb, int ck, const T &t) { group[cb * kNumPairClasses + ck].push_back(t); }
   // assigns blk0 / nbx and copies all groups to the device, ordered on stream s;
@@ -250,6 +324,7 @@ struct TaskSet {
       off[c] = (int)flat.size();
       int b = 0;
       nrblk[c] = rn[c] = rnsh[c] = 0;
+      shape(c);
       for (T t : group[c]) {
         if (on && t.active && !(*on)[t.active - flag_base]) continue;
         place(c, t, b);
@@ -312,6 +387,7 @@ struct LibintInterface {
   // 0 = FP64 (the reference's behaviour), 1 = FP32/FP64 split at abi_split
   int abi_precision = 0;
   double abi_split = 1e-5;
+  DevBuf<float2> dDd;        // scaled density in double-float
   DevBuf<double> dD, dDs, dDn, dGacc, dG, dA, dC, dDsC, dJacc;
   DevBuf<float> dDs32, dDn32, dGacc32, dDsC32, dJacc32;
   DevBuf<float> dDp32, dJp32, dDnP32;   // pair-indexed arrays of the FP32 row kernels
@@ -347,6 +423,7 @@ struct LibintInterface {
     dD.release(); dDs.release(); dDn.release(); dGacc.release(); dG.release(); dA.release(); dC.release();
     dDsC.release(); dJacc.release();
     dDs32.release(); dDn32.release(); dGacc32.release(); dDsC32.release(); dJacc32.release();
+    dDd.release();
     dDp32.release(); dJp32.release(); dDnP32.release(); dpslot.release(); dDnmax32.release();
     dcount.release();
     if (hcount) cudaFreeHost(hcount);
@@ -539,7 +616,7 @@ struct LibintInterface {
     const int n = nbasis, nsh = nshell();
     if (!dDs.ensure((size_t)n * n) || !dDn.ensure((size_t)nsh * nsh) || !dGacc.ensure((size_t)n * n) ||
         !dDs32.ensure((size_t)n * n) || !dDn32.ensure((size_t)nsh * nsh) || !dGacc32.ensure((size_t)n * n) ||
-        !dcount.ensure(kNQC))
+        !dcount.ensure(kNQC) || !dDd.ensure((size_t)n * n) || !dDnmax32.ensure(1))
       return false;
     if (!jk_ready || jk_hf != 0.5 * factor) {
       // pair-indexed arrays of the FP32 row kernels and their slot
@@ -547,7 +624,7 @@ struct LibintInterface {
       const long long pe = pair_elements(sig.start, pe_base);
       const int npairs = (int)sig.h.size();
       if (!dDp32.ensure(std::max(1LL, pe)) || !dJp32.ensure(std::max(1LL, pe)) ||
-          !dDnP32.ensure(std::max(1, npairs)) || !dpslot.ensure(1) || !dDnmax32.ensure(1))
+          !dDnP32.ensure(std::max(1, npairs)) || !dpslot.ensure(1))
         return false;
       PairSlot ps{};
       ps.pairs = sig.d32;
@@ -566,14 +643,15 @@ struct LibintInterface {
       ps.active = nullptr;
       CK(cudaMemcpyAsync(dpslot.p, &ps, sizeof(ps), cudaMemcpyHostToDevice, s));
       jk.clear();
-      SpeciesBufs b{dDs.p, dDs32.p, dDn.p, dDn32.p, dGacc.p, dGacc32.p, dDp32.p, dJp32.p, dDnP32.p, dDnmax32.p};
+      SpeciesBufs b{dDs.p, dDs32.p, dDn.p, dDn32.p, dGacc.p, dGacc32.p, dDp32.p, dJp32.p, dDnP32.p, dDnmax32.p,
+                    dDd.p};
       if (!add_jk_tasks(jk, b, 0.5 * factor, dcount.p)) return false;
       if (!jk.upload(s)) return false;
       jk_hf = 0.5 * factor;
       jk_ready = true;
     }
-    CK(launch_prepare_density(dDin, d_norma, d_shell_of, n, nsh, dDs.p, dDs32.p, dDn.p, dDn32.p, s));
-    if (precision != 0 && is_electron) CK(launch_dn_max(dDn32.p, nsh, dDnmax32.p, s));
+    CK(launch_prepare_density(dDin, d_norma, d_shell_of, n, nsh, dDs.p, dDs32.p, dDd.p, dDn.p, dDn32.p, s));
+    CK(launch_dn_max(dDn32.p, nsh, dDnmax32.p, s));
     CK(cudaMemsetAsync(dGacc.p, 0, sizeof(double) * n * n, s));
     CK(cudaMemsetAsync(dGacc32.p, 0, sizeof(float) * n * n, s));
     CK(cudaMemsetAsync(dcount.p, 0, sizeof(unsigned long long) * kNQC, s));
@@ -609,6 +687,13 @@ struct LibintInterface {
   // J/K tasks of this species into ts: one task per (bra class >= ket class)
   bool add_jk_tasks(TaskSet<JKTask> &ts, const SpeciesBufs &bf, double hf, unsigned long long *counters) {
     if (!ensure_sig()) return false;
+    double qmax = 0;   // largest Schwarz factor of the species
+    for (const PairRec &r : sig.h) qmax = std::max(qmax, r.Q);
+    double cprims[kNumPairClasses], cmost[kNumPairClasses];
+    for (int c = 0; c < kNumPairClasses; ++c) {
+      cprims[c] = sig.prims(c);
+      cmost[c] = sig.most_prims(c);
+    }
     for (int cb = 0; cb < kNumPairClasses; ++cb)
       for (int ck = 0; ck <= cb; ++ck) {
         if (!sig.count(cb) || !sig.count(ck)) continue;
@@ -635,13 +720,21 @@ struct LibintInterface {
         t.nbra = sig.count(cb);
         t.ket0 = sig.start[ck];
         t.nket = sig.count(ck);
+        t.mean_prims = (float)(cprims[cb] * cprims[ck]);
+        t.most_prims = (float)(cmost[cb] * cmost[ck]);
         t.n = nbasis;
         t.nsh = nshell();
         t.triangle = cb == ck;
         t.screen = is_electron ? 1 : 0;
         t.soa32 = sig.soa32;
         t.npairs = (int)sig.h.size();
-        t.Dnmax32 = is_electron ? bf.Dnmax32 : nullptr;
+        t.Dnmax32 = bf.Dnmax32;
+        t.pairsd = sig.dd;
+        t.primsd = sig.ddp;
+        t.Dd = bf.Dd;
+        const dd32 h = split_double(hf);
+        t.hfd = make_float2(h.hi, h.lo);
+        t.tier = (float)(qmax * qmax) * kTierBound;
         if (bf.Dp32) {
           long long pe_base[kNumPairClasses];
           pair_elements(sig.start, pe_base);
@@ -668,6 +761,7 @@ struct LibintInterface {
       tl.rows_pref = rows ? rows[c] : -1;
       tl.ntasks = ts.cnt[c];
       tl.nblocks = ts.nblk[c];
+      tl.tile = ts.tile[c];
       tl.nrblocks = ts.nrblk[c];
       tl.rows_n = ts.rn[c];
       tl.rows_nsh = ts.rnsh[c];
@@ -679,17 +773,23 @@ struct LibintInterface {
       const JKTask *d = ts.d + ts.off[c];
       tl.split = precision == 0 ? 0.0 : split;
       set_fp32_copies(tl);
-      auto add = [&](bool fp32) {
-        if (lanes)
-          jobs.push_back({launch_cost(cb, ck, tl.nblocks), [=](cudaStream_t q) { return launch_jk_tasks(cb, ck, fp32, d, tl, q); }});
-        else
-          return launch_jk_tasks(cb, ck, fp32, d, tl, s);
+      auto add = [&](Arith arith) {
+        if (!lanes) return launch_jk_tasks(cb, ck, arith, d, tl, s);
+        jobs.push_back({launch_cost(cb, ck, tl.nblocks), arith == Arith::f32,
+                        [=](cudaStream_t q) { return launch_jk_tasks(cb, ck, arith, d, tl, q); }});
         return cudaSuccess;
       };
       tl.lower = 0;
-      if (!lower_only) CK(add(false));
+      if (!lower_only) {
+        const bool tiers = ts.tiers(c);
+        tl.tier = tiers ? Tier::upper : Tier::all;
+        CK(add(Arith::f64));
+        tl.tier = Tier::lower;
+        if (tiers) CK(add(Arith::dd));
+        tl.tier = Tier::all;
+      }
       tl.lower = 1;
-      if (precision != 0) CK(add(true));
+      if (precision != 0) CK(add(Arith::f32));
     }
     return !lanes || lanes->run(jobs, s);
   }

@@ -99,6 +99,8 @@ void mp2_columns(const PairList &P, long long colB, MP2Columns &mc) {
 // integrals of every bra pair of PA against the ket pairs [k0, k1) of PB
 bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, int k1, cudaStream_t s) {
   std::vector<Lanes::Job> jobs;
+  double pa[kNumPairClasses];
+  for (int c = 0; c < kNumPairClasses; ++c) pa[c] = PA.prims(c);
   for (int ck = 0; ck < kNumPairClasses; ++ck) {
     const int ka = std::max(k0, PB.start[ck]), kb = std::min(k1, PB.start[ck + 1]);
     if (ka >= kb) continue;
@@ -108,8 +110,9 @@ bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, 
         q.nbra = std::min(PA.start[cb + 1] - b0, 65535 * kWarpsPerBlock);
         q.ket0 = ka;
         q.nket = kb - ka;
+        q.mean_prims = pa[cb] * PB.prims(ck);
         const MXParams p = q;
-        jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128),
+        jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), false,
                         [=](cudaStream_t z) { return launch_mp2x(cb, ck, p, z); }});
       }
   }
@@ -497,7 +500,7 @@ bool mp2_direct(LibintInterface *L, const double *dD, const double *dC, const do
   S.epsA = S.epsB = eps;
   // shell-block norms of D for the screening
   if (!L->dDs.ensure((size_t)n * n) || !L->dDn.ensure((size_t)nsh * nsh)) return false;
-  CK(launch_prepare_density(dD, L->d_norma, L->d_shell_of, n, nsh, L->dDs.p, nullptr, L->dDn.p, nullptr, s));
+  CK(launch_prepare_density(dD, L->d_norma, L->d_shell_of, n, nsh, L->dDs.p, nullptr, nullptr, L->dDn.p, nullptr, s));
   MXParams &q = S.q;
   q.pairs = q.kpairs = L->sig.d;
   q.prims = q.kprims = L->sig.dp;
