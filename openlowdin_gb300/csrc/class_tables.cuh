@@ -49,6 +49,12 @@ constexpr MXFn mx_entry() {
   else return nullptr;
 }
 
+template <int B, int K>
+constexpr G12Fn g12_entry() {
+  if constexpr (templated_class<B, K, kTemplatedMaxL4>()) return &g12_kernel<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
+  else return nullptr;
+}
+
 static_assert(kNumPairClasses == 10, "launch-table rows list every pair class");
 #define LGB_ROW(F, ...)                                                                                   \
   { F<__VA_ARGS__, 0>(), F<__VA_ARGS__, 1>(), F<__VA_ARGS__, 2>(), F<__VA_ARGS__, 3>(), F<__VA_ARGS__, 4>(), \
@@ -92,5 +98,9 @@ constexpr JKFn jkd_entry() {
   extern const MXFn kMX_##B[kNumPairClasses];              \
   const ITFn kIT_##B[kNumPairClasses] = LGB_ROW(it_entry, B); \
   const MXFn kMX_##B[kNumPairClasses] = LGB_ROW(mx_entry, B);
+
+#define LGB_G12_TABLE(B)                     \
+  extern const G12Fn kG12_##B[kNumPairClasses];            \
+  const G12Fn kG12_##B[kNumPairClasses] = LGB_ROW(g12_entry, B);
 
 }  // namespace lgb

@@ -39,11 +39,31 @@ struct QClass {
   static constexpr int NINT = NA * NB * NC * ND;
 };
 
+// Auxiliary integrals of the contracted Gaussian geminal sum_k c_k exp(-g_k r12^2)
+// (geminal_aux, eri_generic.cuh): F[m] = sqrt(pi)/2 sum_k c_k rho (rho+g_k)^{-3/2}
+// (g_k/(rho+g_k))^m exp(-g_k T/(rho+g_k)); gem = {count, g_0.., c_0..}
+template <int L>
+__device__ __forceinline__ void geminal_f(double rho, double T, const double *__restrict__ gem, double (&F)[L + 1]) {
+  const int n = (int)__ldg(gem);
+#pragma unroll
+  for (int m = 0; m <= L; ++m) F[m] = 0.0;
+  for (int k = 0; k < n; ++k) {
+    const double g = __ldg(gem + 1 + k), s = rsqrt(rho + g), t = s * s, r = g * t;
+    double v = 0.88622692545275801365 * __ldg(gem + 1 + n + k) * rho * t * s * exp(-r * T);
+#pragma unroll
+    for (int m = 0; m <= L; ++m) {
+      F[m] += v;
+      v *= r;
+    }
+  }
+}
+
 // Accumulate one primitive quartet into X[(e-E0)*nF + (f-F0)].
-template <typename R, int LA, int LB, int LC, int LD>
+// GEM: the operator is the geminal whose parameters boys64 points at.
+template <typename R, int LA, int LB, int LC, int LD, bool GEM = false>
 __device__ __forceinline__ void vrr_prim(R (&X)[QClass<LA, LB, LC, LD>::nE * QClass<LA, LB, LC, LD>::nF],
                                          const PrimT<R> &pb, const PrimT<R> &pk, const double *boys64,
-                                         const float *boys32) {
+                                         const float *boysd) {
   using QC_ = QClass<LA, LB, LC, LD>;
   constexpr int L = QC_::L, L2 = QC_::L2, NE = QC_::NE, NF = QC_::NF, E0 = QC_::E0, F0 = QC_::F0,
                 nF = QC_::nF;
@@ -64,7 +84,8 @@ __device__ __forceinline__ void vrr_prim(R (&X)[QClass<LA, LB, LC, LD>::nE * QCl
     PQ2 = mad(PQ, PQ, PQ2);
   }
   R F[L + 1];
-  BoysTab<R>::template eval<L>(rho * PQ2, F, boys64, boys32);
+  if constexpr (GEM) geminal_f<L>(rho, rho * PQ2, boys64, F);
+  else BoysTab<R>::template eval<L>(rho * PQ2, F, boys64, boysd);
   // 2 pi^{5/2} K_ab K_cd / (p q sqrt(p + q)) with the constants folded into Kt
   const R pref = pb.Kt * pk.Kt * rs;
   const R o2p = halved(pb.inv_p), o2q = halved(pk.inv_p), o2pq = halved(opq);
@@ -222,10 +243,10 @@ __device__ __forceinline__ void hrr_ket(const R *in, const R (&CD)[3], R *out) {
 // by shuffles, so every lane of the warp must call and ends with the whole
 // quartet; lanes with live = false add nothing.  slice / slices: only every
 // slices-th round of `parts` primitive quartets, from round `slice` on.
-template <typename R, int LA, int LB, int LC, int LD>
+template <typename R, int LA, int LB, int LC, int LD, bool GEM = false>
 __device__ __forceinline__ void eri_quartet(const PairT<R> &bra, const PrimT<R> *pbra, const PairT<R> &ket,
                                             const PrimT<R> *pket,
-                                            const double *boys64, const float *boys32,
+                                            const double *boys64, const float *boysd,
                                             R (&out)[QClass<LA, LB, LC, LD>::NINT], int part = 0, int parts = 1,
                                             bool live = true, int slice = 0, int slices = 1) {
   using QC_ = QClass<LA, LB, LC, LD>;
@@ -242,7 +263,7 @@ __device__ __forceinline__ void eri_quartet(const PairT<R> &bra, const PrimT<R> 
     }
     const PrimT<R> pb = pbra[ib];
     const PrimT<R> pk = pket[ik];
-    vrr_prim<R, LA, LB, LC, LD>(X, pb, pk, boys64, boys32);
+    vrr_prim<R, LA, LB, LC, LD, GEM>(X, pb, pk, boys64, boysd);
     ik += step;
   }
   if (parts > 1)
@@ -261,7 +282,7 @@ __device__ __forceinline__ void eri_quartet(const PairT<R> &bra, const PrimT<R> 
 // fields).
 template <typename R, int LA, int LB, int LC, int LD>
 __device__ __forceinline__ void eri_quartet_k1(const PairT<R> &bra, const PrimT<R> *pbra, const PairT<R> &ket,
-                                               const PrimT<R> &pk, const double *boys64, const float *boys32,
+                                               const PrimT<R> &pk, const double *boys64, const float *boysd,
                                                R (&out)[QClass<LA, LB, LC, LD>::NINT]) {
   using QC_ = QClass<LA, LB, LC, LD>;
   R X[QC_::nE * QC_::nF];
@@ -269,7 +290,7 @@ __device__ __forceinline__ void eri_quartet_k1(const PairT<R> &bra, const PrimT<
   for (int i = 0; i < QC_::nE * QC_::nF; ++i) X[i] = R(0);
   for (int ib = 0; ib < bra.nprim; ++ib) {
     const PrimT<R> pb = pbra[ib];
-    vrr_prim<R, LA, LB, LC, LD>(X, pb, pk, boys64, boys32);
+    vrr_prim<R, LA, LB, LC, LD>(X, pb, pk, boys64, boysd);
   }
   const R AB[3] = {bra.AB[0], bra.AB[1], bra.AB[2]};
   const R CD[3] = {ket.AB[0], ket.AB[1], ket.AB[2]};

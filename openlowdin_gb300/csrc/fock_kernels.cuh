@@ -119,6 +119,98 @@ __global__ void __launch_bounds__(128) schwarz_kernel(SchwarzParams P) {
   P.Q[P.p0 + t] = sqrt(m);
 }
 
+// The six updates of one quartet: g34 += D12 v, the exchange ones g13, g14,
+// g24, g23 += hdeg D v go to the FP64 (or FP32) accumulator, g12 += D34 v to the
+// caller's bra-block sums.
+template <typename R, int LA, int LB, int LC, int LD, typename DF, typename S>
+__device__ __forceinline__ void jk_digest(const R (&I)[QClass<LA, LB, LC, LD>::NINT], const DF &D, int n, int fa,
+                                          int fb, int fc, int fd, S deg, R hdeg, double *G, float *G32,
+                                          R (&j12)[ncart(LA) * ncart(LB)]) {
+  constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
+  // density blocks of the quartet, all asked for at once: one at a time behind
+  // the atomics before them they would cost a trip to L2 each
+  R dcd[NC][ND], dac[NA][NC], dad[NA][ND], dbc[NB][NC], dbd[NB][ND];
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int d = 0; d < ND; ++d) dcd[c][d] = D((fc + c) * n + fd + d);
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) dac[a][c] = D((fa + a) * n + fc + c);
+#pragma unroll
+    for (int d = 0; d < ND; ++d) dad[a][d] = D((fa + a) * n + fd + d);
+  }
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) dbc[b][c] = D((fb + b) * n + fc + c);
+#pragma unroll
+    for (int d = 0; d < ND; ++d) dbd[b][d] = D((fb + b) * n + fd + d);
+  }
+  auto Iat = [&](int a, int b, int c, int d) -> R { return I[((a * NB + b) * NC + c) * ND + d]; };
+  // J12: bra block, summed over this block's kets; J34
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      const R w = scaled(dcd[c][d], deg);
+      R s = R(0);
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          j12[a * NB + b] = mad(w, Iat(a, b, c, d), j12[a * NB + b]);
+          s = mad(D((fa + a) * n + fb + b), Iat(a, b, c, d), s);
+        }
+      atomic_acc<R>(G, G32, (size_t)(fc + c) * n + fd + d, scaled(s, deg));
+    }
+  // K13 (i,k) += D(j,l), K14 (i,l) += D(j,k)
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      R s = R(0);
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int d = 0; d < ND; ++d) s = mad(dbd[b][d], Iat(a, b, c, d), s);
+      atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fc + c, s * hdeg);
+    }
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      R s = R(0);
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s = mad(dbc[b][c], Iat(a, b, c, d), s);
+      atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fd + d, s * hdeg);
+    }
+  }
+  // K24 (j,l) += D(i,k), K23 (j,k) += D(i,l)
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      R s = R(0);
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s = mad(dac[a][c], Iat(a, b, c, d), s);
+      atomic_acc<R>(G, G32, (size_t)(fb + b) * n + fd + d, s * hdeg);
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      R s = R(0);
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int d = 0; d < ND; ++d) s = mad(dad[a][d], Iat(a, b, c, d), s);
+      atomic_acc<R>(G, G32, (size_t)(fb + b) * n + fc + c, s * hdeg);
+    }
+  }
+}
+
 // --------------------------------------------------------------------- J/K --
 // Warp y of a block takes bra pair tile_y * bras + y of its task and the ket
 // pairs tile_x * kets + (lane mod kets): one quartet per lane, or, for
@@ -293,7 +385,6 @@ __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) jk_ta
       if (!__any_sync(0xffffffffu, active)) continue;
     }
     worked = true;
-    const int fc = ket.fa, fd = ket.fb;
     R I[Q::NINT];
     if (active || parts > 1) {
       const PrimT<R> *kp = ket.nprim == 1 ? skp + kl : prims + ket.prim0;
@@ -302,90 +393,8 @@ __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) jk_ta
       if (part) active = false;   // the quartet is digested by its first lane
     }
     if (!active) continue;   // no warp-wide step follows inside the loop
-    // density blocks of the quartet, all asked for at once: one at a time behind
-    // the atomics before them they would cost a trip to L2 each
-    R dcd[NC][ND], dac[NA][NC], dad[NA][ND], dbc[NB][NC], dbd[NB][ND];
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int d = 0; d < ND; ++d) dcd[c][d] = D((fc + c) * n + fd + d);
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) dac[a][c] = D((fa + a) * n + fc + c);
-#pragma unroll
-      for (int d = 0; d < ND; ++d) dad[a][d] = D((fa + a) * n + fd + d);
-    }
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) dbc[b][c] = D((fb + b) * n + fc + c);
-#pragma unroll
-      for (int d = 0; d < ND; ++d) dbd[b][d] = D((fb + b) * n + fd + d);
-    }
     const auto deg = pow2<R>((bra.sa != bra.sb) + (ket.sa != ket.sb) + (bi != ki));
-    const R hdeg = scaled(hf, deg);
-    auto Iat = [&](int a, int b, int c, int d) -> R { return I[((a * NB + b) * NC + c) * ND + d]; };
-    // J12: bra block, summed over this block's kets; J34
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int d = 0; d < ND; ++d) {
-        const R w = scaled(dcd[c][d], deg);
-        R s = R(0);
-#pragma unroll
-        for (int a = 0; a < NA; ++a)
-#pragma unroll
-          for (int b = 0; b < NB; ++b) {
-            j12[a * NB + b] = mad(w, Iat(a, b, c, d), j12[a * NB + b]);
-            s = mad(D((fa + a) * n + fb + b), Iat(a, b, c, d), s);
-          }
-        atomic_acc<R>(G, G32, (size_t)(fc + c) * n + fd + d, scaled(s, deg));
-      }
-    // K13 (i,k) += D(j,l), K14 (i,l) += D(j,k)
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        R s = R(0);
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-          for (int d = 0; d < ND; ++d) s = mad(dbd[b][d], Iat(a, b, c, d), s);
-        atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fc + c, s * hdeg);
-      }
-#pragma unroll
-      for (int d = 0; d < ND; ++d) {
-        R s = R(0);
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-          for (int c = 0; c < NC; ++c) s = mad(dbc[b][c], Iat(a, b, c, d), s);
-        atomic_acc<R>(G, G32, (size_t)(fa + a) * n + fd + d, s * hdeg);
-      }
-    }
-    // K24 (j,l) += D(i,k), K23 (j,k) += D(i,l)
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-#pragma unroll
-      for (int d = 0; d < ND; ++d) {
-        R s = R(0);
-#pragma unroll
-        for (int a = 0; a < NA; ++a)
-#pragma unroll
-          for (int c = 0; c < NC; ++c) s = mad(dac[a][c], Iat(a, b, c, d), s);
-        atomic_acc<R>(G, G32, (size_t)(fb + b) * n + fd + d, s * hdeg);
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        R s = R(0);
-#pragma unroll
-        for (int a = 0; a < NA; ++a)
-#pragma unroll
-          for (int d = 0; d < ND; ++d) s = mad(dad[a][d], Iat(a, b, c, d), s);
-        atomic_acc<R>(G, G32, (size_t)(fb + b) * n + fc + c, s * hdeg);
-      }
-    }
+    jk_digest<R, LA, LB, LC, LD>(I, D, n, fa, fb, ket.fa, ket.fb, deg, scaled(hf, deg), G, G32, j12);
   }
   if (!worked) return;   // warp-uniform
   __syncwarp();
@@ -763,6 +772,67 @@ __global__ void __launch_bounds__(128) cp_tasks_kernel(const CPTask *__restrict_
         atomic_acc<R>(T.JB, T.JB32, (size_t)(fc + c) * nB + fd + d, s);
         if (cddiff) atomic_acc<R>(T.JB, T.JB32, (size_t)(fd + d) * nB + fc + c, s);
       }
+  }
+}
+
+// ----------------------------------------------------------- geminal (G12) --
+// Matrices of a geminal pair potential, one quartet per lane over the launch's
+// bra x ket pairs (no screening): the six updates of one species, or J of the
+// bra species with raw |v| < cut dropped.  FP64 bound (an exponential and a
+// reciprocal square root per term and primitive quartet); two waters (68
+// functions, three terms): 3.10 ms with one quartet per warp on the cooperative
+// kernel, 0.20 ms so.
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(128) g12_kernel(G12Params P) {
+  using Q = QClass<LA, LB, LC, LD>;
+  constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
+  const int kets = P.kets, parts = 32 / kets, part = threadIdx.x / kets, bras = blockDim.y;
+  if (P.triangle && blockIdx.x * kets > blockIdx.y * bras + bras - 1) return;
+  const int kpos = blockIdx.x * kets + (threadIdx.x & (kets - 1));
+  const int bpos = blockIdx.y * bras + threadIdx.y;
+  if (bpos >= P.nbra) return;   // warp-uniform
+  bool active = kpos < P.nket && !(P.triangle && kpos > bpos);
+  if (!__any_sync(0xffffffffu, active)) return;
+  const int bi = P.bra0 + bpos, ki = P.ket0 + min(kpos, P.nket - 1);
+  const PairRec &bra = P.pa[bi];
+  const PairRec &ket = P.pb[ki];
+  double I[Q::NINT];
+  eri_quartet<double, LA, LB, LC, LD, true>(bra, P.pra + bra.prim0, ket, P.prb + ket.prim0, P.gem, nullptr, I, part,
+                                            parts, active);
+  if (part) active = false;   // the quartet is digested by its first lane
+  const int fa = bra.fa, fb = bra.fb, fc = ket.fa, fd = ket.fb, n = P.n;
+  double j12[NA * NB];
+#pragma unroll
+  for (int x = 0; x < NA * NB; ++x) j12[x] = 0.0;
+  if (active) {
+    if (P.intra) {
+      const double deg = pow2<double>((bra.sa != bra.sb) + (ket.sa != ket.sb) + (bi != ki));
+      jk_digest<double, LA, LB, LC, LD>(I, [&](int i) { return __ldg(P.Ds + i); }, n, fa, fb, fc, fd, deg, P.hf * deg,
+                                        P.Gacc, nullptr, j12);
+    } else {
+      const double two = ket.sa != ket.sb ? 2.0 : 1.0;
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+          const double w = two * __ldg(P.Ds + (size_t)(fc + c) * P.nB + fd + d);
+#pragma unroll
+          for (int x = 0; x < NA * NB; ++x) {
+            const double v = I[(x * NC + c) * ND + d];
+            if (!abs_below(v, P.cut)) j12[x] = fma(w, v, j12[x]);
+          }
+        }
+    }
+  }
+  __syncwarp();
+  const bool both = !P.intra && bra.sa != bra.sb;
+#pragma unroll
+  for (int x = 0; x < NA * NB; ++x) {
+    const double v = warp_sum(j12[x]);
+    if (threadIdx.x == 0) {
+      atomicAdd(P.Gacc + (size_t)(fa + x / NB) * n + fb + x % NB, v);
+      if (both) atomicAdd(P.Gacc + (size_t)(fb + x % NB) * n + fa + x / NB, v);
+    }
   }
 }
 

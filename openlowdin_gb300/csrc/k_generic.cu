@@ -27,6 +27,7 @@ extern const JKFn kJKR_0[NPC], kJKR_1[NPC], kJKR_2[NPC], kJKR_3[NPC], kJKR_4[NPC
 extern const CPFn kCP64_0[NPC], kCP64_1[NPC], kCP64_2[NPC], kCP64_3[NPC], kCP64_4[NPC], kCP64_5[NPC];
 extern const CPFn kCP32_0[NPC], kCP32_1[NPC], kCP32_2[NPC], kCP32_3[NPC], kCP32_4[NPC], kCP32_5[NPC];
 extern const ITFn kIT_0[NPC], kIT_1[NPC], kIT_2[NPC], kIT_3[NPC], kIT_4[NPC], kIT_5[NPC];
+extern const G12Fn kG12_0[NPC], kG12_1[NPC], kG12_2[NPC], kG12_3[NPC], kG12_4[NPC], kG12_5[NPC];
 extern const MXFn kMX_0[NPC], kMX_1[NPC], kMX_2[NPC], kMX_3[NPC], kMX_4[NPC], kMX_5[NPC];
 
 namespace {
@@ -36,6 +37,7 @@ const JKFn kJKnone[NPC] = {};
 const CPFn kCPnone[NPC] = {};
 const ITFn kITnone[NPC] = {};
 const MXFn kMXnone[NPC] = {};
+const G12Fn kG12none[NPC] = {};
 #define LGB_F_ROWS(X) X, X, X, X
 const JKFn *const kJK64[NPC] = {kJK64_0, kJK64_1, kJK64_2, kJK64_3, kJK64_4, kJK64_5, LGB_F_ROWS(kJKnone)};
 const JKFn *const kJK32[NPC] = {kJK32_0, kJK32_1, kJK32_2, kJK32_3, kJK32_4, kJK32_5, LGB_F_ROWS(kJKnone)};
@@ -45,6 +47,7 @@ const CPFn *const kCP64[NPC] = {kCP64_0, kCP64_1, kCP64_2, kCP64_3, kCP64_4, kCP
 const CPFn *const kCP32[NPC] = {kCP32_0, kCP32_1, kCP32_2, kCP32_3, kCP32_4, kCP32_5, LGB_F_ROWS(kCPnone)};
 const ITFn *const kIT[NPC] = {kIT_0, kIT_1, kIT_2, kIT_3, kIT_4, kIT_5, LGB_F_ROWS(kITnone)};
 const MXFn *const kMX[NPC] = {kMX_0, kMX_1, kMX_2, kMX_3, kMX_4, kMX_5, LGB_F_ROWS(kMXnone)};
+const G12Fn *const kG12[NPC] = {kG12_0, kG12_1, kG12_2, kG12_3, kG12_4, kG12_5, LGB_F_ROWS(kG12none)};
 #undef LGB_F_ROWS
 
 // LOWDIN_GB300_ROWS=0 keeps the FP32 half of mixed builds on jk_tasks_kernel
@@ -242,8 +245,9 @@ __global__ void __launch_bounds__(128) cp_coop_kernel(const CPTask *__restrict__
 }
 
 // ---------------------------------------------------------- geminal (G12) --
-// Every class runs here (the geminal matrices are not a hot path): one quartet
-// per warp, all quartets of the launch's bra x ket pair ranges, no screening.
+// The classes without a templated kernel (total angular momentum above 4, f
+// shells): one quartet per warp, all quartets of the launch's bra x ket pair
+// ranges, no screening.
 __global__ void __launch_bounds__(128) g12_coop_kernel(G12Params P, GenClass K, double *gscr) {
   LGB_COOP_PROLOGUE(K)
   const int NA = ncart(K.la), NB = ncart(K.lb), NC = ncart(K.lc), ND = ncart(K.ld);
@@ -622,9 +626,18 @@ cudaError_t launch_mp2x(int pcb, int pck, MXParams p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_g12(int pcb, int pck, const G12Params &p, cudaStream_t s) {
+cudaError_t launch_g12(int pcb, int pck, G12Params p, cudaStream_t s) {
   if (!class_supported(pcb, pck) || !p.gem) return cudaErrorNotSupported;
   if (p.nbra <= 0 || p.nket <= 0) return cudaSuccess;
+  const TileShape t = tile_shape({(double)p.nbra * p.nket, p.mean_prims, p.mean_prims, p.nbra, false});
+  const G12Fn f = kG12[pcb][pck];
+  if (f && (p.nbra + t.bras - 1) / t.bras <= 65535) {
+    p.kets = t.kets;
+    f<<<dim3((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras)), dim3(32, t.bras),
+        0, s>>>(p);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   if (!coop_ready()) return cudaErrorInvalidValue;
   const GenClass K = gen_class(pcb, pck);
   const CoopShape c = coop_shape(K, (long long)p.nbra * p.nket);

@@ -321,8 +321,11 @@ struct G12Params {
   double hf;              // 0.5 * exchange factor (intra)
   double cut;             // coupling: raw values with |v| < cut are dropped (1e-10)
   const double *gem;      // {count, exponents..., coefficients...} in device memory
+  double mean_prims;      // mean primitive quartets of a quartet
+  int kets;               // ket pairs per warp (set by the launcher)
 };
-cudaError_t launch_g12(int pcb, int pck, const G12Params &p, cudaStream_t s);
+using G12Fn = void (*)(G12Params);
+cudaError_t launch_g12(int pcb, int pck, G12Params p, cudaStream_t s);
 
 struct SchwarzParams {
   const PairRec *pairs;

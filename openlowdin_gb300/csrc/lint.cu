@@ -673,6 +673,7 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
         P.ket0 = A->sig.start[ck];
         P.nket = A->sig.count(ck);
         P.triangle = cb == ck;
+        P.mean_prims = A->sig.prims(cb) * A->sig.prims(ck);
         add(cb, ck);
       }
     {
@@ -701,6 +702,7 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
       P.nbra = A->all.count(cb);
       P.ket0 = B->all.start[ck];
       P.nket = B->all.count(ck);
+      P.mean_prims = A->all.prims(cb) * B->all.prims(ck);
       add(cb, ck);
     }
   {
