@@ -1,11 +1,16 @@
 // One-electron matrices on the device: overlap S, kinetic T and the
-// point-charge potential V = sum_C Z_C <a|1/|r - C||b> of one species, one
-// thread per unordered shell pair, Obara-Saika recursions (1-D overlap tables
-// for S and T; the vertical recursion with Boys values and a horizontal
-// transfer for V), written normalised (norma_i norma_j) to both (i, j) and
-// (j, i).  Same formulas as the host blocks the library's
-// LibintInterface_compute_1body_ints uses (ContractedGaussian / Overlap /
-// Kinetic / Attraction integrals of the reference, src/ints/*.f90).
+// point-charge potential V = sum_C Z_C <a|1/|r - C||b> of one species,
+// Obara-Saika recursions (1-D overlap tables for S and T; the vertical recursion
+// with Boys values and a horizontal transfer for V), written normalised
+// (norma_i norma_j) to both (i, j) and (j, i).  S and T: one thread per unordered
+// shell pair.  V of s, p and d shells: potential_kernel, a group of lanes per
+// pair with the charges dealt to them and every index a compile-time constant.
+// V is FP64 bound and grows with the charges: for a 387-function chain and its
+// nuclei one thread per pair with run-time indices took 326 us in 244 blocks,
+// all launches together now take 185.  Same formulas as the host blocks the
+// library's LibintInterface_compute_1body_ints uses (ContractedGaussian /
+// Overlap / Kinetic / Attraction integrals of the reference, src/ints/*.f90).
+#include "eri.cuh"
 #include "eri_generic.cuh"
 #include "kernels.cuh"
 
@@ -13,6 +18,92 @@ namespace lgb {
 namespace {
 
 constexpr int kOneMaxL = kMaxL + 2;   // kinetic needs j + 2
+constexpr int kPotMaxL = 2;           // shells of potential_kernel
+
+// V of the class (LA LB), LA >= LB: `lanes` (a power of two) neighbouring lanes
+// per pair, lane g taking charges g, g + lanes, ...; shells of angular momentum
+// l are P.order[P.lstart[l]] .. P.order[P.lstart[l + 1] - 1]
+template <int LA, int LB>
+__global__ void __launch_bounds__(128) potential_kernel(OneBodyParams P, int lanes) {
+  constexpr int L = LA + LB, NE = coff(L + 1), E0 = coff(LA), nE = NE - E0, NA = ncart(LA), NB = ncart(LB);
+  const int na = P.lstart[LA + 1] - P.lstart[LA], nb = P.lstart[LB + 1] - P.lstart[LB];
+  const int npair = LA == LB ? na * (na + 1) / 2 : na * nb;
+  const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / lanes), g = threadIdx.x & (lanes - 1);
+  const int q = min(t, npair - 1);   // every lane takes part in the shuffles
+  int ia, ib;
+  if constexpr (LA == LB) {
+    ia = (int)((sqrtf(8.f * q + 1.f) - 1.f) * 0.5f);
+    while (ia * (ia + 1) / 2 > q) --ia;
+    while ((ia + 1) * (ia + 2) / 2 <= q) ++ia;
+    ib = q - ia * (ia + 1) / 2;
+  } else {
+    ia = q / nb;
+    ib = q - ia * nb;
+  }
+  const int s1 = P.order[P.lstart[LA] + ia], s2 = P.order[P.lstart[LB] + ib];
+  const DevShell A = P.shells[s1], B = P.shells[s2];
+  double AB[3], AB2 = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    AB[d] = A.O[d] - B.O[d];
+    AB2 = fma(AB[d], AB[d], AB2);
+  }
+  double X[nE];
+#pragma unroll
+  for (int e = 0; e < nE; ++e) X[e] = 0.0;
+  for (int pa = 0; pa < A.nprim; ++pa)
+    for (int pb = 0; pb < B.nprim; ++pb) {
+      const double a = P.alpha[A.p0 + pa], b = P.alpha[B.p0 + pb], p = a + b, op = 1.0 / p, o2p = 0.5 * op;
+      const double w = P.cn[A.p0 + pa] * P.cn[B.p0 + pb] * exp(-a * b * op * AB2) * (2.0 * 3.14159265358979323846) * op;
+      double Pc[3], PA[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        Pc[d] = (a * A.O[d] + b * B.O[d]) * op;
+        PA[d] = Pc[d] - A.O[d];
+      }
+      for (int c = g; c < P.ncharge; c += lanes) {
+        double PC[3], PC2 = 0, F[L + 1];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          PC[d] = Pc[d] - __ldg(P.R + 3 * c + d);
+          PC2 = fma(PC[d], PC[d], PC2);
+        }
+        boys_f64<L>(p * PC2, F, P.boys.f64);
+        double W[NE][L + 1];
+#pragma unroll
+        for (int m = 0; m <= L; ++m) W[0][m] = F[m];
+        sfor<1, NE>([&](auto ec) {
+          constexpr int e = decltype(ec)::value;
+          constexpr int d = cdir(e), em = cminus(e, d), ei = ccomp(e, d) - 1;
+          constexpr int emm = ei > 0 ? cminus(em, d) : 0;
+#pragma unroll
+          for (int m = 0; m <= L - clevel(e); ++m) {
+            double v = PA[d] * W[em][m] - PC[d] * W[em][m + 1];
+            if constexpr (ei > 0) v += ei * o2p * (W[emm][m] - W[emm][m + 1]);
+            W[e][m] = v;
+          }
+        });
+        const double zw = __ldg(P.Z + c) * w;
+        sfor<E0, NE>([&](auto ec) {
+          constexpr int e = decltype(ec)::value;
+          X[e - E0] = fma(zw, W[e][0], X[e - E0]);
+        });
+      }
+    }
+  for (int o = 1; o < lanes; o <<= 1)
+#pragma unroll
+    for (int e = 0; e < nE; ++e) X[e] += __shfl_xor_sync(0xffffffffu, X[e], o);
+  if (t >= npair || g) return;
+  double V[NA * NB];
+  hrr<double, LA, LB, 1>(X, AB, V);
+  const int fa = P.first[s1], fb = P.first[s2];
+  const size_t n = P.n;
+#pragma unroll
+  for (int x = 0; x < NA * NB; ++x) {
+    const int i = fa + x / NB, j = fb + x % NB;
+    P.V[i * n + j] = P.V[j * n + i] = V[x] * P.norma[i] * P.norma[j];
+  }
+}
 
 __device__ void ovl1d_dev(int li, int lj, double PA, double PB, double o2p, double s[kMaxL + 1][kOneMaxL + 1]) {
   for (int i = 0; i <= li; ++i)
@@ -32,18 +123,21 @@ __device__ void ovl1d_dev(int li, int lj, double PA, double PB, double o2p, doub
     }
 }
 
+// S and T of every pair, and (WITHV) V of the pairs with an f shell
+template <bool WITHV>
 __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int npair = P.nsh * (P.nsh + 1) / 2;
   if (t >= npair) return;
   // t -> (s1 >= s2)
-  int s1 = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
+  int s1 = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
   while (s1 * (s1 + 1) / 2 > t) --s1;
   while ((s1 + 1) * (s1 + 2) / 2 <= t) ++s1;
   const int s2 = t - s1 * (s1 + 1) / 2;
   const DevShell A = P.shells[s1], B = P.shells[s2];
   const CartInfo *ct = kCartTable.e;
   const int la = A.l, lb = B.l, n1 = ncart(la), n2 = ncart(lb);
+  const bool dov = WITHV && (la > kPotMaxL || lb > kPotMaxL);
   constexpr int kNC2 = ncart(kMaxL) * ncart(kMaxL);
   double S[kNC2], T[kNC2], V[kNC2];
   for (int k = 0; k < n1 * n2; ++k) S[k] = T[k] = V[k] = 0.0;
@@ -55,7 +149,8 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
   // potential: vertical recursion on the bra up to la + lb, then transfer
   const int L = la + lb, NE = coff(L + 1), E0 = coff(la), M = L + 1;
   double W[coff(2 * kMaxL + 1) * (2 * kMaxL + 1)], X[coff(2 * kMaxL + 1)];
-  for (int e = 0; e < NE - E0; ++e) X[e] = 0.0;
+  if (dov)
+    for (int e = 0; e < NE - E0; ++e) X[e] = 0.0;
   for (int pa = 0; pa < A.nprim; ++pa)
     for (int pb = 0; pb < B.nprim; ++pb) {
       const double a = P.alpha[A.p0 + pa], b = P.alpha[B.p0 + pb], p = a + b, o2p = 0.5 / p;
@@ -87,7 +182,7 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
           }
         }
       }
-      if (P.V) {
+      if (dov) {
         const double w = cab * 2.0 * 3.14159265358979323846 / p;
         for (int c = 0; c < P.ncharge; ++c) {
           double PC[3], PC2 = 0, F[kGenMaxL + 1];
@@ -114,7 +209,7 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
         }
       }
     }
-  if (P.V) {
+  if (dov) {
     // horizontal transfer (a, b+1_i| = (a+1_i, b| + AB_i (a, b| over lb
     // levels: level j has rows over totals la .. la + lb - j (the last level
     // only la) and ncart(j) columns; it reads level j - 1 (X for j = 1)
@@ -146,7 +241,7 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
       const int k = f1 * n2 + f2;
       if (P.S) P.S[i * n + j] = P.S[j * n + i] = S[k] * nn;
       if (P.T) P.T[i * n + j] = P.T[j * n + i] = T[k] * nn;
-      if (P.V) P.V[i * n + j] = P.V[j * n + i] = V[k] * nn;
+      if (dov) P.V[i * n + j] = P.V[j * n + i] = V[k] * nn;
     }
 }
 
@@ -155,9 +250,33 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
 cudaError_t launch_one_body(const OneBodyParams &p, cudaStream_t s) {
   const int npair = p.nsh * (p.nsh + 1) / 2;
   if (npair <= 0) return cudaSuccess;
-  one_body_kernel<<<(npair + 127) / 128, 128, 0, s>>>(p);
+  const bool heavy = p.V && p.ncharge > 0 && p.lstart[kPotMaxL + 1] < p.nsh;
+  if (heavy) one_body_kernel<true><<<(npair + 127) / 128, 128, 0, s>>>(p);
+  else if (p.S || p.T) one_body_kernel<false><<<(npair + 127) / 128, 128, 0, s>>>(p);
+  else return cudaSuccess;
   count_launches(1);
   return cudaGetLastError();
+}
+
+cudaError_t launch_potential(int pc, const OneBodyParams &p, cudaStream_t s) {
+  using Fn = void (*)(OneBodyParams, int);
+  static const Fn fn[6] = {&potential_kernel<0, 0>, &potential_kernel<1, 0>, &potential_kernel<1, 1>,
+                           &potential_kernel<2, 0>, &potential_kernel<2, 1>, &potential_kernel<2, 2>};
+  static_assert(kPotMaxL == 2, "one entry per class of potential_kernel");
+  const long long npair = potential_pairs(pc, p);
+  if (npair <= 0 || p.ncharge <= 0) return cudaSuccess;
+  // lanes per pair: up to four warps per scheduler, no more than there are charges
+  int lanes = 1;
+  while (lanes < 32 && 2 * lanes <= p.ncharge && npair / 32 * lanes < 2 * (long long)kFillWarps) lanes *= 2;
+  fn[pc]<<<(unsigned)((npair * lanes + 127) / 128), 128, 0, s>>>(p, lanes);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+long long potential_pairs(int pc, const OneBodyParams &p) {
+  if (pc < 0 || pc >= 6) return 0;
+  const long long na = p.lstart[pc_la(pc) + 1] - p.lstart[pc_la(pc)], nb = p.lstart[pc_lb(pc) + 1] - p.lstart[pc_lb(pc)];
+  return pc_la(pc) == pc_lb(pc) ? na * (na + 1) / 2 : na * nb;
 }
 
 }  // namespace lgb

@@ -548,6 +548,8 @@ struct OneBodyParams {
   const DevShell *shells;
   const double *alpha, *cn;   // per primitive: exponent, coefficient x primitive norm
   const int *first;           // first function of each shell
+  const int *order;           // shells by angular momentum: those of l at order[lstart[l]] ...
+  int lstart[kMaxL + 2];
   const double *norma;
   int nsh, n;
   int ncharge;
@@ -555,7 +557,11 @@ struct OneBodyParams {
   double *S, *T, *V;          // n x n outputs (any may be null)
   BoysTables boys;
 };
+// S and T, and V of the pairs with an f shell
 cudaError_t launch_one_body(const OneBodyParams &p, cudaStream_t s);
+// V of a pair class of s, p and d shells, and its number of pairs (0 for other classes)
+cudaError_t launch_potential(int pc, const OneBodyParams &p, cudaStream_t s);
+long long potential_pairs(int pc, const OneBodyParams &p);
 
 // x[i] = deterministic pseudo-random values in [-1, 1) (benchmark operands)
 cudaError_t launch_fill_hash(float *x, long long n, unsigned seed, cudaStream_t s);

@@ -1018,6 +1018,8 @@ int LowdinGB300_one_body_device(LibintInterface *lint, int ncharge, const double
   p.alpha = lint->d_alpha;
   p.cn = lint->d_cn;
   p.first = lint->d_first;
+  p.order = lint->d_order;
+  std::copy(lint->lstart, lint->lstart + kMaxL + 2, p.lstart);
   p.norma = lint->d_norma;
   p.nsh = lint->nshell();
   p.n = lint->nbasis;
@@ -1039,12 +1041,14 @@ int LowdinGB300_one_body_device(LibintInterface *lint, int ncharge, const double
   } else if (dV) {
     if (cudaMemsetAsync(dV, 0, sizeof(double) * lint->nbasis * lint->nbasis, s) != cudaSuccess) return -1;
   }
-  const cudaError_t e = launch_one_body(p, s);
-  if (e != cudaSuccess) {
-    set_error("%s: %s", __func__, cudaGetErrorString(e));
-    return -1;
-  }
-  return 0;
+  std::vector<Lanes::Job> jobs;
+  jobs.push_back({(double)p.nsh * p.nsh, false, [=](cudaStream_t q) { return launch_one_body(p, q); }});
+  for (int pc = 0; p.V && p.ncharge > 0 && pc < kNumPairClasses; ++pc)
+    if (potential_pairs(pc, p) > 0)
+      jobs.push_back({(double)potential_pairs(pc, p) * p.ncharge * ncart(pc_la(pc)) * ncart(pc_lb(pc)), false,
+                      [=](cudaStream_t q) { return launch_potential(pc, p, q); }});
+  Lanes lanes(s);
+  return lanes.run(jobs, s) ? 0 : -1;
 }
 
 int LowdinGB300_set_precision(LibintInterface *lint, int precision, double split) {

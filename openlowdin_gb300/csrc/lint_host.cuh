@@ -381,6 +381,8 @@ struct LibintInterface {
   DevShell *d_shells = nullptr;
   double *d_alpha = nullptr, *d_cn = nullptr;
   int *d_first = nullptr;
+  int *d_order = nullptr;      // shells by angular momentum, and where each begins
+  int lstart[kMaxL + 2] = {0};
   DevBuf<double> dZR;          // point charges and positions of the last one-body call
   DevBuf<double> dGem;         // geminal parameters of the last G12 call {count, exponents, coefficients}
   // precision of LibintInterface_compute_2body_direct (LowdinGB300_set_precision):
@@ -411,13 +413,15 @@ struct LibintInterface {
     all.release();
     if (d_norma) cudaFree(d_norma);
     if (d_shell_of) cudaFree(d_shell_of);
-    for (void *q : {(void *)d_shells, (void *)d_alpha, (void *)d_cn, (void *)d_first})
+    for (void *q : {(void *)d_shells, (void *)d_alpha, (void *)d_cn, (void *)d_first,
+                    (void *)d_order})
       if (q) cudaFree(q);
     d_norma = nullptr;
     d_shell_of = nullptr;
     d_shells = nullptr;
     d_alpha = d_cn = nullptr;
     d_first = nullptr;
+    d_order = nullptr;
     dZR.release();
     dGem.release();
     dD.release(); dDs.release(); dDn.release(); dGacc.release(); dG.release(); dA.release(); dC.release();
@@ -477,6 +481,12 @@ struct LibintInterface {
     if (!dev_upload(d_shells, ds) || !dev_upload(d_alpha, al) || !dev_upload(d_cn, cn) ||
         !dev_upload(d_first, first))
       return false;
+    std::vector<int> order(nshell());
+    for (int k = 0; k < nshell(); ++k) order[k] = k;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return shells[x].l < shells[y].l; });
+    for (int l = 0; l <= kMaxL + 1; ++l)
+      lstart[l] = (int)std::count_if(shells.begin(), shells.end(), [&](const HostShell &h) { return h.l < l; });
+    if (!dev_upload(d_order, order)) return false;
     have_sig = have_all = false;
     jk_ready = false;
     dirty = false;
