@@ -7,7 +7,7 @@
 // pair with the charges dealt to them and every index a compile-time constant.
 // V is FP64 bound and grows with the charges: for a 387-function chain and its
 // nuclei one thread per pair with run-time indices took 326 us in 244 blocks,
-// all launches together now take 185.  Same formulas as the host blocks the
+// all launches together now take 226.  Same formulas as the host blocks the
 // library's LibintInterface_compute_1body_ints uses (ContractedGaussian /
 // Overlap / Kinetic / Attraction integrals of the reference, src/ints/*.f90).
 #include "eri.cuh"
@@ -20,88 +20,106 @@ namespace {
 constexpr int kOneMaxL = kMaxL + 2;   // kinetic needs j + 2
 constexpr int kPotMaxL = 2;           // shells of potential_kernel
 
-// V of the class (LA LB), LA >= LB: `lanes` (a power of two) neighbouring lanes
-// per pair, lane g taking charges g, g + lanes, ...; shells of angular momentum
-// l are P.order[P.lstart[l]] .. P.order[P.lstart[l + 1] - 1]
+// V of the pairs whose later shell has angular momentum LA and whose earlier one
+// (or the same) LB: `lanes` (a power of two) neighbouring lanes
+// per pair, lane g evaluating charges g, g + lanes, ...; shells of angular
+// momentum l are P.order[P.lstart[l]] .. P.order[P.lstart[l + 1] - 1].  The
+// charges' terms pass through shared memory and are added in the order of the
+// charges, one element of the pair per lane, so the result does not depend on
+// the number of lanes: the sums are those of one thread taking one charge after
+// the other, to the bit.
 template <int LA, int LB>
 __global__ void __launch_bounds__(128) potential_kernel(OneBodyParams P, int lanes) {
   constexpr int L = LA + LB, NE = coff(L + 1), E0 = coff(LA), nE = NE - E0, NA = ncart(LA), NB = ncart(LB);
+  __shared__ double term[128][nE + 1];   // per lane: W of its charge, then Z w
+  __shared__ double sum[128][nE];        // per group (at its first lane): contracted X
   const int na = P.lstart[LA + 1] - P.lstart[LA], nb = P.lstart[LB + 1] - P.lstart[LB];
   const int npair = LA == LB ? na * (na + 1) / 2 : na * nb;
   const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / lanes), g = threadIdx.x & (lanes - 1);
-  const int q = min(t, npair - 1);   // every lane takes part in the shuffles
+  if (t >= npair) return;   // a whole group
+  const int base = threadIdx.x - g;
+  const unsigned group = (lanes == 32 ? 0xffffffffu : ((1u << lanes) - 1u)) << (base & 31);
   int ia, ib;
   if constexpr (LA == LB) {
-    ia = (int)((sqrtf(8.f * q + 1.f) - 1.f) * 0.5f);
-    while (ia * (ia + 1) / 2 > q) --ia;
-    while ((ia + 1) * (ia + 2) / 2 <= q) ++ia;
-    ib = q - ia * (ia + 1) / 2;
+    ia = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
+    while (ia * (ia + 1) / 2 > t) --ia;
+    while ((ia + 1) * (ia + 2) / 2 <= t) ++ia;
+    ib = t - ia * (ia + 1) / 2;
   } else {
-    ia = q / nb;
-    ib = q - ia * nb;
+    ia = t / nb;
+    ib = t - ia * nb;
   }
-  const int s1 = P.order[P.lstart[LA] + ia], s2 = P.order[P.lstart[LB] + ib];
-  const DevShell A = P.shells[s1], B = P.shells[s2];
+  const int oa = P.order[P.lstart[LA] + ia], ob = P.order[P.lstart[LB] + ib];
+  if (oa < ob) return;   // the pair belongs to the class (LB LA)
+  const DevShell A = P.shells[oa], B = P.shells[ob];
   double AB[3], AB2 = 0;
-#pragma unroll
   for (int d = 0; d < 3; ++d) {
     AB[d] = A.O[d] - B.O[d];
-    AB2 = fma(AB[d], AB[d], AB2);
+    AB2 += AB[d] * AB[d];
   }
-  double X[nE];
-#pragma unroll
-  for (int e = 0; e < nE; ++e) X[e] = 0.0;
+  for (int e = g; e < nE; e += lanes) sum[base][e] = 0.0;
   for (int pa = 0; pa < A.nprim; ++pa)
     for (int pb = 0; pb < B.nprim; ++pb) {
-      const double a = P.alpha[A.p0 + pa], b = P.alpha[B.p0 + pb], p = a + b, op = 1.0 / p, o2p = 0.5 * op;
-      const double w = P.cn[A.p0 + pa] * P.cn[B.p0 + pb] * exp(-a * b * op * AB2) * (2.0 * 3.14159265358979323846) * op;
+      const double a = P.alpha[A.p0 + pa], b = P.alpha[B.p0 + pb], p = a + b, o2p = 0.5 / p;
+      const double cab = P.cn[A.p0 + pa] * P.cn[B.p0 + pb] * exp(-a * b / p * AB2);
       double Pc[3], PA[3];
-#pragma unroll
       for (int d = 0; d < 3; ++d) {
-        Pc[d] = (a * A.O[d] + b * B.O[d]) * op;
+        Pc[d] = (a * A.O[d] + b * B.O[d]) / p;
         PA[d] = Pc[d] - A.O[d];
       }
-      for (int c = g; c < P.ncharge; c += lanes) {
-        double PC[3], PC2 = 0, F[L + 1];
+      const double w = cab * 2.0 * 3.14159265358979323846 / p;
+      for (int c0 = 0; c0 < P.ncharge; c0 += lanes) {
+        const int c = c0 + g;
+        if (c < P.ncharge) {
+          double PC[3], PC2 = 0, F[L + 1];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          PC[d] = Pc[d] - __ldg(P.R + 3 * c + d);
-          PC2 = fma(PC[d], PC[d], PC2);
-        }
-        boys_f64<L>(p * PC2, F, P.boys.f64);
-        double W[NE][L + 1];
-#pragma unroll
-        for (int m = 0; m <= L; ++m) W[0][m] = F[m];
-        sfor<1, NE>([&](auto ec) {
-          constexpr int e = decltype(ec)::value;
-          constexpr int d = cdir(e), em = cminus(e, d), ei = ccomp(e, d) - 1;
-          constexpr int emm = ei > 0 ? cminus(em, d) : 0;
-#pragma unroll
-          for (int m = 0; m <= L - clevel(e); ++m) {
-            double v = PA[d] * W[em][m] - PC[d] * W[em][m + 1];
-            if constexpr (ei > 0) v += ei * o2p * (W[emm][m] - W[emm][m + 1]);
-            W[e][m] = v;
+          for (int d = 0; d < 3; ++d) {
+            PC[d] = Pc[d] - P.R[3 * c + d];
+            PC2 += PC[d] * PC[d];
           }
-        });
-        const double zw = __ldg(P.Z + c) * w;
-        sfor<E0, NE>([&](auto ec) {
-          constexpr int e = decltype(ec)::value;
-          X[e - E0] = fma(zw, W[e][0], X[e - E0]);
-        });
+          boys_f64_rt(L, p * PC2, F, P.boys.f64);
+          double W[NE][L + 1];
+#pragma unroll
+          for (int m = 0; m <= L; ++m) W[0][m] = F[m];
+          sfor<1, NE>([&](auto ec) {
+            constexpr int e = decltype(ec)::value;
+            constexpr int d = cdir(e), em = cminus(e, d), ei = ccomp(e, d) - 1;
+            constexpr int emm = ei > 0 ? cminus(em, d) : 0;
+#pragma unroll
+            for (int m = 0; m <= L - clevel(e); ++m) {
+              double v = PA[d] * W[em][m] - PC[d] * W[em][m + 1];
+              if constexpr (ei > 0) v += ei * o2p * (W[emm][m] - W[emm][m + 1]);
+              W[e][m] = v;
+            }
+          });
+          sfor<E0, NE>([&](auto ec) {
+            constexpr int e = decltype(ec)::value;
+            term[threadIdx.x][e - E0] = W[e][0];
+          });
+          term[threadIdx.x][nE] = P.Z[c] * w;
+        }
+        __syncwarp(group);
+        const int cnt = min(lanes, P.ncharge - c0);
+        for (int e = g; e < nE; e += lanes) {
+          double x = sum[base][e];
+          for (int j = 0; j < cnt; ++j) x += term[base + j][nE] * term[base + j][e];
+          sum[base][e] = x;
+        }
+        __syncwarp(group);
       }
     }
-  for (int o = 1; o < lanes; o <<= 1)
+  if (g) return;
+  double X[nE], V[NA * NB];
 #pragma unroll
-    for (int e = 0; e < nE; ++e) X[e] += __shfl_xor_sync(0xffffffffu, X[e], o);
-  if (t >= npair || g) return;
-  double V[NA * NB];
+  for (int e = 0; e < nE; ++e) X[e] = sum[base][e];
   hrr<double, LA, LB, 1>(X, AB, V);
-  const int fa = P.first[s1], fb = P.first[s2];
+  const int fa = P.first[oa], fb = P.first[ob];
   const size_t n = P.n;
 #pragma unroll
   for (int x = 0; x < NA * NB; ++x) {
     const int i = fa + x / NB, j = fb + x % NB;
-    P.V[i * n + j] = P.V[j * n + i] = V[x] * P.norma[i] * P.norma[j];
+    const double nn = P.norma[i] * P.norma[j];
+    P.V[i * n + j] = P.V[j * n + i] = V[x] * nn;
   }
 }
 
@@ -258,25 +276,26 @@ cudaError_t launch_one_body(const OneBodyParams &p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_potential(int pc, const OneBodyParams &p, cudaStream_t s) {
+cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, cudaStream_t s) {
   using Fn = void (*)(OneBodyParams, int);
-  static const Fn fn[6] = {&potential_kernel<0, 0>, &potential_kernel<1, 0>, &potential_kernel<1, 1>,
-                           &potential_kernel<2, 0>, &potential_kernel<2, 1>, &potential_kernel<2, 2>};
+  static const Fn fn[3][3] = {{&potential_kernel<0, 0>, &potential_kernel<0, 1>, &potential_kernel<0, 2>},
+                              {&potential_kernel<1, 0>, &potential_kernel<1, 1>, &potential_kernel<1, 2>},
+                              {&potential_kernel<2, 0>, &potential_kernel<2, 1>, &potential_kernel<2, 2>}};
   static_assert(kPotMaxL == 2, "one entry per class of potential_kernel");
-  const long long npair = potential_pairs(pc, p);
+  const long long npair = potential_pairs(la, lb, p);
   if (npair <= 0 || p.ncharge <= 0) return cudaSuccess;
   // lanes per pair: up to four warps per scheduler, no more than there are charges
   int lanes = 1;
   while (lanes < 32 && 2 * lanes <= p.ncharge && npair / 32 * lanes < 2 * (long long)kFillWarps) lanes *= 2;
-  fn[pc]<<<(unsigned)((npair * lanes + 127) / 128), 128, 0, s>>>(p, lanes);
+  fn[la][lb]<<<(unsigned)((npair * lanes + 127) / 128), 128, 0, s>>>(p, lanes);
   count_launches(1);
   return cudaGetLastError();
 }
 
-long long potential_pairs(int pc, const OneBodyParams &p) {
-  if (pc < 0 || pc >= 6) return 0;
-  const long long na = p.lstart[pc_la(pc) + 1] - p.lstart[pc_la(pc)], nb = p.lstart[pc_lb(pc) + 1] - p.lstart[pc_lb(pc)];
-  return pc_la(pc) == pc_lb(pc) ? na * (na + 1) / 2 : na * nb;
+long long potential_pairs(int la, int lb, const OneBodyParams &p) {
+  if (la < 0 || lb < 0 || la > kPotMaxL || lb > kPotMaxL) return 0;
+  const long long na = p.lstart[la + 1] - p.lstart[la], nb = p.lstart[lb + 1] - p.lstart[lb];
+  return la == lb ? na * (na + 1) / 2 : na * nb;
 }
 
 }  // namespace lgb

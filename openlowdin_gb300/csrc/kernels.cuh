@@ -559,9 +559,10 @@ struct OneBodyParams {
 };
 // S and T, and V of the pairs with an f shell
 cudaError_t launch_one_body(const OneBodyParams &p, cudaStream_t s);
-// V of a pair class of s, p and d shells, and its number of pairs (0 for other classes)
-cudaError_t launch_potential(int pc, const OneBodyParams &p, cudaStream_t s);
-long long potential_pairs(int pc, const OneBodyParams &p);
+// V of the pairs with a later shell of angular momentum la and an earlier one of
+// lb (s, p and d), and the candidates of such a launch (0 for other classes)
+cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, cudaStream_t s);
+long long potential_pairs(int la, int lb, const OneBodyParams &p);
 
 // x[i] = deterministic pseudo-random values in [-1, 1) (benchmark operands)
 cudaError_t launch_fill_hash(float *x, long long n, unsigned seed, cudaStream_t s);

@@ -1043,10 +1043,11 @@ int LowdinGB300_one_body_device(LibintInterface *lint, int ncharge, const double
   }
   std::vector<Lanes::Job> jobs;
   jobs.push_back({(double)p.nsh * p.nsh, false, [=](cudaStream_t q) { return launch_one_body(p, q); }});
-  for (int pc = 0; p.V && p.ncharge > 0 && pc < kNumPairClasses; ++pc)
-    if (potential_pairs(pc, p) > 0)
-      jobs.push_back({(double)potential_pairs(pc, p) * p.ncharge * ncart(pc_la(pc)) * ncart(pc_lb(pc)), false,
-                      [=](cudaStream_t q) { return launch_potential(pc, p, q); }});
+  for (int la = 0; p.V && p.ncharge > 0 && la <= kMaxL; ++la)
+    for (int lb = 0; lb <= kMaxL; ++lb)
+      if (potential_pairs(la, lb, p) > 0)
+        jobs.push_back({(double)potential_pairs(la, lb, p) * p.ncharge * ncart(la) * ncart(lb), false,
+                        [=](cudaStream_t q) { return launch_potential(la, lb, p, q); }});
   Lanes lanes(s);
   return lanes.run(jobs, s) ? 0 : -1;
 }
