@@ -656,6 +656,10 @@ __global__ void __launch_bounds__(32 * kRowWarps) jk32_row_kernel(const JKTask *
 // J_A[i][j] += scale sum_{kl} D_B[k][l] (ij|kl), J_B[k][l] += scale
 // sum_{ij} D_A[i][j] (ij|kl), both as full symmetric matrices; raw |v| < cut is
 // dropped (the reference's 1e-10 test on each integral).
+// A warp keeps its bra pair and walks up to TL.tile.chunk ket tiles; J_A is
+// summed over them before its one reduction.
+// No double-float tier: divided at 2^-12 of the largest Q_ab Q_cd, J of six
+// waters was 1.5e-13 off against 2.7e-14 in FP64.
 template <typename R, int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128) cp_tasks_kernel(const CPTask *__restrict__ tasks, TaskLaunch TL) {
   using Q = QClass<LA, LB, LC, LD>;
@@ -667,112 +671,123 @@ __global__ void __launch_bounds__(128) cp_tasks_kernel(const CPTask *__restrict_
   if (act == kSysOff) return;   // converged system: nothing to build
   if (act == kSysFP64 && TL.mixed && TL.lower) return;   // system held in FP64: the FP64 launch takes it all
   const int local = blockIdx.x - T.blk0;
-  const int tx = local % T.nbx, ty = local / T.nbx;
   const int kets = TL.tile.kets, parts = 32 / kets;
-  const int kl = threadIdx.x & (kets - 1), part = threadIdx.x / kets;
-  const int kpos = tx * kets + kl;
+  const int ty = local / T.nbx;
+  const int kl = threadIdx.x & (kets - 1), part = parts == 1 ? 0 : threadIdx.x / kets;
   const int bpos = ty * blockDim.y + threadIdx.y;
   if (bpos >= T.nbra) return;
-  // pairs are sorted by decreasing Schwarz factor: the warp's first ket has its
-  // largest bound (with room for the FP32 rounding of the factors)
-  if (T.pa32[T.bra0 + bpos].Q * T.pb32[T.ket0 + tx * kets].Q * 1.00001f < TL.cut32) return;
-  bool active = kpos < T.nket;
-  {
-    // |(ij|kl)| <= Q_ab Q_cd for every component (Schwarz), and raw values
-    // below the cut are dropped, so such a quartet contributes nothing; the
-    // test is done in FP32 in mixed launches so both launches agree
-    const int bi = T.bra0 + bpos, ki = T.ket0 + min(kpos, T.nket - 1);
-    const bool tiny = TL.mixed ? T.pa32[bi].Q * T.pb32[ki].Q * 0.999f < TL.cut32
-                                     : abs_below(T.pa[bi].Q * T.pb[ki].Q * (1.0 - 1e-9), TL.cut);
-    if (tiny) active = false;
-  }
-  if (TL.mixed) {
-    // mixed precision: FP32 for quartets whose Q_ab Q_cd max(|D_A|, |D_B|)
-    // bound (FP32, identical in both launches) is below the split
-    const int bi = T.bra0 + bpos, ki = T.ket0 + min(kpos, T.nket - 1);
-    const PairRec32 &b32 = T.pa32[bi];
-    const PairRec32 &k32 = T.pb32[ki];
-    float dm = 0.f;
-    if (T.DnA32) dm = __ldg(T.DnA32 + b32.sa * T.nshA + b32.sb);
-    if (T.DnB32) dm = fmaxf(dm, __ldg(T.DnB32 + k32.sa * T.nshB + k32.sb));
-    const float b = b32.Q * k32.Q * dm;
-    if (act != kSysFP64 && (TL.lower ? !(b < TL.split32) : (b < TL.split32))) active = false;
-    if ((T.DnA32 || T.DnB32) && act != kSysFP64 && b < TL.skip) active = false;
-  }
-  if (__all_sync(0xffffffffu, !active)) return;
-  if (T.count) {
-    const unsigned cnt = __popc(__ballot_sync(0xffffffffu, active && part == 0));
-    if (threadIdx.x == 0) atomicAdd(T.count, (unsigned long long)cnt);
-  }
+  const int bi = T.bra0 + bpos;
+  int k0 = (local - ty * T.nbx) * TL.tile.chunk * kets;
+  const int kend = min(T.nket, k0 + TL.tile.chunk * kets);
+  const float qbra = T.pa32[bi].Q;
+  // |(ij|kl)| <= Q_ab Q_cd for every component (Schwarz), and raw values below
+  // the cut are dropped, so a quartet below it contributes nothing.  Pairs are
+  // sorted by decreasing Schwarz factor: the first ket of a tile bounds all
+  // after it (0.99999: room for the FP32 rounding of the factors).
+  const float reach = 0.99999f * TL.cut32;
+  if (qbra * T.pb32[T.ket0 + k0].Q < reach) return;
   const PairT<R> *pa, *pb;
   const PrimT<R> *pra, *prb;
-  const R *DA, *DB;
   if constexpr (F64) {
-    pa = T.pa; pb = T.pb; pra = T.pra; prb = T.prb; DA = T.DsA; DB = T.DsB;
+    pa = T.pa; pb = T.pb; pra = T.pra; prb = T.prb;
   } else {
-    pa = T.pa32; pb = T.pb32; pra = T.pra32; prb = T.prb32; DA = T.DsA32; DB = T.DsB32;
+    pa = T.pa32; pb = T.pb32; pra = T.pra32; prb = T.prb32;
   }
-  const PairT<R> &bra = pa[T.bra0 + bpos];
-  const PairT<R> ket = pb[T.ket0 + min(kpos, T.nket - 1)];
-  R I[Q::NINT];
-  if (active || parts > 1) {
-    eri_quartet<R, LA, LB, LC, LD>(bra, pra + bra.prim0, ket, prb + ket.prim0, TL.boys.f64, TL.boys.dd, I, part,
-                                   parts, active);
-    if (part) active = false;   // the quartet is digested by its first lane
-  } else {
-#pragma unroll
-    for (int x = 0; x < Q::NINT; ++x) I[x] = R(0);
-  }
-  R cut, scale;
+  auto DA = [&](int i) { return elem<R>(T.DsA, T.DsA32, nullptr, i); };
+  auto DB = [&](int i) { return elem<R>(T.DsB, T.DsB32, nullptr, i); };
+  R scale, cut;
   if constexpr (F64) {
-    cut = TL.cut;
     scale = T.scale;
+    cut = TL.cut;
   } else {
-    cut = TL.cut32;
     scale = T.scale32;
+    cut = TL.cut32;
   }
+  const PairT<R> &bra = pa[bi];
+  const int fa = bra.fa, fb = bra.fb, nA = T.nA, nB = T.nB;
+  const bool abdiff = bra.sa != bra.sb;
+  R ja[NA * NB];
 #pragma unroll
-  for (int x = 0; x < Q::NINT; ++x)
-    if (abs_below(I[x], cut)) I[x] = R(0);
-  auto Iat = [&](int a, int b, int c, int d) -> R { return I[((a * NB + b) * NC + c) * ND + d]; };
-  const int fa = bra.fa, fb = bra.fb, fc = ket.fa, fd = ket.fb;
-  const bool abdiff = bra.sa != bra.sb, cddiff = ket.sa != ket.sb;
-  if (T.JA) {
-    const R wk = active ? R(cddiff ? 2 : 1) * scale : R(0);
-    const int nB = T.nB, nA = T.nA;
+  for (int x = 0; x < NA * NB; ++x) ja[x] = R(0);
+  unsigned cnt = 0;
+  for (; k0 < kend; k0 += kets) {
+    if (qbra * T.pb32[T.ket0 + k0].Q < reach) break;
+    const int kpos = k0 + kl;
+    bool active = kpos < T.nket;
+    const int ki = T.ket0 + min(kpos, T.nket - 1);
+    const PairRec32 &k32 = T.pb32[ki];
+    const float qq = qbra * k32.Q;
+    if (TL.mixed) {
+      // the test is done in FP32 in mixed launches so both launches agree; FP32
+      // for quartets whose Q_ab Q_cd max(|D_A|, |D_B|) bound (FP32, identical in
+      // both launches) is below the split
+      if (qq * 0.999f < TL.cut32) active = false;
+      const PairRec32 &b32 = T.pa32[bi];
+      float dm = 0.f;
+      if (T.DnA32) dm = __ldg(T.DnA32 + b32.sa * T.nshA + b32.sb);
+      if (T.DnB32) dm = fmaxf(dm, __ldg(T.DnB32 + k32.sa * T.nshB + k32.sb));
+      const float b = qq * dm;
+      if (act != kSysFP64 && (TL.lower ? !(b < TL.split32) : (b < TL.split32))) active = false;
+      if ((T.DnA32 || T.DnB32) && act != kSysFP64 && b < TL.skip) active = false;
+    } else if (qq < 1.00001f * TL.cut32) {
+      // too near the cut for FP32 to decide
+      if (qq < 0.99999f * TL.cut32 || abs_below(T.pa[bi].Q * T.pb[ki].Q * (1.0 - 1e-9), TL.cut)) active = false;
+    }
+    if (!__any_sync(0xffffffffu, active)) continue;
+    cnt += __popc(__ballot_sync(0xffffffffu, active && part == 0));
+    const PairT<R> &ket = pb[ki];
+    R I[Q::NINT];
+    if (active || parts > 1) {
+      eri_quartet<R, LA, LB, LC, LD>(bra, pra + bra.prim0, ket, prb + ket.prim0, TL.boys.f64, TL.boys.dd, I, part, parts,
+                                     active);
+      if (part) active = false;   // the quartet is digested by its first lane
+    }
+    if (active) {
 #pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        R s = 0;
+      for (int x = 0; x < Q::NINT; ++x)
+        if (abs_below(I[x], cut)) I[x] = R(0);
+      const int fc = ket.fa, fd = ket.fb;
+      const bool cddiff = ket.sa != ket.sb;
+      if (T.JA) {
+        const R wk = cddiff ? scale + scale : scale;
 #pragma unroll
         for (int c = 0; c < NC; ++c)
 #pragma unroll
-          for (int d = 0; d < ND; ++d) s += __ldg(DB + (fc + c) * nB + fd + d) * Iat(a, b, c, d);
-        s = warp_sum(s * wk);
-        if (threadIdx.x == 0) {
-          atomic_acc<R>(T.JA, T.JA32, (size_t)(fa + a) * nA + fb + b, s);
-          if (abdiff) atomic_acc<R>(T.JA, T.JA32, (size_t)(fb + b) * nA + fa + a, s);
-        }
+          for (int d = 0; d < ND; ++d) {
+            const R w = wk * DB((fc + c) * nB + fd + d);
+#pragma unroll
+            for (int x = 0; x < NA * NB; ++x) ja[x] = mad(w, I[(x * NC + c) * ND + d], ja[x]);
+          }
       }
-  }
-  if (T.JB && active) {
-    const R wb = R(abdiff ? 2 : 1) * scale;
-    const int nA = T.nA, nB = T.nB;
+      if (T.JB) {
+        const R wb = abdiff ? scale + scale : scale;
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
+        for (int c = 0; c < NC; ++c)
 #pragma unroll
-      for (int d = 0; d < ND; ++d) {
-        R s = 0;
+          for (int d = 0; d < ND; ++d) {
+            R s = R(0);
 #pragma unroll
-        for (int a = 0; a < NA; ++a)
-#pragma unroll
-          for (int b = 0; b < NB; ++b) s += __ldg(DA + (fa + a) * nA + fb + b) * Iat(a, b, c, d);
-        s *= wb;
-        atomic_acc<R>(T.JB, T.JB32, (size_t)(fc + c) * nB + fd + d, s);
-        if (cddiff) atomic_acc<R>(T.JB, T.JB32, (size_t)(fd + d) * nB + fc + c, s);
+            for (int x = 0; x < NA * NB; ++x)
+              s = mad(DA((fa + x / NB) * nA + fb + x % NB), I[(x * NC + c) * ND + d], s);
+            s = s * wb;
+            atomic_acc<R>(T.JB, T.JB32, (size_t)(fc + c) * nB + fd + d, s);
+            if (cddiff) atomic_acc<R>(T.JB, T.JB32, (size_t)(fd + d) * nB + fc + c, s);
+          }
       }
+    }
+    __syncwarp();
   }
+  if (!cnt) return;   // warp-uniform
+  if (T.JA)
+#pragma unroll
+    for (int x = 0; x < NA * NB; ++x) {
+      const R s = warp_sum(ja[x]);
+      if (threadIdx.x == 0) {
+        atomic_acc<R>(T.JA, T.JA32, (size_t)(fa + x / NB) * nA + fb + x % NB, s);
+        if (abdiff) atomic_acc<R>(T.JA, T.JA32, (size_t)(fb + x % NB) * nA + fa + x / NB, s);
+      }
+    }
+  if (T.count && threadIdx.x == 0) atomicAdd(T.count, (unsigned long long)cnt);
 }
 
 // ----------------------------------------------------------- geminal (G12) --

@@ -73,6 +73,7 @@ struct LaunchLoad {
   double quartets = 0, mean = 1, most = 1;
   int grid_y = 0;
   bool linear = false;
+  bool walk = false;      // a block can walk several ket tiles
 };
 // A launch below kFillWarps (two warps per scheduler) is as long as its longest
 // quartet, so it splits quartets over as many lanes as they have primitive
@@ -99,7 +100,7 @@ inline TileShape tile_shape(const LaunchLoad &w) {
   // reach and reduces its bra-block Coulomb sums once; where that would leave
   // fewer than 32 warps per scheduler, tiles are worth more than that
   int chunk = 1;
-  while (w.linear && chunk < 8 && warps * slices / (2 * chunk) >= 16 * kFillWarps) chunk *= 2;
+  while (w.walk && chunk < 8 && warps * slices / (2 * chunk) >= 16 * kFillWarps) chunk *= 2;
   return {32 / parts, warps * slices >= 2 * kFillWarps || w.grid_y > 65535 ? kWarpsPerBlock : 1, slices, chunk};
 }
 inline TileShape coop_tile(const LaunchLoad &w) {
@@ -242,7 +243,7 @@ struct TaskLaunch {
   // FP32 copies of the thresholds and the mixed flag (split > 0), so that the
   // kernels issue no FP64 conversion or comparison for them
   int mixed;
-  Tier tier;              // J/K and coupling: the quartets this launch takes
+  Tier tier;              // J/K: the quartets this launch takes
   float eps32, split32, cut32;
   BoysTables boys;
 };

@@ -423,38 +423,47 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
                   pc_lb(ck));
         return false;
       }
+      // The coupling is symmetric in the two species: the one with more pairs
+      // of the class gives the kets, which the lanes of a warp run over.  With
+      // the species as they came, a proton's single (pp| pair left 31 lanes of
+      // each warp idle.
+      const bool swap = A->all.count(cb) > B->all.count(ck);
+      LibintInterface *X = swap ? B : A, *Y = swap ? A : B;
+      const SpeciesBufs &bx = swap ? bb : ba, &by = swap ? ba : bb;
+      double *JX = swap ? JB : JA, *JY = swap ? JA : JB;
+      const int cx = swap ? ck : cb, cy = swap ? cb : ck;
       CPTask t{};
-      t.pa = A->all.d;
-      t.pra = A->all.dp;
-      t.pb = B->all.d;
-      t.prb = B->all.dp;
-      t.pa32 = A->all.d32;
-      t.pra32 = A->all.dp32;
-      t.pb32 = B->all.d32;
-      t.prb32 = B->all.dp32;
-      t.DsA = JB ? ba.Ds : nullptr;
-      t.DsA32 = JB ? ba.Ds32 : nullptr;
-      t.DsB = JA ? bb.Ds : nullptr;
-      t.DsB32 = JA ? bb.Ds32 : nullptr;
-      t.JA = JA;
-      t.JA32 = JA ? ba.G32 : nullptr;
-      t.JB = JB;
-      t.JB32 = JB ? bb.G32 : nullptr;
-      t.DnA32 = ba.Dn32;
-      t.DnB32 = bb.Dn32;
+      t.pa = X->all.d;
+      t.pra = X->all.dp;
+      t.pb = Y->all.d;
+      t.prb = Y->all.dp;
+      t.pa32 = X->all.d32;
+      t.pra32 = X->all.dp32;
+      t.pb32 = Y->all.d32;
+      t.prb32 = Y->all.dp32;
+      t.DsA = JY ? bx.Ds : nullptr;
+      t.DsA32 = JY ? bx.Ds32 : nullptr;
+      t.DsB = JX ? by.Ds : nullptr;
+      t.DsB32 = JX ? by.Ds32 : nullptr;
+      t.JA = JX;
+      t.JA32 = JX ? bx.G32 : nullptr;
+      t.JB = JY;
+      t.JB32 = JY ? by.G32 : nullptr;
+      t.DnA32 = bx.Dn32;
+      t.DnB32 = by.Dn32;
       t.count = counters ? counters + cb * kNumPairClasses + ck : nullptr;
-      t.nshA = A->nshell();
-      t.nshB = B->nshell();
+      t.nshA = X->nshell();
+      t.nshB = Y->nshell();
       t.scale = scale;
       t.scale32 = (float)scale;
-      t.bra0 = A->all.start[cb];
-      t.nbra = A->all.count(cb);
-      t.ket0 = B->all.start[ck];
-      t.nket = B->all.count(ck);
+      t.bra0 = X->all.start[cx];
+      t.nbra = X->all.count(cx);
+      t.ket0 = Y->all.start[cy];
+      t.nket = Y->all.count(cy);
       t.mean_prims = t.most_prims = (float)(pa[cb] * pb[ck]);
-      t.nA = A->nbasis;
-      t.nB = B->nbasis;
-      ts.add(cb, ck, t);
+      t.nA = X->nbasis;
+      t.nB = Y->nbasis;
+      ts.add(cx, cy, t);
     }
   return true;
 }

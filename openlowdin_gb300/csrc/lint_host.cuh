@@ -101,24 +101,18 @@ struct PairList {
     for (int i = start[pc]; i < start[pc + 1]; ++i) n = std::max(n, h[i].nprim);
     return n;
   }
-  // uploads the FP64 records and their FP32 copies
-  bool upload() {
+  // uploads the FP64 records (all that the Schwarz factors need)
+  bool upload64() {
     release();
-    std::vector<PairRec32> h32(h.size());
-    std::vector<PrimRec32> hp32(hp.size());
+    return dev_upload(d, h) && dev_upload(dp, hp);
+  }
+  // uploads the double-float copies (the first J/K build asks for them)
+  bool upload_dd() {
+    if (dd) return true;
     std::vector<PairRecD> hd(h.size());
     std::vector<PrimRecD> hpd(hp.size());
     for (size_t i = 0; i < h.size(); ++i) {
       const PairRec &a = h[i];
-      PairRec32 &b = h32[i];
-      b.sa = a.sa; b.sb = a.sb; b.fa = a.fa; b.fb = a.fb; b.prim0 = a.prim0; b.nprim = a.nprim;
-      b.la = a.la; b.lb = a.lb;
-      for (int k = 0; k < 3; ++k) {
-        b.A[k] = (float)a.A[k];
-        b.AB[k] = (float)a.AB[k];
-      }
-      b.Q = (float)a.Q;
-      b.pad = 0.f;
       PairRecD &c = hd[i];
       c.sa = a.sa; c.sb = a.sb; c.fa = a.fa; c.fb = a.fb; c.prim0 = a.prim0; c.nprim = a.nprim;
       c.la = a.la; c.lb = a.lb;
@@ -131,12 +125,6 @@ struct PairList {
     }
     for (size_t i = 0; i < hp.size(); ++i) {
       const PrimRec &a = hp[i];
-      PrimRec32 &b = hp32[i];
-      b.p = (float)a.p; b.inv_p = (float)a.inv_p; b.Kt = (float)a.Kt; b.pad = 0.f;
-      for (int k = 0; k < 3; ++k) {
-        b.P[k] = (float)a.P[k];
-        b.PA[k] = (float)a.PA[k];
-      }
       PrimRecD &c = hpd[i];
       c.p = split_double(a.p); c.inv_p = split_double(a.inv_p); c.Kt = split_double(a.Kt);
       c.pad = dd32(0.f); c.pad2 = 0.f;
@@ -148,9 +136,35 @@ struct PairList {
         c.P[k][2] = (float)(a.P[k] - (double)h2.hi - (double)h2.lo);
       }
     }
-    if (!(dev_upload(d, h) && dev_upload(dp, hp) && dev_upload(d32, h32) && dev_upload(dp32, hp32) &&
-          dev_upload(dd, hd) && dev_upload(ddp, hpd)))
-      return false;
+    return dev_upload(dd, hd) && dev_upload(ddp, hpd);
+  }
+  // uploads the FP64 records and their FP32 copies
+  bool upload() {
+    release();
+    std::vector<PairRec32> h32(h.size());
+    std::vector<PrimRec32> hp32(hp.size());
+    for (size_t i = 0; i < h.size(); ++i) {
+      const PairRec &a = h[i];
+      PairRec32 &b = h32[i];
+      b.sa = a.sa; b.sb = a.sb; b.fa = a.fa; b.fb = a.fb; b.prim0 = a.prim0; b.nprim = a.nprim;
+      b.la = a.la; b.lb = a.lb;
+      for (int k = 0; k < 3; ++k) {
+        b.A[k] = (float)a.A[k];
+        b.AB[k] = (float)a.AB[k];
+      }
+      b.Q = (float)a.Q;
+      b.pad = 0.f;
+    }
+    for (size_t i = 0; i < hp.size(); ++i) {
+      const PrimRec &a = hp[i];
+      PrimRec32 &b = hp32[i];
+      b.p = (float)a.p; b.inv_p = (float)a.inv_p; b.Kt = (float)a.Kt; b.pad = 0.f;
+      for (int k = 0; k < 3; ++k) {
+        b.P[k] = (float)a.P[k];
+        b.PA[k] = (float)a.PA[k];
+      }
+    }
+    if (!(dev_upload(d, h) && dev_upload(dp, hp) && dev_upload(d32, h32) && dev_upload(dp32, hp32))) return false;
     bool one = !h.empty();
     for (const auto &r : h) one = one && r.nprim == 1;
     if (one) {
@@ -275,6 +289,7 @@ struct TaskSet {
     LaunchLoad w;
     w.mean = 0;
     w.linear = std::is_same<T, JKTask>::value;
+    w.walk = true;
     for (const T &t : group[c]) {
       double q = (double)t.nbra * t.nket;
       if constexpr (std::is_same<T, JKTask>::value)
@@ -302,7 +317,7 @@ struct TaskSet {
   void clear() {
     for (auto &g : group) g.clear();
   }
-  // whether every task of group c can run in two tiers
+  // whether group c runs in two tiers: every task has its double-float form
   bool tiers(int c) const {
     if constexpr (std::is_same<T, JKTask>::value) {
       double q = 0;
@@ -588,7 +603,7 @@ struct LibintInterface {
         if (sigf) raw.push_back(make_pair(s1, s2, rawp));
       }
     bin_pairs(sig, raw, rawp, false);
-    if (!sig.upload()) return false;
+    if (!sig.upload64()) return false;
     if (!compute_schwarz(sig)) return false;
     // sort by decreasing Schwarz factor inside each class
     std::vector<PairRec> tmp = sig.h;
@@ -607,7 +622,7 @@ struct LibintInterface {
     for (int s1 = 0; s1 < nshell(); ++s1)
       for (int s2 = 0; s2 <= s1; ++s2) raw.push_back(make_pair(s1, s2, rawp));
     bin_pairs(all, raw, rawp, false);
-    if (!all.upload()) return false;
+    if (!all.upload64()) return false;
     // Schwarz factors of every pair: exact skip of quartets whose bound is
     // below the coupling cut, and the mixed-precision split; sorted by Q inside
     // a class so skipped quartets cluster into whole warps
@@ -697,6 +712,7 @@ struct LibintInterface {
   // J/K tasks of this species into ts: one task per (bra class >= ket class)
   bool add_jk_tasks(TaskSet<JKTask> &ts, const SpeciesBufs &bf, double hf, unsigned long long *counters) {
     if (!ensure_sig()) return false;
+    if (bf.Dd && !sig.upload_dd()) return false;
     double qmax = 0;   // largest Schwarz factor of the species
     for (const PairRec &r : sig.h) qmax = std::max(qmax, r.Q);
     double cprims[kNumPairClasses], cmost[kNumPairClasses];
