@@ -540,6 +540,15 @@ template <typename T>
 cudaError_t launch_split_bf16(const T *src, long long rows, int cols, long long lds, int np, __nv_bfloat16 *const *out,
                               long long ldo, cudaStream_t s);
 
+// FP64 products C_z = A_z B_z (k_dgemm.cu): element (row, column) of a matrix at
+// p[row * rs + column * cs + z * batch stride]
+struct DMat {
+  const double *p;
+  long long rs, cs, z;
+};
+cudaError_t launch_dgemm(int M, int N, int K, const DMat &A, const DMat &B, double *C, long long scm, long long scn,
+                         long long zc, int batch, cudaStream_t s);
+
 // one-electron matrices of one species (k_onebody.cu)
 struct DevShell {
   int l, nprim, p0, pad;

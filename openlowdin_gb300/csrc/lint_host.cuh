@@ -16,8 +16,6 @@
 #include <type_traits>
 #include <vector>
 
-#include <cublas_v2.h>
-
 #include "../../include/lowdin_gb300.h"
 #include "kernels.cuh"
 

@@ -22,42 +22,6 @@
 // a significant ket shell pair (all nc^2 of a diagonal pair).
 namespace {
 
-std::mutex g_blas_mu;
-std::vector<std::pair<int, cublasHandle_t>> g_blas;
-
-bool blas_handle(cublasHandle_t *out) {
-  int dev = 0;
-  CK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(g_blas_mu);
-  for (auto &e : g_blas)
-    if (e.first == dev) {
-      *out = e.second;
-      return true;
-    }
-  cublasHandle_t h = nullptr;
-  if (cublasCreate(&h) != CUBLAS_STATUS_SUCCESS) {
-    set_error("cublasCreate failed");
-    return false;
-  }
-  g_blas.push_back({dev, h});
-  *out = h;
-  return true;
-}
-
-// row-major C_b = op(A_b) op(B_b), b < batch, with element strides between batches
-bool dgemm_rm(cublasHandle_t h, bool ta, bool tb, int m, int n, int k, const double *A, int lda, long long sA,
-              const double *B, int ldb, long long sB, double *C, int ldc, long long sC, int batch) {
-  const double one = 1.0, zero = 0.0;
-  const cublasStatus_t st =
-      cublasDgemmStridedBatched(h, tb ? CUBLAS_OP_T : CUBLAS_OP_N, ta ? CUBLAS_OP_T : CUBLAS_OP_N, n, m, k, &one, B,
-                                ldb, sB, A, lda, sA, &zero, C, ldc, sC, batch);
-  if (st != CUBLAS_STATUS_SUCCESS) {
-    set_error("cublasDgemmStridedBatched failed (status %d, m=%d n=%d k=%d batch=%d)", (int)st, m, n, k, batch);
-    return false;
-  }
-  return true;
-}
-
 struct MP2Stats {
   long long ncols = 0;
   int batches = 0;
@@ -232,15 +196,9 @@ long long mp2_max_batch(const MP2Columns &mc, const PairList &P) {
   return colB;
 }
 
-// FP64 back end: cuBLAS DGEMM for the four quarters
+// FP64 back end: the four quarters on the FP64 tensor instruction (k_dgemm.cu)
 bool mp2_fp64(MP2Setup &S, size_t budget, double *e2out, cudaStream_t s) {
   const int nA = S.nA, nB = S.nB, oA = S.oA, vA = S.vA, oB = S.oB, vB = S.vB;
-  cublasHandle_t blas;
-  if (!blas_handle(&blas)) return false;
-  if (cublasSetStream(blas, s) != CUBLAS_STATUS_SUCCESS) {
-    set_error("cublasSetStream failed");
-    return false;
-  }
   const PairList &PB = *S.PB;
   const size_t per_col = (size_t)nA * nA * sizeof(double) + (size_t)oA * nA * sizeof(double);
   MP2Columns mc;
@@ -280,22 +238,21 @@ bool mp2_fp64(MP2Setup &S, size_t budget, double *e2out, cudaStream_t s) {
     q.ncol = nb;
     CK(cudaMemsetAsync(X.p, 0, (size_t)nA * nb * nA * sizeof(double), s));
     if (!mp2_batch_ints(*S.PA, PB, q, k0, k1, s)) return false;
-    // T1 (oA x nb*nA) = CoA^T X ; Y[i][c0 + col][a] = T1[i] (nb x nA) CvA
-    if (!dgemm_rm(blas, true, false, oA, nb * nA, nA, CoA.p, oA, 0, X.p, nb * nA, 0, T1.p, nb * nA, 0, 1))
-      return false;
-    if (!dgemm_rm(blas, false, false, nb, vA, nA, T1.p, nA, (long long)nb * nA, CvA.p, vA, 0, Y.p + (size_t)c0 * vA,
-                  vA, ncols * vA, oA))
-      return false;
+    // T1 (oA x nb*nA) = CoA^T X ; Y[i][c0 + col][a] = T1[i] (nb x nA) CvA, its
+    // rows a against columns (i, col), so that both run on the long side
+    CK(launch_dgemm(oA, nb * nA, nA, {CoA.p, 1, oA, 0}, {X.p, (long long)nb * nA, 1, 0}, T1.p, (long long)nb * nA, 1, 0,
+                    1, s));
+    CK(launch_dgemm(vA, nb, nA, {CvA.p, 1, vA, 0}, {T1.p, 1, nA, (long long)nb * nA}, Y.p + (size_t)c0 * vA, 1, vA,
+                    ncols * vA, oA, s));
   }
   CK(cudaMemsetAsync(Z.p, 0, (size_t)nB * nB * vA * sizeof(double), s));
   for (int i = 0; i < oA; ++i) {
     CK(launch_mp2_unpack<double>(Y.p + (size_t)i * ncols * vA, dcolpair.p, ncols, nB, vA, Z.p, s));
     // W (oB x nB*vA) = CoB^T Z ; M_j (vB x vA) = CvB^T W_j
-    if (!dgemm_rm(blas, true, false, oB, nB * vA, nB, CoB.p, oB, 0, Z.p, nB * vA, 0, W.p, nB * vA, 0, 1))
-      return false;
-    if (!dgemm_rm(blas, true, false, vB, vA, nB, CvB.p, vB, 0, W.p, vA, (long long)nB * vA, M.p, vA,
-                  (long long)vB * vA, oB))
-      return false;
+    CK(launch_dgemm(oB, nB * vA, nB, {CoB.p, 1, oB, 0}, {Z.p, (long long)nB * vA, 1, 0}, W.p, (long long)nB * vA, 1, 0, 1,
+                    s));
+    CK(launch_dgemm(vB, vA, nB, {CvB.p, 1, vB, 0}, {W.p, vA, 1, (long long)nB * vA}, M.p, vA, 1, (long long)vB * vA, oB,
+                    s));
     const double ei = S.epsA[S.nfA + i];
     if (S.coupling)
       CK(launch_mp2_energy_coupling<double>(M.p, oB, vB, vA, ei, EoB.p, EvA.p, EvB.p, 1e-10, S.factor, e2.p, s));
