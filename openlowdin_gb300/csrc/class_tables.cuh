@@ -45,10 +45,16 @@ constexpr ITFn it_entry() {
 
 template <int B, int K>
 constexpr MXFn mx_entry() {
-  if constexpr (templated_class<B, K>()) return &mp2x_kernel<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
+  if constexpr (templated_class<B, K>()) return &mp2x_kernel<double, pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
   else return nullptr;
 }
 
+template <int B, int K>
+constexpr MXFn mxd_entry() {
+  if constexpr (templated_class<B, K, kTemplatedMaxL4>() && QClass<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>::NINT <= 27)
+    return &mp2x_kernel<dd32, pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
+  else return nullptr;
+}
 template <int B, int K>
 constexpr G12Fn g12_entry() {
   if constexpr (templated_class<B, K, kTemplatedMaxL4>()) return &g12_kernel<pc_la(B), pc_lb(B), pc_la(K), pc_lb(K)>;
@@ -98,6 +104,10 @@ constexpr JKFn jkd_entry() {
   extern const MXFn kMX_##B[kNumPairClasses];              \
   const ITFn kIT_##B[kNumPairClasses] = LGB_ROW(it_entry, B); \
   const MXFn kMX_##B[kNumPairClasses] = LGB_ROW(mx_entry, B);
+
+#define LGB_MXD_TABLE(B)                     \
+  extern const MXFn kMXD_##B[kNumPairClasses];             \
+  const MXFn kMXD_##B[kNumPairClasses] = LGB_ROW(mxd_entry, B);
 
 #define LGB_G12_TABLE(B)                     \
   extern const G12Fn kG12_##B[kNumPairClasses];            \

@@ -81,6 +81,14 @@ __device__ __forceinline__ void atomic_acc(double *g64, float *g32, size_t i, R 
   else atomicAdd(g32 + i, v);
 }
 
+// |v| > cut of a raw integral
+__device__ __forceinline__ bool above_cut(double v, double cut) { return abs_above(v, cut); }
+__device__ __forceinline__ bool above_cut(dd32 v, double cut) {
+  const float a = fabsf(fadd(v.hi, v.lo)), c = (float)cut;
+  if (fabsf(a - c) <= 1e-5f * c) return abs_above(to_double(v), cut);   // too near for FP32
+  return a > c;
+}
+
 // element i of a matrix kept in FP64, FP32 and double-float
 template <typename R>
 __device__ __forceinline__ R elem(const double *m64, const float *m32, const float2 *md, int i) {
@@ -925,24 +933,43 @@ __global__ void __launch_bounds__(128) it_kernel(ITParams P) {
 // ------------------------------------------------------ MP2 transform input --
 // Warp y: bra pair tile_y * bras + y; its lanes: ket pairs tile_x * kets + (lane
 // mod kets) of the batch, 32 / kets lanes each.
-template <int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(128) mp2x_kernel(MXParams P) {
+// R = dd32 writes the split-BF16 form only: the pieces hold at most the 24 bits of
+// an FP32 value, which double-float integrals (2^-45) round to as FP64 ones do.
+template <typename R, int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) mp2x_kernel(MXParams P) {
   using Q = QClass<LA, LB, LC, LD>;
+  constexpr bool DD = std::is_same<R, dd32>::value;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
-  const int kets = P.kets, parts = 32 / kets, part = threadIdx.x / kets;
+  const int kets = P.kets, parts = 32 / kets, part = parts == 1 ? 0 : threadIdx.x / kets;
   const int kpos = blockIdx.x * kets + (threadIdx.x & (kets - 1));
   const int bpos = blockIdx.y * blockDim.y + threadIdx.y;
   if (bpos >= P.nbra) return;   // warp-uniform
   const int bi = P.bra0 + bpos, ki = P.ket0 + min(kpos, P.nket - 1);
-  const PairRec bra = P.pairs[bi];
-  const PairRec ket = P.kpairs[ki];
-  bool active = kpos < P.nket && abs_above(bra.Q * ket.Q * (1.0 - 1e-9), P.cut);
-  if (active && P.screen && abs_below(bra.Q * ket.Q * dnorm6(P.Dn, P.nsh, bra.sa, bra.sb, ket.sa, ket.sb), P.eps))
-    active = false;
+  bool active = kpos < P.nket;
+  // quartet selection as in FP64; where the FP32 factors decide beyond their
+  // rounding (Q and norms: 4e-7), without an FP64 instruction
+  auto keeps = [&]() {
+    const double qq = P.pairs[bi].Q * P.kpairs[ki].Q;
+    if (!abs_above(qq * (1.0 - 1e-9), P.cut)) return false;
+    const PairRec &x = P.pairs[bi], &y = P.kpairs[ki];
+    return !(P.screen && abs_below(qq * dnorm6(P.Dn, P.nsh, x.sa, x.sb, y.sa, y.sb), P.eps));
+  };
+  const PairT<R> *pb, *pk;
+  const PrimT<R> *rb, *rk;
+  if constexpr (DD) {
+    pb = P.pairsd; pk = P.kpairsd; rb = P.primsd; rk = P.kprimsd;
+    const float qq = pb[bi].Q.hi * pk[ki].Q.hi, cut = (float)P.cut;
+    if (qq < 0.99999f * cut) active = false;
+    else if (active && (P.screen || qq < 1.00001f * cut)) active = keeps();
+  } else {
+    pb = P.pairs; pk = P.kpairs; rb = P.prims; rk = P.kprims;
+    if (active) active = keeps();
+  }
   if (parts == 1 ? !active : __all_sync(0xffffffffu, !active)) return;
-  double I[Q::NINT];
-  eri_quartet<double, LA, LB, LC, LD>(bra, P.prims + bra.prim0, ket, P.kprims + ket.prim0, P.boys.f64, P.boys.dd,
-                                      I, part, parts, active);
+  const PairT<R> &bra = pb[bi];
+  const PairT<R> ket = pk[ki];
+  R I[Q::NINT];
+  eri_quartet<R, LA, LB, LC, LD>(bra, rb + bra.prim0, ket, rk + ket.prim0, P.boys.f64, P.boys.dd, I, part, parts, active);
   if (part || !active) return;
   const int col0 = __ldg(P.colbase + ki) - P.col_first;
   const bool two = bra.sa != bra.sb;
@@ -955,25 +982,28 @@ __global__ void __launch_bounds__(128) mp2x_kernel(MXParams P) {
       for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
-          const double v = I[((a * NB + b) * NC + c) * ND + d];
-          if (!abs_above(v, P.cut)) continue;
+          const R v = I[((a * NB + b) * NC + c) * ND + d];
+          if (!above_cut(v, P.cut)) continue;
           const size_t col = col0 + c * ND + d;
-          const size_t i1 = ((bra.fa + a) * ncol + col) * n + bra.fb + b;
-          const size_t i2 = ((bra.fb + b) * ncol + col) * n + bra.fa + a;
-          if (P.X) {
-            P.X[i1] = v;
-            if (two) P.X[i2] = v;
-          } else {
-            // Xt[col * Kp + nu][mu] and the mirrored bra orientation
-            __nv_bfloat16 pc[kMaxPieces];
-            bf16_pieces((float)v, P.np, pc);   // three pieces hold the FP32 value exactly
-            const size_t kp = P.Kp;
-            const size_t j1 = (col * kp + bra.fb + b) * kp + bra.fa + a;
-            const size_t j2 = (col * kp + bra.fa + a) * kp + bra.fb + b;
-            for (int k = 0; k < P.np; ++k) {
-              P.Xp[k][j1] = pc[k];
-              if (two) P.Xp[k][j2] = pc[k];
+          if constexpr (!DD) {
+            if (P.X) {
+              P.X[((bra.fa + a) * ncol + col) * n + bra.fb + b] = v;
+              if (two) P.X[((bra.fb + b) * ncol + col) * n + bra.fa + a] = v;
+              continue;
             }
+          }
+          // Xt[col * Kp + nu][mu] and the mirrored bra orientation
+          float x;
+          if constexpr (DD) x = fadd(v.hi, v.lo);
+          else x = (float)v;
+          __nv_bfloat16 pc[kMaxPieces];
+          bf16_pieces(x, P.np, pc);   // three pieces hold the FP32 value exactly
+          const size_t kp = P.Kp;
+          const size_t j1 = (col * kp + bra.fb + b) * kp + bra.fa + a;
+          const size_t j2 = (col * kp + bra.fa + a) * kp + bra.fb + b;
+          for (int k = 0; k < P.np; ++k) {
+            P.Xp[k][j1] = pc[k];
+            if (two) P.Xp[k][j2] = pc[k];
           }
         }
 }

@@ -27,6 +27,7 @@ extern const JKFn kJKR_0[NPC], kJKR_1[NPC], kJKR_2[NPC], kJKR_3[NPC], kJKR_4[NPC
 extern const CPFn kCP64_0[NPC], kCP64_1[NPC], kCP64_2[NPC], kCP64_3[NPC], kCP64_4[NPC], kCP64_5[NPC];
 extern const CPFn kCP32_0[NPC], kCP32_1[NPC], kCP32_2[NPC], kCP32_3[NPC], kCP32_4[NPC], kCP32_5[NPC];
 extern const ITFn kIT_0[NPC], kIT_1[NPC], kIT_2[NPC], kIT_3[NPC], kIT_4[NPC], kIT_5[NPC];
+extern const MXFn kMXD_0[NPC], kMXD_1[NPC], kMXD_2[NPC], kMXD_3[NPC], kMXD_4[NPC], kMXD_5[NPC];
 extern const G12Fn kG12_0[NPC], kG12_1[NPC], kG12_2[NPC], kG12_3[NPC], kG12_4[NPC], kG12_5[NPC];
 extern const MXFn kMX_0[NPC], kMX_1[NPC], kMX_2[NPC], kMX_3[NPC], kMX_4[NPC], kMX_5[NPC];
 
@@ -47,6 +48,7 @@ const CPFn *const kCP64[NPC] = {kCP64_0, kCP64_1, kCP64_2, kCP64_3, kCP64_4, kCP
 const CPFn *const kCP32[NPC] = {kCP32_0, kCP32_1, kCP32_2, kCP32_3, kCP32_4, kCP32_5, LGB_F_ROWS(kCPnone)};
 const ITFn *const kIT[NPC] = {kIT_0, kIT_1, kIT_2, kIT_3, kIT_4, kIT_5, LGB_F_ROWS(kITnone)};
 const MXFn *const kMX[NPC] = {kMX_0, kMX_1, kMX_2, kMX_3, kMX_4, kMX_5, LGB_F_ROWS(kMXnone)};
+const MXFn *const kMXD[NPC] = {kMXD_0, kMXD_1, kMXD_2, kMXD_3, kMXD_4, kMXD_5, LGB_F_ROWS(kMXnone)};
 const G12Fn *const kG12[NPC] = {kG12_0, kG12_1, kG12_2, kG12_3, kG12_4, kG12_5, LGB_F_ROWS(kG12none)};
 #undef LGB_F_ROWS
 
@@ -609,7 +611,8 @@ cudaError_t launch_it(int pcb, int pck, ITParams p, cudaStream_t s) {
 cudaError_t launch_mp2x(int pcb, int pck, MXParams p, cudaStream_t s) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (p.nbra <= 0 || p.nket <= 0) return cudaSuccess;
-  const MXFn f = kMX[pcb][pck];
+  // the split form in double-float (pairsd given)
+  const MXFn f = !p.X && p.pairsd && kMXD[pcb][pck] ? kMXD[pcb][pck] : kMX[pcb][pck];
   if (f) {
     const TileShape t = tile_shape({(double)p.nbra * p.nket, p.mean_prims, p.mean_prims, p.nbra, false});
     p.kets = t.kets;

@@ -1,0 +1,6 @@
+// MP2 transform input in double-float of bra pair class 5 (dd) for every ket pair class.
+#include "class_tables.cuh"
+
+namespace lgb {
+LGB_MXD_TABLE(5)
+}  // namespace lgb

@@ -346,6 +346,10 @@ struct MXParams {
   const PrimRec *prims;
   const PairRec *kpairs;  // ket pairs (species B; A's own list for one species)
   const PrimRec *kprims;
+  const PairRecD *pairsd = nullptr;    // double-float records, for the split form (null: FP64)
+  const PrimRecD *primsd = nullptr;
+  const PairRecD *kpairsd = nullptr;
+  const PrimRecD *kprimsd = nullptr;
   int bra0, nbra;
   int ket0, nket;
   const int *colbase;     // per pair record: first column of its components

@@ -146,7 +146,7 @@ struct MointWriter {
 // columns (lam sig) to B.
 struct MP2Setup {
   LibintInterface *A, *B;
-  const PairList *PA, *PB;
+  PairList *PA, *PB;
   bool coupling;
   double factor;
   int nA, nB, oA, vA, oB, vB, noccA, nfA, noccB, nfB;
@@ -361,6 +361,11 @@ bool mp2_split(MP2Setup &S, int np, size_t budget, double *e2out, cudaStream_t s
   MXParams q = S.q;
   q.colbase = dcolbase.p;
   q.X = nullptr;
+  if (!S.PA->upload_dd() || !S.PB->upload_dd()) return false;
+  q.pairsd = S.PA->dd;
+  q.primsd = S.PA->ddp;
+  q.kpairsd = S.PB->dd;
+  q.kprimsd = S.PB->ddp;
   for (int k = 0; k < kMaxPieces; ++k) q.Xp[k] = X.p[k].p;
   q.np = np;
   q.Kp = KA;
