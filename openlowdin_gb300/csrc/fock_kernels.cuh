@@ -931,8 +931,8 @@ __global__ void __launch_bounds__(128) it_kernel(ITParams P) {
 }
 
 // ------------------------------------------------------ MP2 transform input --
-// Warp y: bra pair tile_y * bras + y; its lanes: ket pairs tile_x * kets + (lane
-// mod kets) of the batch, 32 / kets lanes each.
+// Warp y: (lam sig) pair tile_y * bras + y of the batch; its lanes: (mu nu) pairs
+// tile_x * kets + (lane mod kets), 32 / kets lanes each.
 // R = dd32 writes the split-BF16 form only: the pieces hold at most the 24 bits of
 // an FP32 value, which double-float integrals (2^-45) round to as FP64 ones do.
 template <typename R, int LA, int LB, int LC, int LD>
@@ -971,8 +971,8 @@ __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) mp2x_
   R I[Q::NINT];
   eri_quartet<R, LA, LB, LC, LD>(bra, rb + bra.prim0, ket, rk + ket.prim0, P.boys.f64, P.boys.dd, I, part, parts, active);
   if (part || !active) return;
-  const int col0 = __ldg(P.colbase + ki) - P.col_first;
-  const bool two = bra.sa != bra.sb;
+  const int col0 = __ldg(P.colbase + bi) - P.col_first;
+  const bool two = ket.sa != ket.sb;
   const size_t n = P.n, ncol = P.ncol;
 #pragma unroll
   for (int a = 0; a < NA; ++a)
@@ -984,11 +984,11 @@ __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) mp2x_
         for (int d = 0; d < ND; ++d) {
           const R v = I[((a * NB + b) * NC + c) * ND + d];
           if (!above_cut(v, P.cut)) continue;
-          const size_t col = col0 + c * ND + d;
+          const size_t col = col0 + a * NB + b;
           if constexpr (!DD) {
             if (P.X) {
-              P.X[((bra.fa + a) * ncol + col) * n + bra.fb + b] = v;
-              if (two) P.X[((bra.fb + b) * ncol + col) * n + bra.fa + a] = v;
+              P.X[((ket.fa + c) * ncol + col) * n + ket.fb + d] = v;
+              if (two) P.X[((ket.fb + d) * ncol + col) * n + ket.fa + c] = v;
               continue;
             }
           }
@@ -999,8 +999,8 @@ __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) mp2x_
           __nv_bfloat16 pc[kMaxPieces];
           bf16_pieces(x, P.np, pc);   // three pieces hold the FP32 value exactly
           const size_t kp = P.Kp;
-          const size_t j1 = (col * kp + bra.fb + b) * kp + bra.fa + a;
-          const size_t j2 = (col * kp + bra.fa + a) * kp + bra.fb + b;
+          const size_t j1 = (col * kp + ket.fb + d) * kp + ket.fa + c;
+          const size_t j2 = (col * kp + ket.fa + c) * kp + ket.fb + d;
           for (int k = 0; k < P.np; ++k) {
             P.Xp[k][j1] = pc[k];
             if (two) P.Xp[k][j2] = pc[k];

@@ -414,24 +414,24 @@ __global__ void __launch_bounds__(128) mp2x_coop_kernel(MXParams P, GenClass K, 
     if (!abs_above(bra.Q * ket.Q * (1.0 - 1e-9), P.cut)) continue;
     if (P.screen && abs_below(bra.Q * ket.Q * dnorm6(P.Dn, P.nsh, bra.sa, bra.sb, ket.sa, ket.sb), P.eps)) continue;
     eri_coop(g, ct, Lo, K.la, K.lb, K.lc, K.ld, bra, P.prims, ket, P.kprims, P.boys.f64, sm);
-    const int col0 = __ldg(P.colbase + ki) - P.col_first;
-    const bool two = bra.sa != bra.sb;
+    const int col0 = __ldg(P.colbase + bi) - P.col_first;
+    const bool two = ket.sa != ket.sb;
     const size_t n = P.n, ncol = P.ncol;
     for (int t = lane; t < NA * NB * NC * ND; t += 32) {
       const int a = t / (NB * NC * ND), b = (t / (NC * ND)) % NB, c = (t / ND) % NC, d = t % ND;
       const double v = I[t];
       if (!abs_above(v, P.cut)) continue;
-      const size_t col = col0 + c * ND + d;
+      const size_t col = col0 + a * NB + b;
       if (P.X) {
-        P.X[((bra.fa + a) * ncol + col) * n + bra.fb + b] = v;
-        if (two) P.X[((bra.fb + b) * ncol + col) * n + bra.fa + a] = v;
+        P.X[((ket.fa + c) * ncol + col) * n + ket.fb + d] = v;
+        if (two) P.X[((ket.fb + d) * ncol + col) * n + ket.fa + c] = v;
       } else {
         // Xt[col * Kp + nu][mu] and the mirrored bra orientation
         __nv_bfloat16 pc[kMaxPieces];
         bf16_pieces((float)v, P.np, pc);   // three pieces hold the FP32 value exactly
         const size_t kp = P.Kp;
-        const size_t j1 = (col * kp + bra.fb + b) * kp + bra.fa + a;
-        const size_t j2 = (col * kp + bra.fa + a) * kp + bra.fb + b;
+        const size_t j1 = (col * kp + ket.fb + d) * kp + ket.fa + c;
+        const size_t j2 = (col * kp + ket.fa + c) * kp + ket.fb + d;
         for (int k = 0; k < P.np; ++k) {
           P.Xp[k][j1] = pc[k];
           if (two) P.Xp[k][j2] = pc[k];

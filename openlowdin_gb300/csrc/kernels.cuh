@@ -336,15 +336,18 @@ struct SchwarzParams {
   BoysTables boys;
 };
 
-// MP2 transform input: raw integrals (mu nu|lam sig) of every significant bra
-// pair and the ket pairs of one column batch, written to
-// X[mu][col][nu] (both bra orientations), col = colbase[ket pair] + c * ND + d
-// for ket components (c, d); quartets that the screening drops and raw values
-// with |v| <= cut stay at the zero the caller cleared X to.
+// MP2 transform input: raw integrals (mu nu|lam sig) of every significant (mu
+// nu) pair and the (lam sig) pairs of one column batch, written to X[mu][col][nu]
+// (both orientations of mu nu), col = colbase[pair] + a * NB + b for components
+// (a, b) of the (lam sig) pair; quartets that the screening drops and raw values
+// with |v| <= cut stay at the zero the caller cleared X to.  The (lam sig) pair is
+// the kernels' bra, the (mu nu) pairs run over the lanes: blocks in flight then
+// write few columns (1.5 MB each at 480 functions), which the L2 holds until
+// their sectors are full.
 struct MXParams {
-  const PairRec *pairs;   // bra pairs (species A)
+  const PairRec *pairs;   // (lam sig) pairs: the columns (species B; A's own list for one species)
   const PrimRec *prims;
-  const PairRec *kpairs;  // ket pairs (species B; A's own list for one species)
+  const PairRec *kpairs;  // (mu nu) pairs (species A)
   const PrimRec *kprims;
   const PairRecD *pairsd = nullptr;    // double-float records, for the split form (null: FP64)
   const PrimRecD *primsd = nullptr;

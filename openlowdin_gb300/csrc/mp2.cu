@@ -60,24 +60,24 @@ void mp2_columns(const PairList &P, long long colB, MP2Columns &mc) {
   mc.bfirst.push_back(npairs);
 }
 
-// integrals of every bra pair of PA against the ket pairs [k0, k1) of PB
+// integrals of every (mu nu) pair of PA with the column pairs [k0, k1) of PB
 bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, int k1, cudaStream_t s) {
   std::vector<Lanes::Job> jobs;
   double pa[kNumPairClasses];
   for (int c = 0; c < kNumPairClasses; ++c) pa[c] = PA.prims(c);
   for (int ck = 0; ck < kNumPairClasses; ++ck) {
     const int ka = std::max(k0, PB.start[ck]), kb = std::min(k1, PB.start[ck + 1]);
-    if (ka >= kb) continue;
-    for (int cb = 0; cb < kNumPairClasses; ++cb)
-      for (int b0 = PA.start[cb]; b0 < PA.start[cb + 1]; b0 += 65535 * kWarpsPerBlock) {  // grid y limit
-        q.bra0 = b0;
-        q.nbra = std::min(PA.start[cb + 1] - b0, 65535 * kWarpsPerBlock);
-        q.ket0 = ka;
-        q.nket = kb - ka;
-        q.mean_prims = pa[cb] * PB.prims(ck);
-        const MXParams p = q;
+    for (int c0 = ka; c0 < kb; c0 += 65535 * kWarpsPerBlock)   // grid y limit
+      for (int cb = 0; cb < kNumPairClasses; ++cb) {
+        if (!PA.count(cb)) continue;
+        MXParams p = q;
+        p.bra0 = c0;
+        p.nbra = std::min(kb - c0, 65535 * kWarpsPerBlock);
+        p.ket0 = PA.start[cb];
+        p.nket = PA.count(cb);
+        p.mean_prims = pa[cb] * PB.prims(ck);
         jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), false,
-                        [=](cudaStream_t z) { return launch_mp2x(cb, ck, p, z); }});
+                        [=](cudaStream_t z) { return launch_mp2x(ck, cb, p, z); }});
       }
   }
   Lanes lanes(s);
@@ -362,10 +362,10 @@ bool mp2_split(MP2Setup &S, int np, size_t budget, double *e2out, cudaStream_t s
   q.colbase = dcolbase.p;
   q.X = nullptr;
   if (!S.PA->upload_dd() || !S.PB->upload_dd()) return false;
-  q.pairsd = S.PA->dd;
-  q.primsd = S.PA->ddp;
-  q.kpairsd = S.PB->dd;
-  q.kprimsd = S.PB->ddp;
+  q.pairsd = S.PB->dd;
+  q.primsd = S.PB->ddp;
+  q.kpairsd = S.PA->dd;
+  q.kprimsd = S.PA->ddp;
   for (int k = 0; k < kMaxPieces; ++k) q.Xp[k] = X.p[k].p;
   q.np = np;
   q.Kp = KA;
@@ -514,10 +514,10 @@ bool mp2_coupling(LibintInterface *A, LibintInterface *B, const double *dCA, con
   // coupling integrals: no density screening (Libint2Iface.cpp:1296-1622),
   // quartets whose Schwarz bound is below the raw cut contribute nothing
   MXParams &q = S.q;
-  q.pairs = A->all.d;
-  q.prims = A->all.dp;
-  q.kpairs = B->all.d;
-  q.kprims = B->all.dp;
+  q.pairs = B->all.d;
+  q.prims = B->all.dp;
+  q.kpairs = A->all.d;
+  q.kprims = A->all.dp;
   q.screen = 0;
   q.eps = 0.0;
   q.cut = 1e-10;
