@@ -48,6 +48,13 @@ __global__ void prepare_density_kernel(const double *__restrict__ D, const doubl
   }
 }
 
+// clears up to kClearMax arrays (lengths in 4-byte words)
+__global__ void clear_kernel(ClearList L) {
+  for (int k = 0; k < L.n; ++k)
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < L.words[k]; i += (size_t)gridDim.x * blockDim.x)
+      L.p[k][i] = 0u;
+}
+
 __global__ void scale_density_kernel(const double *__restrict__ D, const double *__restrict__ norma, int n,
                                      double *__restrict__ Ds, float *__restrict__ Ds32) {
   const size_t nn = (size_t)n * n;
@@ -307,8 +314,6 @@ cudaError_t launch_dn_max_batch(const SpeciesSlot *slots, int nslots, int max_ns
 }
 
 cudaError_t launch_dn_max(const float *Dn32, int nsh, float *out, cudaStream_t s) {
-  const cudaError_t e = cudaMemsetAsync(out, 0, sizeof(float), s);
-  if (e != cudaSuccess) return e;
   dn_max_kernel<<<dn_max_grid(nsh), 256, 0, s>>>(Dn32, nsh, out);
   count_launches(1);
   return cudaGetLastError();
@@ -356,15 +361,27 @@ cudaError_t measure_fma_tflops(bool fp64, double *tflops) {
 }
 
 cudaError_t launch_prepare_density(const double *D, const double *norma, const int *shell_of, int n, int nsh,
-                                   double *Ds, float *Ds32, float2 *Dd, double *Dn, float *Dn32, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(Dn, 0, sizeof(double) * nsh * nsh, s);
-  if (e != cudaSuccess) return e;
-  if (Dn32) {
-    e = cudaMemsetAsync(Dn32, 0, sizeof(float) * nsh * nsh, s);
+                                   double *Ds, float *Ds32, float2 *Dd, double *Dn, float *Dn32, cudaStream_t s,
+                                   bool cleared) {
+  if (!cleared) {
+    cudaError_t e = cudaMemsetAsync(Dn, 0, sizeof(double) * nsh * nsh, s);
     if (e != cudaSuccess) return e;
+    if (Dn32) {
+      e = cudaMemsetAsync(Dn32, 0, sizeof(float) * nsh * nsh, s);
+      if (e != cudaSuccess) return e;
+    }
   }
   prepare_density_kernel<<<grid_for((size_t)n * n, 256), 256, 0, s>>>(D, norma, shell_of, n, nsh, Ds, Ds32, Dd,
                                                                       Dn, Dn32);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_clear(const ClearList &L, cudaStream_t s) {
+  size_t most = 0;
+  for (int k = 0; k < L.n; ++k) most = L.words[k] > most ? L.words[k] : most;
+  if (!most) return cudaSuccess;
+  clear_kernel<<<grid_for((most + 3) / 4, 256), 256, 0, s>>>(L);
   count_launches(1);
   return cudaGetLastError();
 }

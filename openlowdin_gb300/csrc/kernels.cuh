@@ -224,9 +224,15 @@ struct CPTask {
 // 41.7 -> 18.2 ms.
 enum class Tier { all, upper, lower };
 constexpr float kTierBound = 1.f / 4096;
+// Mixed builds, whose quartets below the split are evaluated in FP32 anyway (1e-5
+// times 2^-22), take the double-float tier up to 1/16 of the largest bound; a
+// system held in FP64 for its check keeps kTierBound.  724-function chain, a
+// later iteration's density change: 40.1 -> 34.1 ms.
+constexpr float kMixedTier = 256.f;
 // candidate quartets of a class below which one FP64 launch is shorter than two
-// launches (one water, 120 to 14,000 a class: 116 us in one, 163 us in two)
-constexpr double kTierMinQuartets = 2e5;
+// launches (one water, 120 to 14,000 a class: 116 us in one, 163 us in two; four
+// waters with d: 1.09 ms with the line at 2e5, 1.00 at 5e4, 1.02 at 2e4)
+constexpr double kTierMinQuartets = 5e4;
 
 struct TaskLaunch {
   int ntasks;
@@ -427,7 +433,22 @@ inline bool class_generic(int pcb, int pck) {
 
 // small kernels (the *32 arguments may be null)
 cudaError_t launch_prepare_density(const double *D, const double *norma, const int *shell_of, int n, int nsh,
-                                   double *Ds, float *Ds32, float2 *Dd, double *Dn, float *Dn32, cudaStream_t s);
+                                   double *Ds, float *Ds32, float2 *Dd, double *Dn, float *Dn32, cudaStream_t s,
+                                   bool cleared = false);   // cleared: Dn and Dn32 are zero already
+// zero arrays in one launch (a small build is as long as its launches: six
+// memsets of a few KB took a sixth of it)
+constexpr int kClearMax = 6;
+struct ClearList {
+  unsigned *p[kClearMax];
+  size_t words[kClearMax];
+  int n = 0;
+  template <typename T>
+  void add(T *q, size_t count) {
+    p[n] = reinterpret_cast<unsigned *>(q);
+    words[n++] = count * sizeof(T) / 4;
+  }
+};
+cudaError_t launch_clear(const ClearList &L, cudaStream_t s);
 cudaError_t launch_scale_density(const double *D, const double *norma, int n, double *Ds, float *Ds32,
                                  cudaStream_t s);
 cudaError_t launch_symmetrize(const double *Gacc, const float *Gacc32, const double *norma, int n, double scale,
@@ -459,7 +480,7 @@ cudaError_t launch_prepare_batch(const SpeciesSlot *slots, int nslots, long long
 // Dnmax32 of every slot that has Dn32 (after launch_prepare_batch; the
 // Dnmax32 values must be zero beforehand); max_nsh: largest nsh of a slot
 cudaError_t launch_dn_max_batch(const SpeciesSlot *slots, int nslots, int max_nsh, cudaStream_t s);
-// *out = max of Dn32[0 .. nsh * nsh) (set to zero here first)
+// *out = max of *out (zero beforehand) and Dn32[0 .. nsh * nsh)
 cudaError_t launch_dn_max(const float *Dn32, int nsh, float *out, cudaStream_t s);
 
 // pair-indexed copies of a species' FP32 density for the FP32 row kernels:

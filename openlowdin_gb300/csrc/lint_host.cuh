@@ -673,11 +673,16 @@ struct LibintInterface {
       jk_hf = 0.5 * factor;
       jk_ready = true;
     }
-    CK(launch_prepare_density(dDin, d_norma, d_shell_of, n, nsh, dDs.p, dDs32.p, dDd.p, dDn.p, dDn32.p, s));
+    ClearList z;
+    z.add(dDn.p, (size_t)nsh * nsh);
+    z.add(dDn32.p, (size_t)nsh * nsh);
+    z.add(dDnmax32.p, 1);
+    z.add(dGacc.p, (size_t)n * n);
+    z.add(dGacc32.p, (size_t)n * n);
+    z.add(dcount.p, kNQC);
+    CK(launch_clear(z, s));
+    CK(launch_prepare_density(dDin, d_norma, d_shell_of, n, nsh, dDs.p, dDs32.p, dDd.p, dDn.p, dDn32.p, s, true));
     CK(launch_dn_max(dDn32.p, nsh, dDnmax32.p, s));
-    CK(cudaMemsetAsync(dGacc.p, 0, sizeof(double) * n * n, s));
-    CK(cudaMemsetAsync(dGacc32.p, 0, sizeof(float) * n * n, s));
-    CK(cudaMemsetAsync(dcount.p, 0, sizeof(unsigned long long) * kNQC, s));
     if (precision != 0) CK(launch_pair_gather(dpslot.p, 1, (long long)sig.h.size(), s));
     {
       Lanes lanes(s);
