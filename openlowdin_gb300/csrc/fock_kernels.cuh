@@ -86,7 +86,7 @@ __device__ __forceinline__ bool above_cut(double v, double cut) { return abs_abo
 __device__ __forceinline__ bool above_cut(dd32 v, double cut) {
   const float a = fabsf(fadd(v.hi, v.lo)), c = (float)cut;
   if (fabsf(a - c) <= 1e-5f * c) return abs_above(to_double(v), cut);   // too near for FP32
-  return a > c;
+  return !(a <= c);   // NaN is kept, as abs_above keeps it
 }
 
 // element i of a matrix kept in FP64, FP32 and double-float

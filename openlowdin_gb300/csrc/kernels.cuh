@@ -217,11 +217,11 @@ struct CPTask {
 // some 2^-45, times a bound below kTierBound of the largest stays below the
 // FP64 rounding of the sums that the largest quartets go into.  Error of the
 // two-particle matrix against an 80-bit evaluation (2-norm over 2-norm), FP64
-// alone -> two tiers: 4 waters (136 functions) 3.0e-15 -> 2.8e-15, 176-function
-// chain 6.0e-15 -> 4.8e-15, 3 waters with d 3.9e-15 -> 3.6e-15, 12 protons
+// alone -> two tiers: 4 waters (136 functions) 3.0e-15 -> 3.0e-15, 176-function
+// chain 6.0e-15 -> 4.8e-15, 3 waters with d 3.9e-15 -> 3.5e-15, 12 protons
 // 1.6e-14 -> 1.6e-14 (the sums of eight ket tiles at a time that came with it
 // round less often).  387-function chain (5 % of the quartets above the bound):
-// 41.7 -> 18.2 ms.
+// 41.7 -> 17.9 ms.
 enum class Tier { all, upper, lower };
 constexpr float kTierBound = 1.f / 4096;
 // Mixed builds, whose quartets below the split are evaluated in FP32 anyway (1e-5
