@@ -24,7 +24,7 @@ Sections of the JSON line:
                        the reference program's calling pattern, FP64), the
                        MP2 of MP2 requests through LowdinGB300_mp2_direct with
                        host-resident orbitals copied in.
-  roofline          -- the FP64 J/K kernels (one plain build of the stream's
+  roofline          -- the plain J/K kernels (one plain build of the stream's
                        largest molecule, CUDA events) against the FP64 FMA
                        peak measured in the run; the FP32 row kernels beside.
   cpu_baseline      -- the oracle port (C/OpenMP, all host threads) on every
@@ -445,8 +445,8 @@ def mp2_profile_case(args):
 
 
 def mp2_section(args):
-    """MP2 four-index transform of a d-shell water cluster: FP64 (cuBLAS
-    DGEMM) vs split-BF16 tensor cores (3 pieces, 8 products), same SCF
+    """MP2 four-index transform of a d-shell water cluster: FP64 matrix
+    instructions vs split-BF16 tensor cores (3 pieces, 8 products), same SCF
     orbitals; plus the tensor-core GEMM engine alone on the transform's
     first-quarter shape."""
     import numpy as np
@@ -579,8 +579,8 @@ def apmo_batch_section(args, dev):
 
 # --------------------------------------------------------------- roofline --
 def roofline_section(sysd):
-    """FP64 J/K kernels: one plain Fock build of `sysd` at its core-guess
-    density (CUDA events on the launching stream, 3 builds), FLOPs from the
+    """Plain J/K kernels (FP64 and double-float tiers): one plain Fock build of
+    `sysd` at its core-guess density (CUDA events on the launching stream, 3 builds), FLOPs from the
     frozen per-class model over the quartets the build evaluated, against the
     FP64 FMA throughput measured in this run.  Beside it the FP32 row kernels:
     the same build with every quartet in FP32 (split above every bound)."""
@@ -628,7 +628,9 @@ def roofline_section(sysd):
             traffic = None
     return {"bound": "fp64", "achieved": f64["achieved_tflops"], "peak": peak64, "unit": "TFLOP/s",
             "frac": f64["achieved_tflops"] / peak64 if peak64 > 0 else None, "traffic": traffic,
-            "kernel": "jk_tasks_kernel<double> (every J/K class launch of one plain FP64 Fock build)",
+            "kernel": "jk_tasks_kernel<double> for the quartets above 2^-12 of the largest bound and "
+                      "jk_tasks_kernel<dd32> (double-float, on the FP32 pipe) below it: every J/K class launch of "
+                      "one plain Fock build; the fraction of the FP64 peak can therefore exceed 1",
             "system": f"chain molecule, {S.nbasis(sysd['species'][0])} functions (largest request of the stream)",
             "ms_per_build": f64["ms_per_build"], "quartets": f64["quartets"], "flop_per_build": f64["flop_per_build"],
             "peak_source": "FP64 FMA throughput measured on this GPU in this run (LowdinGB300_measure_fma_tflops: "

@@ -235,7 +235,8 @@ int LowdinGB300_batch_set_active(LowdinGB300_Batch *b, const int *flags, void *s
 /* precision bits: 1 = two-particle quartets whose Schwarz-density bound
    Q_ab Q_cd max|D block| is below `split` run in FP32 (the rest FP64); 2 = the
    same split for coupling quartets (bound Q_ab Q_cd max(|D_A|, |D_B|)).
-   0 = FP64 throughout. */
+   0 = every quartet to FP64 accuracy (quartets below 2^-12 of the largest bound
+   in double-float on the FP32 pipe, added into FP64 sums). */
 int LowdinGB300_batch_fock(LowdinGB300_Batch *b, int precision, double split, void *stream);
 /* Mixed builds (precision != 0) also drop the quartets whose density-weighted
    bound (the FP32 bound of the split) is below `skip`: with incremental
@@ -293,12 +294,13 @@ int LowdinGB300_twobody_device_noalloc(LibintInterface *lint, const double *dD, 
    coefficients, row p = orbital p (the layout LibintInterface_compute_2body_directIT
    reads); eps: host orbital energies (n); orbitals [n_frozen, n_occ) are the
    active occupied ones, [n_occ, n) the virtual ones.  precision 0: FP64
-   throughout (cuBLAS DGEMM for the dense contractions); 1 / 2: the four dense
+   throughout (own FP64 matrix kernels for the dense contractions); 1 / 2: the four dense
    contractions as split-BF16 tensor-core products, operands in 2 / 3 BF16
    pieces (LowdinGB300_gemm_bf16_split's engine; with 3 pieces the first
-   quarter uses LowdinGB300_gemm_bf16_precise's), integrals and the energy sum
-   in FP64.  x_budget_gb bounds the per-batch integral array (0: 8 GB).  Writes E_MP2 to *e2 (host) and
-   synchronises `stream`.  Returns 0, or -1 with LowdinGB300_last_error() set. */
+   quarter uses LowdinGB300_gemm_bf16_precise's), integrals in FP64 or
+   double-float (they end in at most 24 bits) and the energy sum in FP64.
+   x_budget_gb bounds the per-batch integral array (0: 8 GB).  Writes E_MP2 to
+   *e2 (host) and synchronises `stream`.  Returns 0, or -1 with LowdinGB300_last_error() set. */
 int LowdinGB300_mp2_direct(LibintInterface *lint, const double *dD, const double *dC, const double *eps,
                            int n_occ, int n_frozen, int precision, double x_budget_gb, double *e2, void *stream);
 /* Inter-species MP2 term of species a and b (APMO; replaces the two-species
