@@ -72,10 +72,7 @@ struct PairList {
   PairRecD *dd = nullptr;     // double-float copies
   PrimRecD *ddp = nullptr;
   void release() {
-    if (dd) cudaFree(dd);
-    if (ddp) cudaFree(ddp);
-    dd = nullptr;
-    ddp = nullptr;
+    release_dd();
     if (d) cudaFree(d);
     if (dp) cudaFree(dp);
     if (d32) cudaFree(d32);
@@ -104,9 +101,16 @@ struct PairList {
     release();
     return dev_upload(d, h) && dev_upload(dp, hp);
   }
-  // uploads the double-float copies (the first J/K build asks for them)
+  void release_dd() {
+    if (dd) cudaFree(dd);
+    if (ddp) cudaFree(ddp);
+    dd = nullptr;
+    ddp = nullptr;
+  }
+  // uploads the double-float copies (the first J/K build asks for them), both
+  // or none: a kernel that is given the pairs reads their primitives too
   bool upload_dd() {
-    if (dd) return true;
+    if (dd && ddp) return true;
     std::vector<PairRecD> hd(h.size());
     std::vector<PrimRecD> hpd(hp.size());
     for (size_t i = 0; i < h.size(); ++i) {
@@ -134,7 +138,9 @@ struct PairList {
         c.P[k][2] = (float)(a.P[k] - (double)h2.hi - (double)h2.lo);
       }
     }
-    return dev_upload(dd, hd) && dev_upload(ddp, hpd);
+    if (dev_upload(dd, hd) && dev_upload(ddp, hpd)) return true;
+    release_dd();
+    return false;
   }
   // uploads the FP64 records and their FP32 copies
   bool upload() {
