@@ -247,19 +247,15 @@ struct LowdinGB300_Batch {
       drop_graphs();
       tasks_dirty = false;
     }
-    if (!use_graph || calls++ == 0) {
-      Lanes lanes(s);
-      return fock_sequence(precision, split, s, lanes);
-    }
+    if (!use_graph || calls++ == 0) return fock_sequence(precision, split, s);
     Graph &g = graphs[precision & 3];
     if (!g.exec || g.split != split || g.skip != skip) {
       if (g.exec) cudaGraphExecDestroy(g.exec);
       g = Graph{};
       if (!capture) CK(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking));
       const long long l0 = launch_count();
-      Lanes lanes(capture, true);   // held until the capture has ended
       CK(cudaStreamBeginCapture(capture, cudaStreamCaptureModeThreadLocal));
-      const bool ok = fock_sequence(precision, split, capture, lanes);
+      const bool ok = fock_sequence(precision, split, capture);
       cudaGraph_t graph = nullptr;
       const cudaError_t e = cudaStreamEndCapture(capture, &graph);
       const long long captured = launch_count() - l0;
@@ -330,10 +326,10 @@ struct LowdinGB300_Batch {
       for (int v = 1; v >= 0 && ok; --v) {
         signed char pref[kNQC];
         for (int k = 0; k < kNQC; ++k) pref[k] = (signed char)v;
-        ok = LibintInterface::launch_jk_groups(jk, 1, split, boys, s, skip, pref, c, true);
+        ok = LibintInterface::launch_jk_groups(jk, 1, split, boys, s, false, skip, pref, c, true);
         if (!ok) break;
         if (cudaEventRecord(e0, s) != cudaSuccess) ok = false;
-        for (int r = 0; r < 2 && ok; ++r) ok = LibintInterface::launch_jk_groups(jk, 1, split, boys, s, skip, pref, c, true);
+        for (int r = 0; r < 2 && ok; ++r) ok = LibintInterface::launch_jk_groups(jk, 1, split, boys, s, false, skip, pref, c, true);
         if (ok && (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
                    cudaEventElapsedTime(&ms[v], e0, e1) != cudaSuccess))
           ok = false;
@@ -364,7 +360,7 @@ struct LowdinGB300_Batch {
   }
 
   // every launch of one build, in stream order
-  bool fock_sequence(int precision, double split, cudaStream_t s, Lanes &lanes) {
+  bool fock_sequence(int precision, double split, cudaStream_t s) {
     CK(cudaMemsetAsync(Dn.p, 0, Dn.n * sizeof(double), s));
     CK(cudaMemsetAsync(Dn32.p, 0, Dn32.n * sizeof(float), s));
     CK(cudaMemsetAsync(cnt.p, 0, 2 * kNQC * sizeof(unsigned long long), s));
@@ -373,11 +369,10 @@ struct LowdinGB300_Batch {
     CK(cudaMemsetAsync(Dnmax32.p, 0, Dnmax32.n * sizeof(float), s));
     CK(launch_dn_max_batch(slots.p, nslots, max_nsh, s));
     if (jk_mixed && npslots) CK(launch_pair_gather(pslots.p, npslots, ptotal, s));
-    if (!LibintInterface::launch_jk_groups(jk, jk_mixed, jk_mixed ? split : 0.0, boys, s, skip, rows_choice,
-                                           -1, false, &lanes))
+    if (!LibintInterface::launch_jk_groups(jk, jk_mixed, jk_mixed ? split : 0.0, boys, s, true, skip, rows_choice))
       return false;
     if (jk_mixed && npslots) CK(launch_pair_scatter(pslots.p, npslots, ptotal, s));
-    if (!launch_cp_groups(cp, (precision & 2) ? 2 : 0, split, boys, s, skip, &lanes)) return false;
+    if (!launch_cp_groups(cp, (precision & 2) ? 2 : 0, split, boys, s, skip)) return false;
     CK(launch_finalize_batch(slots.p, nslots, total, s));
     return true;
   }

@@ -248,6 +248,7 @@ constexpr int jk_min_blocks() {
 }
 template <typename R, int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) jk_tasks_kernel(const JKTask *__restrict__ tasks, TaskLaunch TL) {
+  if (beside_block()) return;
   using Q = QClass<LA, LB, LC, LD>;
   constexpr bool F64 = std::is_same<R, double>::value, DD = std::is_same<R, dd32>::value;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
@@ -448,6 +449,7 @@ __device__ __forceinline__ int find_task_rows(const T *__restrict__ tasks, int n
 
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(32 * kRowWarps) jk32_row_kernel(const JKTask *__restrict__ tasks, TaskLaunch TL) {
+  if (beside_block()) return;
   using Q = QClass<LA, LB, LC, LD>;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND, NR = NA + NB, NRP = row_pitch(NA + NB);
   extern __shared__ float rsm[];
@@ -671,6 +673,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) jk32_row_kernel(const JKTask *
 // where one takes 249 (six waters).
 template <typename R, int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128) cp_tasks_kernel(const CPTask *__restrict__ tasks, TaskLaunch TL) {
+  if (beside_block()) return;
   using Q = QClass<LA, LB, LC, LD>;
   constexpr bool F64 = std::is_same<R, double>::value;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
@@ -808,6 +811,7 @@ __global__ void __launch_bounds__(128) cp_tasks_kernel(const CPTask *__restrict_
 // kernel, 0.20 ms so.
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128) g12_kernel(G12Params P) {
+  if (beside_block()) return;
   using Q = QClass<LA, LB, LC, LD>;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
   const int kets = P.kets, parts = 32 / kets, part = threadIdx.x / kets, bras = blockDim.y;
@@ -882,6 +886,7 @@ __device__ __forceinline__ void it_role(F &&val, const double *__restrict__ Cs, 
 
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128) it_kernel(ITParams P) {
+  if (beside_block()) return;
   using Q = QClass<LA, LB, LC, LD>;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
   const int kets = P.kets, parts = 32 / kets, bras = blockDim.y;
@@ -938,6 +943,7 @@ __global__ void __launch_bounds__(128) it_kernel(ITParams P) {
 // an FP32 value, which double-float integrals (2^-45) round to as FP64 ones do.
 template <typename R, int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) mp2x_kernel(MXParams P) {
+  if (beside_block()) return;
   using Q = QClass<LA, LB, LC, LD>;
   constexpr bool DD = std::is_same<R, dd32>::value;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;

@@ -93,10 +93,11 @@ __device__ __forceinline__ const Task &coop_unit(const Task *tasks, const TaskLa
                     : smem + (size_t)warp * Lo.total;                     \
   const double *I = sm + Lo.out;                                          \
   const WarpGroup g;                                                      \
-  const long long w0 = (long long)blockIdx.x * nwarps + warp, wstep = (long long)gridDim.x * nwarps;
+  const long long w0 = (long long)blockIdx.x * nwarps + warp, wstep = (long long)besides() * nwarps;
 
 // ------------------------------------------------------------------ J/K --
 __global__ void __launch_bounds__(128) jk_coop_kernel(const JKTask *__restrict__ tasks, TaskLaunch TL, GenClass K, double *gscr) {
+  if (beside_block()) return;
   LGB_COOP_PROLOGUE(K)
   const int NA = ncart(K.la), NB = ncart(K.lb), NC = ncart(K.lc), ND = ncart(K.ld);
   for (long long u = w0; u < (long long)TL.nblocks * TL.tile.slices; u += wstep) {
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(128) jk_coop_kernel(const JKTask *__restrict__
 
 // ------------------------------------------------------------- coupling --
 __global__ void __launch_bounds__(128) cp_coop_kernel(const CPTask *__restrict__ tasks, TaskLaunch TL, GenClass K, double *gscr) {
+  if (beside_block()) return;
   LGB_COOP_PROLOGUE(K)
   const int NA = ncart(K.la), NB = ncart(K.lb), NC = ncart(K.lc), ND = ncart(K.ld);
   for (long long u = w0; u < (long long)TL.nblocks * TL.tile.slices; u += wstep) {
@@ -251,6 +253,7 @@ __global__ void __launch_bounds__(128) cp_coop_kernel(const CPTask *__restrict__
 // shells): one quartet per warp, all quartets of the launch's bra x ket pair
 // ranges, no screening.
 __global__ void __launch_bounds__(128) g12_coop_kernel(G12Params P, GenClass K, double *gscr) {
+  if (beside_block()) return;
   LGB_COOP_PROLOGUE(K)
   const int NA = ncart(K.la), NB = ncart(K.lb), NC = ncart(K.lc), ND = ncart(K.ld);
   const long long nq = (long long)P.nbra * P.nket;
@@ -356,6 +359,7 @@ __device__ __forceinline__ void it_map(int r, int mu, int nu, int l, int s, int 
 }
 
 __global__ void __launch_bounds__(128) it_coop_kernel(ITParams P, GenClass K, double *gscr) {
+  if (beside_block()) return;
   LGB_COOP_PROLOGUE(K)
   const int NA = ncart(K.la), NB = ncart(K.lb), NC = ncart(K.lc), ND = ncart(K.ld);
   const long long nq = (long long)P.nbra * P.nket;
@@ -404,6 +408,7 @@ __global__ void __launch_bounds__(128) it_coop_kernel(ITParams P, GenClass K, do
 
 // ------------------------------------------------------ MP2 transform input --
 __global__ void __launch_bounds__(128) mp2x_coop_kernel(MXParams P, GenClass K, double *gscr) {
+  if (beside_block()) return;
   LGB_COOP_PROLOGUE(K)
   const int NB = ncart(K.lb), NC = ncart(K.lc), ND = ncart(K.ld), NA = ncart(K.la);
   const long long nq = (long long)P.nbra * P.nket;
@@ -443,6 +448,7 @@ __global__ void __launch_bounds__(128) mp2x_coop_kernel(MXParams P, GenClass K, 
 
 // ----------------------------------------------------------------- Schwarz --
 __global__ void __launch_bounds__(128) schwarz_coop_kernel(SchwarzParams P, GenClass K, double *gscr) {
+  if (beside_block()) return;
   LGB_COOP_PROLOGUE(K)
   const int N = ncart(K.la) * ncart(K.lb);
   for (long long t = w0; t < P.np; t += wstep) {
@@ -501,22 +507,21 @@ CoopShape coop_shape(const GenClass &K, long long units) {
   return CoopShape{dim3((unsigned)ctas), dim3((unsigned)(32 * w)), per * w, 0};
 }
 
-// launches kernel `f` with shape c on stream s, with its global scratch when
-// the shape asks for one (stream-ordered allocation, freed after the launch)
+// launches kernel `f` with shape c, with its global scratch when the shape asks
+// for one: a share of the group's, or a stream-ordered allocation of its own
 template <typename F, typename... Args>
-cudaError_t coop_launch(F f, const CoopShape &c, cudaStream_t s, Args... args) {
+cudaError_t coop_launch(F f, const CoopShape &c, Queue &q, Args... args) {
+  if (q.sizing || !c.scratch || q.scratch) {
+    double *scr = c.scratch ? q.scratch + q.need : nullptr;
+    q.need += c.scratch;
+    return launch_beside(q, f, c.grid, c.block, c.smem, args..., scr);
+  }
   double *scr = nullptr;
-  if (c.scratch) {
-    const cudaError_t e = cudaMallocAsync((void **)&scr, c.scratch * sizeof(double), s);
-    if (e != cudaSuccess) return e;
-  }
-  f<<<c.grid, c.block, c.smem, s>>>(args..., scr);
-  cudaError_t e = cudaGetLastError();
-  if (scr) {
-    const cudaError_t e2 = cudaFreeAsync(scr, s);
-    if (e == cudaSuccess) e = e2;
-  }
-  return e;
+  const cudaError_t e = cudaMallocAsync((void **)&scr, c.scratch * sizeof(double), q.s);
+  if (e != cudaSuccess) return e;
+  const cudaError_t e1 = launch_beside(q, f, c.grid, c.block, c.smem, args..., scr);
+  const cudaError_t e2 = cudaFreeAsync(scr, q.s);
+  return e1 == cudaSuccess ? e2 : e1;
 }
 
 }  // namespace
@@ -531,10 +536,12 @@ bool jk_rows_used(int pcb, int pck, int n, int nsh) {
   return row_smem_bytes(ncart(pc_la(pcb)) + ncart(pc_lb(pcb)), n, nsh) <= (size_t)kRowMaxSmem;
 }
 
+bool jk_fp32_class(int pcb, int pck) { return class_supported(pcb, pck) && kJK32[pcb][pck]; }
+bool cp_fp32_class(int pcb, int pck) { return class_supported(pcb, pck) && kCP32[pcb][pck]; }
 bool jk_dd_class(int pcb, int pck) { return class_supported(pcb, pck) && kJKD[pcb][pck]; }
 
 cudaError_t launch_jk_tasks(int pcb, int pck, Arith arith, const JKTask *dtasks, const TaskLaunch &tl,
-                            cudaStream_t s) {
+                            Queue &q) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (tl.ntasks <= 0 || tl.nblocks <= 0) return cudaSuccess;
   const bool fp32 = arith == Arith::f32;
@@ -549,66 +556,69 @@ cudaError_t launch_jk_tasks(int pcb, int pck, Arith arith, const JKTask *dtasks,
       });
       if (e != cudaSuccess) return e;
     }
-    if (tl.nrblocks > 0) r<<<tl.nrblocks, 32 * kRowWarps, smem, s>>>(dtasks, tl);
-    count_launches(1);
-    return cudaGetLastError();
+    if (tl.nrblocks <= 0) return cudaSuccess;
+    count_launches(q.sizing ? 0 : 1);
+    return launch_beside(q, r, tl.nrblocks, 32 * kRowWarps, smem, dtasks, tl);
   }
   // a class without an FP32 kernel is evaluated in FP64 in the FP32 half too
   const JKFn f = arith == Arith::dd ? kJKD[pcb][pck]
                  : fp32 && kJK32[pcb][pck] ? kJK32[pcb][pck]
                                            : kJK64[pcb][pck];
   if (f) {
-    f<<<tl.nblocks * tl.tile.slices, dim3(32, tl.tile.bras), 0, s>>>(dtasks, tl);
+    const cudaError_t e = launch_beside(q, f, tl.nblocks * tl.tile.slices, dim3(32, tl.tile.bras), 0, dtasks, tl);
+    if (e != cudaSuccess) return e;
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K = gen_class(pcb, pck);
     const CoopShape c = coop_shape(K, (long long)tl.nblocks * tl.tile.slices);
-    const cudaError_t e = coop_launch(jk_coop_kernel, c, s, dtasks, tl, K);
+    const cudaError_t e = coop_launch(jk_coop_kernel, c, q, dtasks, tl, K);
     if (e != cudaSuccess) return e;
   }
-  count_launches(1);
-  return cudaGetLastError();
+  count_launches(q.sizing ? 0 : 1);
+  return cudaSuccess;
 }
 
 cudaError_t launch_cp_tasks(int pcb, int pck, bool fp32, const CPTask *dtasks, const TaskLaunch &tl,
-                            cudaStream_t s) {
+                            Queue &q) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (tl.ntasks <= 0 || tl.nblocks <= 0) return cudaSuccess;
   const CPFn f = fp32 && kCP32[pcb][pck] ? kCP32[pcb][pck] : kCP64[pcb][pck];
   if (f) {
-    f<<<tl.nblocks, dim3(32, tl.tile.bras), 0, s>>>(dtasks, tl);
+    const cudaError_t e = launch_beside(q, f, tl.nblocks, dim3(32, tl.tile.bras), 0, dtasks, tl);
+    if (e != cudaSuccess) return e;
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K = gen_class(pcb, pck);
     const CoopShape c = coop_shape(K, (long long)tl.nblocks * tl.tile.slices);
-    const cudaError_t e = coop_launch(cp_coop_kernel, c, s, dtasks, tl, K);
+    const cudaError_t e = coop_launch(cp_coop_kernel, c, q, dtasks, tl, K);
     if (e != cudaSuccess) return e;
   }
-  count_launches(1);
-  return cudaGetLastError();
+  count_launches(q.sizing ? 0 : 1);
+  return cudaSuccess;
 }
 
-cudaError_t launch_it(int pcb, int pck, ITParams p, cudaStream_t s) {
+cudaError_t launch_it(int pcb, int pck, ITParams p, Queue &q) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (p.nbra <= 0 || p.nket <= 0) return cudaSuccess;
   const ITFn f = kIT[pcb][pck];
   if (f) {
     const TileShape t = tile_shape({(double)p.nbra * p.nket, p.mean_prims, p.mean_prims, p.nbra, false});
     p.kets = t.kets;
-    f<<<dim3((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras)), dim3(32, t.bras),
-        0, s>>>(p);
+    const dim3 grid((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras));
+    const cudaError_t e = launch_beside(q, f, grid, dim3(32, t.bras), 0, p);
+    if (e != cudaSuccess) return e;
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K = gen_class(pcb, pck);
     const CoopShape c = coop_shape(K, (long long)p.nbra * p.nket);
-    const cudaError_t e = coop_launch(it_coop_kernel, c, s, p, K);
+    const cudaError_t e = coop_launch(it_coop_kernel, c, q, p, K);
     if (e != cudaSuccess) return e;
   }
-  count_launches(1);
-  return cudaGetLastError();
+  count_launches(q.sizing ? 0 : 1);
+  return cudaSuccess;
 }
 
-cudaError_t launch_mp2x(int pcb, int pck, MXParams p, cudaStream_t s) {
+cudaError_t launch_mp2x(int pcb, int pck, MXParams p, Queue &q) {
   if (!class_supported(pcb, pck)) return cudaErrorNotSupported;
   if (p.nbra <= 0 || p.nket <= 0) return cudaSuccess;
   // the split form in double-float (pairsd given)
@@ -616,38 +626,39 @@ cudaError_t launch_mp2x(int pcb, int pck, MXParams p, cudaStream_t s) {
   if (f) {
     const TileShape t = tile_shape({(double)p.nbra * p.nket, p.mean_prims, p.mean_prims, p.nbra, false});
     p.kets = t.kets;
-    f<<<dim3((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras)), dim3(32, t.bras),
-        0, s>>>(p);
+    const dim3 grid((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras));
+    const cudaError_t e = launch_beside(q, f, grid, dim3(32, t.bras), 0, p);
+    if (e != cudaSuccess) return e;
   } else {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K = gen_class(pcb, pck);
     const CoopShape c = coop_shape(K, (long long)p.nbra * p.nket);
-    const cudaError_t e = coop_launch(mp2x_coop_kernel, c, s, p, K);
+    const cudaError_t e = coop_launch(mp2x_coop_kernel, c, q, p, K);
     if (e != cudaSuccess) return e;
   }
-  count_launches(1);
-  return cudaGetLastError();
+  count_launches(q.sizing ? 0 : 1);
+  return cudaSuccess;
 }
 
-cudaError_t launch_g12(int pcb, int pck, G12Params p, cudaStream_t s) {
+cudaError_t launch_g12(int pcb, int pck, G12Params p, Queue &q) {
   if (!class_supported(pcb, pck) || !p.gem) return cudaErrorNotSupported;
   if (p.nbra <= 0 || p.nket <= 0) return cudaSuccess;
   const TileShape t = tile_shape({(double)p.nbra * p.nket, p.mean_prims, p.mean_prims, p.nbra, false});
   const G12Fn f = kG12[pcb][pck];
   if (f && (p.nbra + t.bras - 1) / t.bras <= 65535) {
     p.kets = t.kets;
-    f<<<dim3((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras)), dim3(32, t.bras),
-        0, s>>>(p);
-    count_launches(1);
-    return cudaGetLastError();
+    const dim3 grid((unsigned)((p.nket + t.kets - 1) / t.kets), (unsigned)((p.nbra + t.bras - 1) / t.bras));
+    const cudaError_t e = launch_beside(q, f, grid, dim3(32, t.bras), 0, p);
+    if (e == cudaSuccess) count_launches(q.sizing ? 0 : 1);
+    return e;
   }
   if (!coop_ready()) return cudaErrorInvalidValue;
   const GenClass K = gen_class(pcb, pck);
   const CoopShape c = coop_shape(K, (long long)p.nbra * p.nket);
-  const cudaError_t e = coop_launch(g12_coop_kernel, c, s, p, K);
+  const cudaError_t e = coop_launch(g12_coop_kernel, c, q, p, K);
   if (e != cudaSuccess) return e;
-  count_launches(1);
-  return cudaGetLastError();
+  count_launches(q.sizing ? 0 : 1);
+  return cudaSuccess;
 }
 
 cudaError_t launch_schwarz(int pc, const SchwarzParams &p, cudaStream_t s) {
@@ -659,7 +670,8 @@ cudaError_t launch_schwarz(int pc, const SchwarzParams &p, cudaStream_t s) {
     if (!coop_ready()) return cudaErrorInvalidValue;
     const GenClass K{pc_la(pc), pc_lb(pc), pc_la(pc), pc_lb(pc)};
     const CoopShape c = coop_shape(K, p.np);
-    const cudaError_t e = coop_launch(schwarz_coop_kernel, c, s, p, K);
+    Queue q{s};
+    const cudaError_t e = coop_launch(schwarz_coop_kernel, c, q, p, K);
     if (e != cudaSuccess) return e;
   }
   count_launches(1);

@@ -30,6 +30,7 @@ constexpr int kPotMaxL = 2;           // shells of potential_kernel
 // the other, to the bit.
 template <int LA, int LB>
 __global__ void __launch_bounds__(128) potential_kernel(OneBodyParams P, int lanes) {
+  if (beside_block()) return;
   constexpr int L = LA + LB, NE = coff(L + 1), E0 = coff(LA), nE = NE - E0, NA = ncart(LA), NB = ncart(LB);
   __shared__ double term[128][nE + 1];   // per lane: W of its charge, then Z w
   __shared__ double sum[128][nE];        // per group (at its first lane): contracted X
@@ -144,6 +145,7 @@ __device__ void ovl1d_dev(int li, int lj, double PA, double PB, double o2p, doub
 // S and T of every pair, and (WITHV) V of the pairs with an f shell
 template <bool WITHV>
 __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
+  if (beside_block()) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int npair = P.nsh * (P.nsh + 1) / 2;
   if (t >= npair) return;
@@ -265,18 +267,15 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
 
 }  // namespace
 
-cudaError_t launch_one_body(const OneBodyParams &p, cudaStream_t s) {
+cudaError_t launch_one_body(const OneBodyParams &p, Queue &q) {
   const int npair = p.nsh * (p.nsh + 1) / 2;
-  if (npair <= 0) return cudaSuccess;
   const bool heavy = p.V && p.ncharge > 0 && p.lstart[kPotMaxL + 1] < p.nsh;
-  if (heavy) one_body_kernel<true><<<(npair + 127) / 128, 128, 0, s>>>(p);
-  else if (p.S || p.T) one_body_kernel<false><<<(npair + 127) / 128, 128, 0, s>>>(p);
-  else return cudaSuccess;
-  count_launches(1);
-  return cudaGetLastError();
+  if (npair <= 0 || (!heavy && !p.S && !p.T)) return cudaSuccess;
+  count_launches(q.sizing ? 0 : 1);
+  return launch_beside(q, heavy ? &one_body_kernel<true> : &one_body_kernel<false>, (npair + 127) / 128, 128, 0, p);
 }
 
-cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, cudaStream_t s) {
+cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, Queue &q) {
   using Fn = void (*)(OneBodyParams, int);
   static const Fn fn[3][3] = {{&potential_kernel<0, 0>, &potential_kernel<0, 1>, &potential_kernel<0, 2>},
                               {&potential_kernel<1, 0>, &potential_kernel<1, 1>, &potential_kernel<1, 2>},
@@ -287,9 +286,8 @@ cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, cudaStream_
   // lanes per pair: up to four warps per scheduler, no more than there are charges
   int lanes = 1;
   while (lanes < 32 && 2 * lanes <= p.ncharge && npair / 32 * lanes < 2 * (long long)kFillWarps) lanes *= 2;
-  fn[la][lb]<<<(unsigned)((npair * lanes + 127) / 128), 128, 0, s>>>(p, lanes);
-  count_launches(1);
-  return cudaGetLastError();
+  count_launches(q.sizing ? 0 : 1);
+  return launch_beside(q, fn[la][lb], (unsigned)((npair * lanes + 127) / 128), 128, 0, p, lanes);
 }
 
 long long potential_pairs(int la, int lb, const OneBodyParams &p) {

@@ -110,6 +110,43 @@ inline TileShape coop_tile(const LaunchLoad &w) {
   return {kets, 1, w.linear ? share_slices(w.quartets / kets, w.most / 2) : 1};
 }
 
+// Where a launch goes: stream s and, in a group of launches that need no order
+// among themselves, whether the one before it on s is of the group too.
+struct Queue {
+  cudaStream_t s;
+  bool group = false, beside = false;
+  // Global scratch of the launches (doubles).  An allocation between two
+  // launches would set them apart, so a group is gone through twice: with
+  // `sizing` on, launches only add up what they need; then they take it.
+  bool sizing = false;
+  size_t need = 0;
+  double *scratch = nullptr;
+};
+// Launches kernel f (its first statement: beside_block) on q.s.  In a group it
+// need not wait for the launch before it: a programmatic dependency of the same
+// stream, so nothing else of the process waits for it either.  With one side
+// stream per launch, joined by events, the waiting side streams held the
+// hardware queues that they share with other callers' streams: a build that
+// was queued behind 0.8 s of other work held up 10 of 30 independent builds.
+template <typename... P, typename... A>
+inline cudaError_t launch_beside(Queue &q, void (*f)(P...), dim3 grid, dim3 block, size_t smem, A... a) {
+  if (q.sizing) return cudaSuccess;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid.x + 1, grid.y, grid.z);   // beside_block
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = q.s;
+  c.attrs = &at;
+  c.numAttrs = q.beside ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&c, f, (P)a...);
+  if (e != cudaSuccess) cudaGetLastError();   // reported here
+  q.beside = q.group && e == cudaSuccess;
+  return e;
+}
+
 struct BoysTables {
   const double *f64;
   const float *dd;        // double-float rows (boys_dd)
@@ -332,7 +369,7 @@ struct G12Params {
   int kets;               // ket pairs per warp (set by the launcher)
 };
 using G12Fn = void (*)(G12Params);
-cudaError_t launch_g12(int pcb, int pck, G12Params p, cudaStream_t s);
+cudaError_t launch_g12(int pcb, int pck, G12Params p, Queue &q);
 
 struct SchwarzParams {
   const PairRec *pairs;
@@ -383,17 +420,20 @@ using MXFn = void (*)(MXParams);
 // launchers (every class with l <= kMaxL)
 enum class Arith { f64, f32, dd };
 cudaError_t launch_jk_tasks(int pcb, int pck, Arith arith, const JKTask *dtasks, const TaskLaunch &tl,
-                            cudaStream_t s);
+                            Queue &q);
+// whether the class has FP32 kernels (without one its FP32 half is evaluated in FP64)
+bool jk_fp32_class(int pcb, int pck);
+bool cp_fp32_class(int pcb, int pck);
 // whether the class has a double-float J/K kernel
 bool jk_dd_class(int pcb, int pck);
 // whether the FP32 launch of class (pcb, pck) over species of up to n
 // functions / nsh shells runs on the bra-row kernel
 bool jk_rows_used(int pcb, int pck, int n, int nsh);
 cudaError_t launch_cp_tasks(int pcb, int pck, bool fp32, const CPTask *dtasks, const TaskLaunch &tl,
-                            cudaStream_t s);
-cudaError_t launch_it(int pcb, int pck, ITParams p, cudaStream_t s);
+                            Queue &q);
+cudaError_t launch_it(int pcb, int pck, ITParams p, Queue &q);
 cudaError_t launch_schwarz(int pc, const SchwarzParams &p, cudaStream_t s);
-cudaError_t launch_mp2x(int pcb, int pck, MXParams p, cudaStream_t s);
+cudaError_t launch_mp2x(int pcb, int pck, MXParams p, Queue &q);
 // MP2 transform helpers (k_mp2.cu).  Coefficients: C[p][mu] rows are
 // orbitals; Co[mu][i] = norma[mu] C[n_frozen + i][mu] (n x o), Cv[mu][a] =
 // norma[mu] C[n_occ + a][mu] (n x v); the *32 outputs may be null.
@@ -596,10 +636,10 @@ struct OneBodyParams {
   BoysTables boys;
 };
 // S and T, and V of the pairs with an f shell
-cudaError_t launch_one_body(const OneBodyParams &p, cudaStream_t s);
+cudaError_t launch_one_body(const OneBodyParams &p, Queue &q);
 // V of the pairs with a later shell of angular momentum la and an earlier one of
 // lb (s, p and d), and the candidates of such a launch (0 for other classes)
-cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, cudaStream_t s);
+cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, Queue &q);
 long long potential_pairs(int la, int lb, const OneBodyParams &p);
 
 // x[i] = deterministic pseudo-random values in [-1, 1) (benchmark operands)

@@ -26,108 +26,28 @@ void set_error(const char *fmt, ...) {
   if (strict && strict[0] == '1') abort();
 }
 
-// ------------------------------------------------------------------ lanes --
-// Seven side streams and the caller's own: a build has 6 (s, p) to 21 (s, p,
-// d) class launches, and each further lane costs the host a wait, a record and
-// another wait.  Measured, one stream -> lanes: one water (34 functions, 6
-// launches of 6-170 CTAs) 192 -> 116 us; four waters with d (21 launches, the
-// eight cooperative ones of 16-264 CTAs) 3.88 -> 1.43 ms; electron-proton
-// coupling of six waters 504 -> 380 us; a 387-function chain, whose launches
-// fill the GPU by themselves, 41.7 -> 41.6 ms.
-constexpr int kSideLanes = 7;
-constexpr size_t kLanePool = 16;   // sets kept per process; a set above it is destroyed when given back
-
-struct LaneSet {
-  int device = -1;
-  cudaStream_t s[kSideLanes] = {};
-  cudaEvent_t fork = nullptr, done[kSideLanes] = {};
-  bool create() {
-    CK(cudaGetDevice(&device));
-    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-    for (int k = 0; k < kSideLanes; ++k) {
-      CK(cudaStreamCreateWithFlags(&s[k], cudaStreamNonBlocking));
-      CK(cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming));
-    }
-    return true;
-  }
-  ~LaneSet() {
-    for (int k = 0; k < kSideLanes; ++k) {
-      if (s[k]) cudaStreamDestroy(s[k]);
-      if (done[k]) cudaEventDestroy(done[k]);
-    }
-    if (fork) cudaEventDestroy(fork);
-  }
-};
-
-namespace {
-std::mutex g_lane_mu;
-std::vector<LaneSet *> g_lane_free;
-}  // namespace
-
-Lanes::Lanes(cudaStream_t s, bool captured) {
-  if (!captured) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-      cudaGetLastError();   // the legacy stream beside another stream's capture: stay on s
-      return;
-    }
-    if (st != cudaStreamCaptureStatusNone) return;
-  }
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
-  {
-    std::lock_guard<std::mutex> lk(g_lane_mu);
-    for (size_t k = g_lane_free.size(); k-- > 0;)
-      if (g_lane_free[k]->device == dev) {
-        set_ = g_lane_free[k];
-        g_lane_free.erase(g_lane_free.begin() + k);
-        return;
-      }
-  }
-  LaneSet *n = new LaneSet();
-  if (n->create()) set_ = n;
-  else delete n;
-}
-
-Lanes::~Lanes() {
-  if (!set_) return;
-  {
-    std::lock_guard<std::mutex> lk(g_lane_mu);
-    if (g_lane_free.size() < kLanePool) {
-      g_lane_free.push_back(set_);
-      return;
-    }
-  }
-  delete set_;
-}
-
-bool Lanes::run(std::vector<Job> &jobs, cudaStream_t s) {
-  std::stable_sort(jobs.begin(), jobs.end(), [](const Job &a, const Job &b) {
-    return a.in_order != b.in_order ? a.in_order : !a.in_order && a.cost > b.cost;
+bool run_jobs(std::vector<LaunchJob> &jobs, cudaStream_t s) {
+  std::stable_sort(jobs.begin(), jobs.end(), [](const LaunchJob &a, const LaunchJob &b) {
+    return a.in_order != b.in_order ? b.in_order : !a.in_order && a.cost > b.cost;
   });
-  const int lanes = set_ ? (int)std::min<size_t>(jobs.size(), kSideLanes + 1) : 1;
-  const int first = lanes > 1 && !jobs.empty() && jobs[0].in_order ? 1 : 0;   // lane 0 is s itself
-  if (lanes > 1) CK(cudaEventRecord(set_->fork, s));
-  double load[kSideLanes + 1] = {};
-  bool used[kSideLanes + 1] = {};
+  Queue q{s, true};
+  q.sizing = true;
+  for (const LaunchJob &j : jobs) CK(j.launch(q));
+  q.sizing = false;
+  if (q.need) CK(cudaMallocAsync((void **)&q.scratch, q.need * sizeof(double), s));
+  q.need = 0;
   cudaError_t err = cudaSuccess;
-  for (Job &j : jobs) {
-    const int k = j.in_order ? 0 : (int)(std::min_element(load + first, load + lanes) - load);
-    cudaStream_t q = k ? set_->s[k - 1] : s;
-    if (k && !used[k]) err = cudaStreamWaitEvent(q, set_->fork, 0);
-    used[k] = true;
-    load[k] += j.cost;
-    if (err == cudaSuccess) err = j.launch(q);
+  bool ordered = false;
+  for (const LaunchJob &j : jobs) {
+    if (ordered) q.beside = false;
+    err = j.launch(q);
     if (err != cudaSuccess) break;
+    ordered = j.in_order;
   }
-  // the lanes are joined also after a failed launch: s then still ends behind
-  // whatever was queued
-  for (int k = 1; k < lanes; ++k)
-    if (used[k]) {
-      cudaError_t e = cudaEventRecord(set_->done[k - 1], set_->s[k - 1]);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(s, set_->done[k - 1], 0);
-      if (err == cudaSuccess) err = e;
-    }
+  if (q.scratch) {
+    const cudaError_t e = cudaFreeAsync(q.scratch, s);
+    if (err == cudaSuccess) err = e;
+  }
   CK(err);
   return true;
 }
@@ -470,8 +390,8 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
 
 // mode 0: FP64, 1: FP32 throughout, 2: split at `split` (FP64 above, FP32 below)
 bool launch_cp_groups(const TaskSet<CPTask> &ts, int mode, double split, BoysTables boys, cudaStream_t s,
-                      double skip, Lanes *lanes) {
-  std::vector<Lanes::Job> jobs;
+                      double skip) {
+  std::vector<LaunchJob> jobs;
   for (int c = 0; c < kNQC; ++c) {
     if (!ts.cnt[c]) continue;
     TaskLaunch tl{};
@@ -487,17 +407,17 @@ bool launch_cp_groups(const TaskSet<CPTask> &ts, int mode, double split, BoysTab
     const int cb = c / kNumPairClasses, ck = c % kNumPairClasses;
     const CPTask *d = ts.d + ts.off[c];
     auto add = [&](bool fp32) {
-      if (!lanes) return launch_cp_tasks(cb, ck, fp32, d, tl, s);
-      jobs.push_back({launch_cost(cb, ck, tl.nblocks), fp32,
-                      [=](cudaStream_t q) { return launch_cp_tasks(cb, ck, fp32, d, tl, q); }});
-      return cudaSuccess;
+      // fewest blocks first: a launch lets the next one begin with its last block
+      // (six waters 251 us costliest first, 235 so; twelve 0.90 and 0.92 ms)
+      jobs.push_back({-(double)tl.nblocks, fp32 && cp_fp32_class(cb, ck),
+                      [=](Queue &q) { return launch_cp_tasks(cb, ck, fp32, d, tl, q); }});
     };
     tl.lower = 0;
-    CK(add(mode == 1));
+    add(mode == 1);
     tl.lower = 1;
-    if (mode == 2) CK(add(true));
+    if (mode == 2) add(true);
   }
-  return !lanes || lanes->run(jobs, s);
+  return run_jobs(jobs, s);
 }
 
 bool coupling(LibintInterface *A, LibintInterface *B, const double *dDa, const double *dDb, double *dJa,
@@ -525,10 +445,7 @@ bool coupling(LibintInterface *A, LibintInterface *B, const double *dDa, const d
   SpeciesBufs bb{B->dDsC.p, B->dDsC32.p, nullptr, nullptr, B->dJacc.p, B->dJacc32.p};
   if (!add_cp_tasks(A->cp, A, B, ba, bb, dJa != nullptr, dJb != nullptr, 1.0)) return false;
   if (!A->cp.upload(s)) return false;
-  {
-    Lanes lanes(s);
-    if (!launch_cp_groups(A->cp, fp32 ? 1 : 0, 0.0, A->boys, s, 0.0, &lanes)) return false;
-  }
+  if (!launch_cp_groups(A->cp, fp32 ? 1 : 0, 0.0, A->boys, s)) return false;
   if (dJa) CK(launch_coupling_extract(A->dJacc.p, A->dJacc32.p, A->d_norma, nA, 1.0, 0, dJa, s));
   if (dJb) CK(launch_coupling_extract(B->dJacc.p, B->dJacc32.p, B->d_norma, nB, 1.0, 0, dJb, s));
   return true;
@@ -562,10 +479,10 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
   q.cut = 1e-10;
   q.eps = DBL_EPSILON;
   q.nsh = nsh;
-  std::vector<Lanes::Job> jobs;
+  std::vector<LaunchJob> jobs;
   auto add = [&](int cb, int ck) {
     const ITParams p = q;
-    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), false, [=](cudaStream_t z) { return launch_it(cb, ck, p, z); }});
+    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), false, [=](Queue &z) { return launch_it(cb, ck, p, z); }});
   };
   if (intra) {
     if (!A->dD.ensure((size_t)nA * nA) || !A->dDs.ensure((size_t)nA * nA) || !A->dDn.ensure((size_t)nsh * nsh))
@@ -614,10 +531,7 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
         add(cb, ck);
       }
   }
-  {
-    Lanes lanes(s);
-    if (!lanes.run(jobs, s)) return false;
-  }
+  if (!run_jobs(jobs, s)) return false;
   CK(launch_scale_cube(A->dA.p, A->d_norma, K->d_norma, nA, nB, s));
   CK(cudaMemcpyAsync(hOut, A->dA.p, cube * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
@@ -660,10 +574,10 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
   G12Params P{};
   P.gem = A->dGem.p;
   P.n = n;
-  std::vector<Lanes::Job> jobs;
+  std::vector<LaunchJob> jobs;
   auto add = [&](int cb, int ck) {
     const G12Params p = P;
-    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket), false, [=](cudaStream_t z) { return launch_g12(cb, ck, p, z); }});
+    jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket), false, [=](Queue &z) { return launch_g12(cb, ck, p, z); }});
   };
   if (!B) {
     CK(launch_scale_density(dD, A->d_norma, n, A->dDs.p, A->dDs32.p, s));
@@ -685,10 +599,7 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
         P.mean_prims = A->sig.prims(cb) * A->sig.prims(ck);
         add(cb, ck);
       }
-    {
-      Lanes lanes(s);
-      if (!lanes.run(jobs, s)) return false;
-    }
+    if (!run_jobs(jobs, s)) return false;
     CK(launch_symmetrize(A->dGacc.p, nullptr, A->d_norma, n, 0.25, dOut, s));
     return true;
   }
@@ -714,10 +625,7 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
       P.mean_prims = A->all.prims(cb) * B->all.prims(ck);
       add(cb, ck);
     }
-  {
-    Lanes lanes(s);
-    if (!lanes.run(jobs, s)) return false;
-  }
+  if (!run_jobs(jobs, s)) return false;
   CK(launch_coupling_extract(A->dJacc.p, nullptr, A->d_norma, n, 1.0, 1, dOut, s));
   return true;
 }
@@ -1050,15 +958,15 @@ int LowdinGB300_one_body_device(LibintInterface *lint, int ncharge, const double
   } else if (dV) {
     if (cudaMemsetAsync(dV, 0, sizeof(double) * lint->nbasis * lint->nbasis, s) != cudaSuccess) return -1;
   }
-  std::vector<Lanes::Job> jobs;
-  jobs.push_back({(double)p.nsh * p.nsh, false, [=](cudaStream_t q) { return launch_one_body(p, q); }});
+  std::vector<LaunchJob> jobs;
+  // one thread per pair, so the longest: first, that the others run beside it
+  jobs.push_back({HUGE_VAL, false, [=](Queue &q) { return launch_one_body(p, q); }});
   for (int la = 0; p.V && p.ncharge > 0 && la <= kMaxL; ++la)
     for (int lb = 0; lb <= kMaxL; ++lb)
       if (potential_pairs(la, lb, p) > 0)
         jobs.push_back({(double)potential_pairs(la, lb, p) * p.ncharge * ncart(la) * ncart(lb), false,
-                        [=](cudaStream_t q) { return launch_potential(la, lb, p, q); }});
-  Lanes lanes(s);
-  return lanes.run(jobs, s) ? 0 : -1;
+                        [=](Queue &q) { return launch_potential(la, lb, p, q); }});
+  return run_jobs(jobs, s) ? 0 : -1;
 }
 
 int LowdinGB300_set_precision(LibintInterface *lint, int precision, double split) {
@@ -1250,7 +1158,7 @@ int LowdinGB300_twobody_device_noalloc(LibintInterface *lint, const double *dD, 
     set_error("%s: preparation failed", __func__);
     return -1;
   }
-  if (!LibintInterface::launch_jk_groups(ts, precision, split, lint->boys, s)) return -1;
+  if (!LibintInterface::launch_jk_groups(ts, precision, split, lint->boys, s, false)) return -1;
   if (launch_symmetrize(Gacc, Gacc32, lint->d_norma, n, 0.25, dG, s) != cudaSuccess) {
     set_error("%s: symmetrisation failed", __func__);
     return -1;

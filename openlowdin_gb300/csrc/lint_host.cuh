@@ -228,38 +228,23 @@ inline double launch_cost(int cb, int ck, double blocks) {
   const int L = pc_L(cb) + pc_L(ck);
   return (blocks + 300.0) * ncart(pc_la(cb)) * ncart(pc_lb(cb)) * ncart(pc_la(ck)) * ncart(pc_lb(ck)) * (L + 1);
 }
-// Streams for the quartet-class launches of one build.  The classes of a build
-// only add into the same accumulators, so they need no order among
-// themselves; on one stream each of them waits for the last block of the one
-// before.  A lease takes a set of side streams from a bounded per-device pool
-// and gives it back when it goes out of scope; a set is only ever used by one
-// lease at a time, and work left on its streams merely orders the next user's
-// launches behind it.
-struct LaneSet;
-class Lanes {
- public:
-  // side streams for launches forked from `s`.  None when s is being captured
-  // (a set given back before the capture ends would carry another caller's
-  // launches into the graph), unless `captured`: the caller holds the lease
-  // until its own capture has ended.
-  explicit Lanes(cudaStream_t s, bool captured = false);
-  ~Lanes();
-  Lanes(const Lanes &) = delete;
-  Lanes &operator=(const Lanes &) = delete;
-  // runs the queued launches: costliest first, each on the lane with the
-  // least work so far, every lane ordered behind `s` and s behind every lane.
-  // Launches that accumulate in FP32, whose sums depend on the order of the
-  // classes in the sixth digit, keep their order, on s
-  struct Job {
-    double cost;
-    bool in_order;
-    std::function<cudaError_t(cudaStream_t)> launch;
-  };
-  bool run(std::vector<Job> &jobs, cudaStream_t s);
-
- private:
-  LaneSet *set_ = nullptr;
+// Quartet-class launches of one build.  The classes of a build only add into
+// the same accumulators, so they need no order among themselves; one after
+// another, each would wait for the last block of the one before.
+struct LaunchJob {
+  double cost;
+  // a launch that accumulates in FP32, whose sums depend on the order of the
+  // classes in the sixth digit
+  bool in_order;
+  std::function<cudaError_t(Queue &)> launch;
 };
+// Runs the jobs on s beside one another (launch_beside), costliest first, then
+// those in order one after another; what is queued on s afterwards is behind
+// them all.  Eight are in flight at most.  One after another -> so: one water (34
+// functions, 6 launches of 6-170 blocks) 184 -> 114 us; two waters in a contracted
+// basis (21 launches) 1.78 -> 0.59 ms; four waters with d 1.71 -> 0.95 ms; a
+// 387-function chain, whose launches fill the GPU by themselves, 18.1 -> 18.0 ms.
+bool run_jobs(std::vector<LaunchJob> &jobs, cudaStream_t s);
 
 // device buffers of one species in one build: scaled density (FP64 + FP32),
 // shell-block norms (FP64 + FP32) and the output accumulators (FP64 + FP32)
@@ -690,10 +675,7 @@ struct LibintInterface {
     CK(launch_prepare_density(dDin, d_norma, d_shell_of, n, nsh, dDs.p, dDs32.p, dDd.p, dDn.p, dDn32.p, s, true));
     CK(launch_dn_max(dDn32.p, nsh, dDnmax32.p, s));
     if (precision != 0) CK(launch_pair_gather(dpslot.p, 1, (long long)sig.h.size(), s));
-    {
-      Lanes lanes(s);
-      if (!launch_jk_groups(jk, precision, split, boys, s, 0.0, nullptr, -1, false, &lanes)) return false;
-    }
+    if (!launch_jk_groups(jk, precision, split, boys, s, true)) return false;
     if (precision != 0) CK(launch_pair_scatter(dpslot.p, 1, (long long)sig.h.size(), s));
     CK(launch_symmetrize(dGacc.p, dGacc32.p, d_norma, n, 0.25, dGout, s));
     // the quartet counts travel with the result; they are summed when asked for
@@ -785,11 +767,13 @@ struct LibintInterface {
   // rows: per quartet class the FP32 kernel of mixed launches (-1 size rule,
   // 0 jk_tasks_kernel, 1 bra-row kernel; null: size rule); only: a single
   // class (-1: all) and, with lower_only, only its FP32 launch (autotuning);
-  // lanes: side streams for the launches (null: all on s, in class order)
+  // beside: the launches run beside one another (else one after another, in
+  // class order)
   static bool launch_jk_groups(const TaskSet<JKTask> &ts, int precision, double split, BoysTables boys,
-                               cudaStream_t s, double skip = 0.0, const signed char *rows = nullptr,
-                               int only = -1, bool lower_only = false, Lanes *lanes = nullptr) {
-    std::vector<Lanes::Job> jobs;
+                               cudaStream_t s, bool beside, double skip = 0.0,
+                               const signed char *rows = nullptr, int only = -1, bool lower_only = false) {
+    std::vector<LaunchJob> jobs;
+    Queue serial{s};
     for (int c = 0; c < kNQC; ++c) {
       if (!ts.cnt[c] || (only >= 0 && c != only)) continue;
       TaskLaunch tl{};
@@ -809,9 +793,9 @@ struct LibintInterface {
       tl.split = precision == 0 ? 0.0 : split;
       set_fp32_copies(tl);
       auto add = [&](Arith arith) {
-        if (!lanes) return launch_jk_tasks(cb, ck, arith, d, tl, s);
-        jobs.push_back({launch_cost(cb, ck, tl.nblocks), arith == Arith::f32,
-                        [=](cudaStream_t q) { return launch_jk_tasks(cb, ck, arith, d, tl, q); }});
+        if (!beside) return launch_jk_tasks(cb, ck, arith, d, tl, serial);
+        jobs.push_back({launch_cost(cb, ck, tl.nblocks), arith == Arith::f32 && jk_fp32_class(cb, ck),
+                        [=](Queue &q) { return launch_jk_tasks(cb, ck, arith, d, tl, q); }});
         return cudaSuccess;
       };
       tl.lower = 0;
@@ -826,7 +810,7 @@ struct LibintInterface {
       tl.lower = 1;
       if (precision != 0) CK(add(Arith::f32));
     }
-    return !lanes || lanes->run(jobs, s);
+    return !beside || run_jobs(jobs, s);
   }
 };
 
@@ -838,7 +822,7 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
                   unsigned long long *counters = nullptr);
 // mode 0: FP64, 1: FP32 throughout, 2: split at `split` (FP64 above, FP32 below)
 bool launch_cp_groups(const TaskSet<CPTask> &ts, int mode, double split, BoysTables boys, cudaStream_t s,
-                      double skip = 0.0, Lanes *lanes = nullptr);
+                      double skip = 0.0);
 bool coupling(LibintInterface *A, LibintInterface *B, const double *dDa, const double *dDb, double *dJa,
               double *dJb, bool fp32, cudaStream_t s);
 bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, const double *hC, int p,

@@ -62,7 +62,7 @@ void mp2_columns(const PairList &P, long long colB, MP2Columns &mc) {
 
 // integrals of every (mu nu) pair of PA with the column pairs [k0, k1) of PB
 bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, int k1, cudaStream_t s) {
-  std::vector<Lanes::Job> jobs;
+  std::vector<LaunchJob> jobs;
   double pa[kNumPairClasses];
   for (int c = 0; c < kNumPairClasses; ++c) pa[c] = PA.prims(c);
   for (int ck = 0; ck < kNumPairClasses; ++ck) {
@@ -77,11 +77,10 @@ bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, 
         p.nket = PA.count(cb);
         p.mean_prims = pa[cb] * PB.prims(ck);
         jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), false,
-                        [=](cudaStream_t z) { return launch_mp2x(ck, cb, p, z); }});
+                        [=](Queue &z) { return launch_mp2x(ck, cb, p, z); }});
       }
   }
-  Lanes lanes(s);
-  return lanes.run(jobs, s);
+  return run_jobs(jobs, s);
 }
 
 // Writer of the reference's transformed-integral file `<species>moint.dat`
