@@ -159,27 +159,29 @@ __global__ void prepare_batch_kernel(const SpeciesSlot *__restrict__ slots, int 
 }
 
 // largest of Dn32 by the norms' bit patterns (non-negative floats order as
-// integers; a NaN orders above all and so keeps every tile): block x takes
-// every gridDim.x-th run of 256 norms, its maximum goes to *out.  One block
+// integers; a NaN orders above all and so keeps every tile): block b of `blocks`
+// takes every blocks-th run of 256 norms, its maximum goes to *out.  One block
 // walking whole columns took 34 us for 512 shells, a chain of 512 loads.
-__device__ __forceinline__ void dn_max_block(const float *__restrict__ Dn32, int nsh, float *__restrict__ out) {
-  const size_t nn = (size_t)nsh * nsh, step = (size_t)gridDim.x * blockDim.x;
+__device__ __forceinline__ void dn_max_block(const float *__restrict__ Dn32, int nsh, float *__restrict__ out, int b,
+                                             int blocks) {
+  const size_t nn = (size_t)nsh * nsh, step = (size_t)blocks * blockDim.x;
   int m = 0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nn; i += step)
+  for (size_t i = b * (size_t)blockDim.x + threadIdx.x; i < nn; i += step)
     m = max(m, __float_as_int(Dn32[i]));
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(reinterpret_cast<int *>(out), m);
 }
 
+// species on grid x, which holds any number of them (grid y ends at 65,535)
 __global__ void dn_max_batch_kernel(const SpeciesSlot *__restrict__ slots) {
-  const SpeciesSlot &S = slots[blockIdx.y];
-  if (!S.Dn32 || !S.Dnmax32 || (size_t)blockIdx.x * blockDim.x >= (size_t)S.nsh * S.nsh) return;
+  const SpeciesSlot &S = slots[blockIdx.x];
+  if (!S.Dn32 || !S.Dnmax32 || (size_t)blockIdx.y * blockDim.x >= (size_t)S.nsh * S.nsh) return;
   if (S.active && __ldg(S.active) == 0) return;
-  dn_max_block(S.Dn32, S.nsh, S.Dnmax32);
+  dn_max_block(S.Dn32, S.nsh, S.Dnmax32, blockIdx.y, gridDim.y);
 }
 
 __global__ void dn_max_kernel(const float *__restrict__ Dn32, int nsh, float *__restrict__ out) {
-  dn_max_block(Dn32, nsh, out);
+  dn_max_block(Dn32, nsh, out, blockIdx.x, gridDim.x);
 }
 
 // G = gscale N (Gacc + Gacc^T) N (0 when the species builds none), J = N Jacc N,
@@ -308,7 +310,7 @@ static int dn_max_grid(int nsh) {
 
 cudaError_t launch_dn_max_batch(const SpeciesSlot *slots, int nslots, int max_nsh, cudaStream_t s) {
   if (nslots <= 0 || max_nsh <= 0) return cudaSuccess;
-  dn_max_batch_kernel<<<dim3((unsigned)dn_max_grid(max_nsh), (unsigned)nslots), 256, 0, s>>>(slots);
+  dn_max_batch_kernel<<<dim3((unsigned)nslots, (unsigned)dn_max_grid(max_nsh)), 256, 0, s>>>(slots);
   count_launches(1);
   return cudaGetLastError();
 }
