@@ -105,11 +105,11 @@ __device__ __forceinline__ float schwarz32(const PairRec32 &p) { return p.Q; }
 __device__ __forceinline__ float schwarz32(const PairRecD &p) { return p.Q.hi; }
 
 // Bound of the double-float quartets of a species: `tier` (kTierBound times
-// its largest product of Schwarz factors) times the largest density element.
-// Zero, so that everything stays in FP64, for densities whose products could
-// leave the FP32 exponent range, infinities and NaN.
-__device__ __forceinline__ float tier_bound(float tier, float d) {
-  return d > 1e-12f && d < 1e20f ? tier * d : 0.f;
+// its largest product of Schwarz factors) times the largest density element,
+// and `cap` at most.  Zero, so that everything stays in FP64, for densities
+// whose products could leave the FP32 exponent range, infinities and NaN.
+__device__ __forceinline__ float tier_bound(float tier, float d, float cap) {
+  return d > 1e-12f && d < 1e20f ? fminf(tier * d, cap) : 0.f;
 }
 
 // ----------------------------------------------------------------- Schwarz --
@@ -293,8 +293,9 @@ __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) jk_ta
   // largest norm of all), w >= tb in the FP64 launch, w < tb in the
   // double-float one
   const float dmax = T.Dnmax32 ? __ldg(T.Dnmax32) : -1.f;
-  const float tb =
-      TL.tier == Tier::all ? 0.f : tier_bound(TL.mixed && !all64 ? kMixedTier * T.tier : T.tier, dmax);
+  const float tb = TL.tier == Tier::all ? 0.f
+                   : TL.mixed && !all64 ? tier_bound(kMixedTier * T.tier, dmax, TL.tier_cap)
+                                        : tier_bound(T.tier, dmax, kTierCap);
   if (TL.tier == Tier::lower && (tb == 0.f || (T.screen && !(lo < tb)))) return;
   // Pairs are sorted by decreasing Schwarz factor inside a class and Dnmax32
   // bounds the six norms, so the first bra and the first ket of a range bound

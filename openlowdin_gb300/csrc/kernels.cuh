@@ -209,6 +209,7 @@ struct JKTask {
   const float *Dnmax32;
   // double-float form (null: FP64 alone): pair and primitive records, density,
   // and tier: bound below which a quartet is evaluated in it, per unit of *Dnmax32
+  // (0: FP64 alone)
   const PairRecD *pairsd;
   const PrimRecD *primsd;
   const float2 *Dd;
@@ -248,24 +249,33 @@ struct CPTask {
   float mean_prims, most_prims;   // mean and largest number of primitive quartets
 };
 
-// FP64 builds evaluate a quartet whose density-weighted bound is small against
-// the build's largest one in double-float arithmetic (dd32.cuh), on the FP32
-// pipe, and add its integrals into the same FP64 sums.  Its relative error,
-// some 2^-45, times a bound below kTierBound of the largest stays below the
-// FP64 rounding of the sums that the largest quartets go into.  Error of the
-// two-particle matrix against an 80-bit evaluation (2-norm over 2-norm), FP64
-// alone -> two tiers: 4 waters (136 functions) 3.0e-15 -> 3.0e-15, 176-function
-// chain 6.0e-15 -> 4.8e-15, 3 waters with d 3.9e-15 -> 3.5e-15, 12 protons
-// 1.6e-14 -> 1.6e-14 (the sums of eight ket tiles at a time that came with it
-// round less often).  387-function chain (5 % of the quartets above the bound):
-// 41.7 -> 17.9 ms.
+// FP64 builds of screened species (electrons) evaluate a quartet whose
+// density-weighted bound is small in double-float arithmetic (dd32.cuh), on the
+// FP32 pipe, and add its integrals into the same FP64 sums.  Its error, measured
+// against the FP64 integrals, is 2^-42.8 of that bound in the middle and 2^-41.3
+// at worst (the recursion amplifies FP64's own rounding by as much).  Small
+// means: below kTierBound of the build's largest bound, so that the error stays
+// 2^5 below the FP64 rounding of the largest quartets, and below kTierCap, so
+// that it stays near the screening threshold of 2^-52 whatever the largest bound
+// is: the quartets that screening drops leave 2e-11 in the matrix, and the
+// error against the unscreened 64-bit matrix is the same with and without the
+// tier in each power of ten of the elements' size (chains of 150 and 387
+// functions, 8 waters, 4 waters with d).  Species without screening keep FP64:
+// each of their elements has the relative precision of its own quartets.
+// Error of the matrix against an 80-bit evaluation of the same quartets (2-norm
+// over 2-norm), FP64 alone -> two tiers: 4 waters (136 functions) 3.0e-15 ->
+// 3.0e-15, 176-function chain 6.0e-15 -> 4.8e-15, 3 waters with d 3.9e-15 ->
+// 3.5e-15.  387-function chain (5 % of the quartets above the bound): 41.7 ->
+// 18.4 ms (18.1 without the cap, 21.6 with one of 2^-12).
 enum class Tier { all, upper, lower };
-constexpr float kTierBound = 1.f / 4096;
-// Mixed builds, whose quartets below the split are evaluated in FP32 anyway (1e-5
-// times 2^-22), take the double-float tier up to 1/16 of the largest bound; a
-// system held in FP64 for its check keeps kTierBound.  724-function chain, a
-// later iteration's density change: 40.1 -> 34.1 ms.
-constexpr float kMixedTier = 256.f;
+constexpr float kTierBound = 1.f / 4096, kTierCap = 1.f / 64;
+// Mixed builds, whose quartets below the split are evaluated in FP32 (error some
+// 2^-22 of a bound up to the split), take the tier up to 1/16 of the largest
+// bound, where its error stays below that of the FP32 quartets: up to 2^18
+// splits, and the tier of FP64 builds in any case.  A system held in FP64 for
+// its check keeps the tier of FP64 builds.  724-function chain, a later
+// iteration's density change, split 1e-5: 40.1 -> 34.3 ms.
+constexpr float kMixedTier = 256.f, kMixedCap = 0x1p18f;
 // candidate quartets of a class below which one FP64 launch is shorter than two
 // launches (one water, 120 to 14,000 a class: 116 us in one, 163 us in two; four
 // waters with d: 1.09 ms with the line at 2e5, 1.00 at 5e4, 1.02 at 2e4)
@@ -288,6 +298,7 @@ struct TaskLaunch {
   int mixed;
   Tier tier;              // J/K: the quartets this launch takes
   float eps32, split32, cut32;
+  float tier_cap;         // cap of the double-float tier of mixed builds
   BoysTables boys;
 };
 inline void set_fp32_copies(TaskLaunch &tl) {
@@ -295,6 +306,7 @@ inline void set_fp32_copies(TaskLaunch &tl) {
   tl.eps32 = (float)tl.eps;
   tl.split32 = (float)tl.split;
   tl.cut32 = (float)tl.cut;
+  tl.tier_cap = kMixedCap * tl.split32 > kTierCap ? kMixedCap * tl.split32 : kTierCap;
 }
 
 // Kernel entry types of the class-templated launch tables (class_tables.cuh);

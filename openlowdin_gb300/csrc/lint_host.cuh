@@ -306,13 +306,14 @@ struct TaskSet {
   void clear() {
     for (auto &g : group) g.clear();
   }
-  // whether group c runs in two tiers: every task has its double-float form
+  // whether group c runs in two tiers: its tasks with a tier have their
+  // double-float form and are worth a second launch
   bool tiers(int c) const {
     if constexpr (std::is_same<T, JKTask>::value) {
       double q = 0;
       for (const T &t : group[c]) {
-        if (!t.Dd || !t.Dnmax32) return false;
-        q += (double)t.nbra * t.nket;
+        if (t.tier > 0.f && (!t.Dd || !t.Dnmax32)) return false;
+        if (t.tier > 0.f) q += (double)t.nbra * t.nket;
       }
       return q >= kTierMinQuartets && jk_dd_class(c / kNumPairClasses, c % kNumPairClasses);
     }
@@ -704,8 +705,13 @@ struct LibintInterface {
   bool add_jk_tasks(TaskSet<JKTask> &ts, const SpeciesBufs &bf, double hf, unsigned long long *counters) {
     if (!ensure_sig()) return false;
     if (bf.Dd && !sig.upload_dd()) return false;
+    // the double-float tier: screened species whose scaled density (D times two
+    // norms) keeps clear of the ends of the FP32 exponent range
     double qmax = 0;   // largest Schwarz factor of the species
     for (const PairRec &r : sig.h) qmax = std::max(qmax, r.Q);
+    const bool in_range =
+        std::all_of(norma.begin(), norma.end(), [](double x) { return std::fabs(x) > 1e-8 && std::fabs(x) < 1e8; });
+    const float tier = is_electron && in_range ? (float)(qmax * qmax) * kTierBound : 0.f;
     double cprims[kNumPairClasses], cmost[kNumPairClasses];
     for (int c = 0; c < kNumPairClasses; ++c) {
       cprims[c] = sig.prims(c);
@@ -751,7 +757,7 @@ struct LibintInterface {
         t.Dd = bf.Dd;
         const dd32 h = split_double(hf);
         t.hfd = make_float2(h.hi, h.lo);
-        t.tier = (float)(qmax * qmax) * kTierBound;
+        t.tier = tier;
         if (bf.Dp32) {
           long long pe_base[kNumPairClasses];
           pair_elements(sig.start, pe_base);
