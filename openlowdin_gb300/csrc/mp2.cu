@@ -318,6 +318,8 @@ bool mp2_split(MP2Setup &S, int np, size_t budget, double *e2out, cudaStream_t s
       if (cp >> 31) ent[fill[lam]++] = make_int2(sig | lam << 16, (int)c);
     }
   }
+  // before the check of what is free
+  if (!S.PA->upload_dd() || !S.PB->upload_dd()) return false;
   const size_t need = (size_t)vA * oA * ncols * 4 + (size_t)colB * per_col +
                       ((size_t)vA * KB * KB + (size_t)oB * vA * KB + (size_t)(oA + vA) * KA + (size_t)(oB + vB) * KB) *
                           2 * np +
@@ -360,7 +362,6 @@ bool mp2_split(MP2Setup &S, int np, size_t budget, double *e2out, cudaStream_t s
   MXParams q = S.q;
   q.colbase = dcolbase.p;
   q.X = nullptr;
-  if (!S.PA->upload_dd() || !S.PB->upload_dd()) return false;
   q.pairsd = S.PB->dd;
   q.primsd = S.PB->ddp;
   q.kpairsd = S.PA->dd;
