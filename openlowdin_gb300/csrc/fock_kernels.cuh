@@ -940,8 +940,14 @@ __global__ void __launch_bounds__(128) it_kernel(ITParams P) {
 // ------------------------------------------------------ MP2 transform input --
 // Warp y: (lam sig) pair tile_y * bras + y of the batch; its lanes: (mu nu) pairs
 // tile_x * kets + (lane mod kets), 32 / kets lanes each.
-// R = dd32 writes the split-BF16 form only: the pieces hold at most the 24 bits of
-// an FP32 value, which double-float integrals (2^-45) round to as FP64 ones do.
+// R = dd32 writes the split-BF16 form only, whose pieces hold an integral to 2^-16 or
+// 2^-24 of itself.  A double-float integral is within 2^-41 Q_ab Q_cd of the FP64 one,
+// 2^-43 in the middle: at least 2^17 below the rounding of the quartet's largest
+// integral to 24 bits, and so below what that does to any (ia|jb).  An integral
+// that its terms cancel down to the cut may have fewer than 24 correct bits
+// there, and weighs as little: E_MP2 of twelve waters with d is the same to the
+// last digit with FP64 integrals (116.3 ms; double-float 114.4; four waters in a
+// contracted basis 7.4 and 5.0 ms).
 template <typename R, int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) mp2x_kernel(MXParams P) {
   if (beside_block()) return;
