@@ -163,17 +163,27 @@ void LowdinGB300_gaussian_potential(LibintInterface *lint, int ncomp, const doub
                                     const double *exponents, const double *origins, double *result);
 
 /* Precision of this handle's LibintInterface_compute_2body_direct (host
-   buffers, the reference's own call): 0 = FP64 (default, the reference's
-   behaviour); 1 = quartets whose Schwarz bound times the density's shell-block
-   maximum is below `split` run in FP32, the rest in FP64 (a caller that passes
+   buffers, the reference's own call): 0 = FP64 (default) and 1 = mixed at
+   `split`, both as LowdinGB300_twobody_device has them (a caller that passes
    density changes gets the incremental mixed-precision build of the
    batched SCF).  The coupling and first-quarter calls stay FP64.  Returns 0, or
    -1 for an unknown precision or a split outside (0, 1). */
 int LowdinGB300_set_precision(LibintInterface *lint, int precision, double split);
 
 /* Device-resident two-particle matrix: dG = J[dD] + factor K[dD] (n x n device
-   buffers, full symmetric).  precision: 0 = FP64, 1 = mixed (quartets whose
-   Schwarz-density bound is below `split` run in FP32, the rest in FP64).
+   buffers, full symmetric).  precision:
+     0 = FP64 sums of FP64 integrals, but for electrons: there a quartet whose
+         Schwarz-density bound B is below both 2^-12 of Q_max^2 max|D| and 2^-6
+         is evaluated in double-float on the FP32 pipe and added to the same
+         FP64 sums.  Such a quartet is within 2^-41 B of its FP64 value.  The
+         accuracy is that of FP64 in units of Q_max^2 max|D|, and per element
+         that of the density screening (quartets with B < 2^-52 are dropped, as
+         in the reference), not the 52 bits of an element fed by small quartets
+         alone.  LowdinGB300_twobody_device_noalloc uses FP64 alone, as do basis
+         sets with norms of the contractions beyond 1e-8 .. 1e8;
+     1 = mixed: quartets with B below `split` run in FP32, those above as in 0
+         with the ends at 2^-4 of Q_max^2 max|D| and at the larger of 2^-6 and
+         2^18 split (their error stays below that of the FP32 quartets).
    Work is queued on `stream` (a cudaStream_t, 0 = legacy default); returns 0
    on success, -1 on error (see LowdinGB300_last_error). */
 int LowdinGB300_twobody_device(LibintInterface *lint, const double *dD, double *dG, double factor, int precision,
@@ -228,15 +238,15 @@ int LowdinGB300_batch_finalize(LowdinGB300_Batch *b, void *stream);
    integral launches of a system whose flag is 0 return at once, leaving its
    G and J unwritten (a converged molecule of the batch costs no quartets);
    1 = built; 2 = built, and in mixed builds every quartet of the system is
-   evaluated in FP64 (a system whose mixed-precision solution failed its FP64
-   check continues in FP64 inside the same batch).  All systems are 1 after
+   evaluated as in precision 0 (a system whose mixed-precision solution failed
+   its FP64 check continues so inside the same batch).  All systems are 1 after
    finalize. */
 int LowdinGB300_batch_set_active(LowdinGB300_Batch *b, const int *flags, void *stream);
 /* precision bits: 1 = two-particle quartets whose Schwarz-density bound
-   Q_ab Q_cd max|D block| is below `split` run in FP32 (the rest FP64); 2 = the
-   same split for coupling quartets (bound Q_ab Q_cd max(|D_A|, |D_B|)).
-   0 = every quartet to FP64 accuracy (quartets below 2^-12 of the largest bound
-   in double-float on the FP32 pipe, added into FP64 sums). */
+   Q_ab Q_cd max|D block| is below `split` run in FP32 (the rest as in mixed
+   builds of LowdinGB300_twobody_device, per species); 2 = the same split for
+   coupling quartets (bound Q_ab Q_cd max(|D_A|, |D_B|)), the rest in FP64.
+   0 = precision 0 of LowdinGB300_twobody_device, couplings in FP64. */
 int LowdinGB300_batch_fock(LowdinGB300_Batch *b, int precision, double split, void *stream);
 /* Mixed builds (precision != 0) also drop the quartets whose density-weighted
    bound (the FP32 bound of the split) is below `skip`: with incremental
@@ -298,7 +308,8 @@ int LowdinGB300_twobody_device_noalloc(LibintInterface *lint, const double *dD, 
    contractions as split-BF16 tensor-core products, operands in 2 / 3 BF16
    pieces (LowdinGB300_gemm_bf16_split's engine; with 3 pieces the first
    quarter uses LowdinGB300_gemm_bf16_precise's), integrals in FP64 or
-   double-float (they end in at most 24 bits) and the energy sum in FP64.
+   double-float (within 2^-41 Q_ab Q_cd, far below the pieces' rounding of the
+   large ones) and the energy sum in FP64.
    x_budget_gb bounds the per-batch integral array (0: 8 GB).  Writes E_MP2 to
    *e2 (host) and synchronises `stream`.  Returns 0, or -1 with LowdinGB300_last_error() set. */
 int LowdinGB300_mp2_direct(LibintInterface *lint, const double *dD, const double *dC, const double *eps,
