@@ -239,11 +239,17 @@ __device__ __forceinline__ void jk_digest(const R (&I)[QClass<LA, LB, LC, LD>::N
 // on loads (L1 hits half of the scattered density and norm reads), so more warps
 // pay until spills outweigh them: 387-function chain, (ps|ss) 5.5 ms at 4
 // blocks, 4.6 at 5, 5.3 at 6; (ss|ss) 2.2 -> 1.85 at 8; (ps|ps) 3.8 -> 3.6 and
-// (pp|ss) 2.1 -> 1.6 at 4.
+// (pp|ss) 2.1 -> 1.6 at 4.  FP64 and FP32: where one block is enough, the compiler
+// takes 1.6 to 2.5 times the registers that it did without a number.  FP64 alone
+// (the allocation-free entry), one block -> these: 150-function chain 2.50 -> 2.35
+// ms, 4 waters 0.87 -> 0.82, 387-function chain 39.9 -> 38.4; with more blocks
+// ((ss|ss) 8, (ps|ss) 6, (ps|ps) 5, (pp|ps) 3) 2.31, 0.81 and 37.9, but contracted
+// waters 2.5 -> 2.7.  FP32 (bra rows off), a mixed batch of 32 chains 38.4 -> 35.9.
 template <typename R, int LA, int LB, int LC, int LD>
 constexpr int jk_min_blocks() {
-  if (!std::is_same<R, dd32>::value) return 1;
   constexpr int N = QClass<LA, LB, LC, LD>::NINT;
+  if (std::is_same<R, double>::value) return N == 1 ? 6 : N <= 3 ? 4 : N <= 9 ? 3 : N <= 27 ? 2 : 1;
+  if (std::is_same<R, float>::value) return N == 1 ? 10 : N <= 9 ? 8 : N <= 27 ? 5 : N <= 81 ? 3 : 1;
   return N == 1 ? 8 : N <= 3 ? 5 : N <= 9 ? 4 : 1;
 }
 template <typename R, int LA, int LB, int LC, int LD>
@@ -385,7 +391,10 @@ __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) jk_ta
         if (TL.tier == Tier::upper ? w < tb : !(w < tb)) active = false;
       }
     } else if (T.screen) {
-      const double b = T.pairs[bi].Q * T.pairs[ki].Q * dnorm6(T.Dn, T.nsh, bra.sa, bra.sb, ket.sa, ket.sb);
+      double qk;
+      if constexpr (F64) qk = ket.Q;
+      else qk = T.pairs[ki].Q;
+      const double b = T.pairs[bi].Q * qk * dnorm6(T.Dn, T.nsh, bra.sa, bra.sb, ket.sa, ket.sb);
       if (abs_below(b, TL.eps)) active = false;
     }
     const unsigned live = __ballot_sync(0xffffffffu, active && part == 0);
