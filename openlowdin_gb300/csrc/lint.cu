@@ -330,11 +330,6 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
   // JA (from D_B) accumulates into ba.G / ba.G32, JB (from D_A) into bb.G / bb.G32
   double *JA = want_a ? ba.G : nullptr, *JB = want_b ? bb.G : nullptr;
   if (!A->ensure_all() || !B->ensure_all()) return false;
-  double pa[kNumPairClasses], pb[kNumPairClasses];
-  for (int c = 0; c < kNumPairClasses; ++c) {
-    pa[c] = A->all.prims(c);
-    pb[c] = B->all.prims(c);
-  }
   for (int cb = 0; cb < kNumPairClasses; ++cb)
     for (int ck = 0; ck < kNumPairClasses; ++ck) {
       if (!A->all.count(cb) || !B->all.count(ck)) continue;
@@ -380,7 +375,7 @@ bool add_cp_tasks(TaskSet<CPTask> &ts, LibintInterface *A, LibintInterface *B, c
       t.nbra = X->all.count(cx);
       t.ket0 = Y->all.start[cy];
       t.nket = Y->all.count(cy);
-      t.mean_prims = t.most_prims = (float)(pa[cb] * pb[ck]);
+      t.mean_prims = t.most_prims = (float)(A->all.prims[cb] * B->all.prims[ck]);
       t.nA = X->nbasis;
       t.nB = Y->nbasis;
       ts.add(cx, cy, t);
@@ -506,7 +501,7 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
         q.ket0 = A->sig.start[ck];
         q.nket = A->sig.count(ck);
         q.triangle = cb == ck;
-        q.mean_prims = A->sig.prims(cb) * A->sig.prims(ck);
+        q.mean_prims = A->sig.prims[cb] * A->sig.prims[ck];
         add(cb, ck);
       }
   } else {
@@ -527,7 +522,7 @@ bool first_quarter(LibintInterface *A, LibintInterface *B, const double *hD, con
         q.ket0 = B->all.start[ck];
         q.nket = B->all.count(ck);
         q.triangle = 0;
-        q.mean_prims = A->all.prims(cb) * B->all.prims(ck);
+        q.mean_prims = A->all.prims[cb] * B->all.prims[ck];
         add(cb, ck);
       }
   }
@@ -596,7 +591,7 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
         P.ket0 = A->sig.start[ck];
         P.nket = A->sig.count(ck);
         P.triangle = cb == ck;
-        P.mean_prims = A->sig.prims(cb) * A->sig.prims(ck);
+        P.mean_prims = A->sig.prims[cb] * A->sig.prims[ck];
         add(cb, ck);
       }
     if (!run_jobs(jobs, s)) return false;
@@ -622,7 +617,7 @@ bool g12_build(LibintInterface *A, LibintInterface *B, const double *dD, double 
       P.nbra = A->all.count(cb);
       P.ket0 = B->all.start[ck];
       P.nket = B->all.count(ck);
-      P.mean_prims = A->all.prims(cb) * B->all.prims(ck);
+      P.mean_prims = A->all.prims[cb] * B->all.prims[ck];
       add(cb, ck);
     }
   if (!run_jobs(jobs, s)) return false;

@@ -85,16 +85,21 @@ struct PairList {
     soa32 = nullptr;
   }
   int count(int pc) const { return start[pc + 1] - start[pc]; }
-  // mean primitive pairs of a class
-  double prims(int pc) const {
-    double n = 0;
-    for (int i = start[pc]; i < start[pc + 1]; ++i) n += h[i].nprim;
-    return count(pc) ? n / count(pc) : 1.0;
-  }
-  double most_prims(int pc) const {
-    int n = 1;
-    for (int i = start[pc]; i < start[pc + 1]; ++i) n = std::max(n, h[i].nprim);
-    return n;
+  // of the list as binned: mean and largest number of primitive pairs of a
+  // class, largest Schwarz factor (every build asks for them)
+  double prims[kNumPairClasses], most_prims[kNumPairClasses], qmax = 0;
+  void summarise() {
+    qmax = 0;
+    for (int c = 0; c < kNumPairClasses; ++c) {
+      double n = 0, most = 1;
+      for (int i = start[c]; i < start[c + 1]; ++i) {
+        n += h[i].nprim;
+        most = std::max(most, (double)h[i].nprim);
+        qmax = std::max(qmax, h[i].Q);
+      }
+      prims[c] = count(c) ? n / count(c) : 1.0;
+      most_prims[c] = most;
+    }
   }
   // uploads the FP64 records (all that the Schwarz factors need)
   bool upload64() {
@@ -554,6 +559,7 @@ struct LibintInterface {
       L.start[pair_class(r.la, r.lb) + 1]++;
     }
     for (int c = 0; c < kNumPairClasses; ++c) L.start[c + 1] += L.start[c];
+    L.summarise();
   }
 
   bool compute_schwarz(PairList &L) {
@@ -707,16 +713,9 @@ struct LibintInterface {
     if (bf.Dd && !sig.upload_dd()) return false;
     // the double-float tier: screened species whose scaled density (D times two
     // norms) keeps clear of the ends of the FP32 exponent range
-    double qmax = 0;   // largest Schwarz factor of the species
-    for (const PairRec &r : sig.h) qmax = std::max(qmax, r.Q);
     const bool in_range =
         std::all_of(norma.begin(), norma.end(), [](double x) { return std::fabs(x) > 1e-8 && std::fabs(x) < 1e8; });
-    const float tier = is_electron && in_range ? (float)(qmax * qmax) * kTierBound : 0.f;
-    double cprims[kNumPairClasses], cmost[kNumPairClasses];
-    for (int c = 0; c < kNumPairClasses; ++c) {
-      cprims[c] = sig.prims(c);
-      cmost[c] = sig.most_prims(c);
-    }
+    const float tier = is_electron && in_range ? (float)(sig.qmax * sig.qmax) * kTierBound : 0.f;
     for (int cb = 0; cb < kNumPairClasses; ++cb)
       for (int ck = 0; ck <= cb; ++ck) {
         if (!sig.count(cb) || !sig.count(ck)) continue;
@@ -743,8 +742,8 @@ struct LibintInterface {
         t.nbra = sig.count(cb);
         t.ket0 = sig.start[ck];
         t.nket = sig.count(ck);
-        t.mean_prims = (float)(cprims[cb] * cprims[ck]);
-        t.most_prims = (float)(cmost[cb] * cmost[ck]);
+        t.mean_prims = (float)(sig.prims[cb] * sig.prims[ck]);
+        t.most_prims = (float)(sig.most_prims[cb] * sig.most_prims[ck]);
         t.n = nbasis;
         t.nsh = nshell();
         t.triangle = cb == ck;

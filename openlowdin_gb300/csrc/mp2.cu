@@ -63,8 +63,6 @@ void mp2_columns(const PairList &P, long long colB, MP2Columns &mc) {
 // integrals of every (mu nu) pair of PA with the column pairs [k0, k1) of PB
 bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, int k1, cudaStream_t s) {
   std::vector<LaunchJob> jobs;
-  double pa[kNumPairClasses];
-  for (int c = 0; c < kNumPairClasses; ++c) pa[c] = PA.prims(c);
   for (int ck = 0; ck < kNumPairClasses; ++ck) {
     const int ka = std::max(k0, PB.start[ck]), kb = std::min(k1, PB.start[ck + 1]);
     for (int c0 = ka; c0 < kb; c0 += 65535 * kWarpsPerBlock)   // grid y limit
@@ -75,7 +73,7 @@ bool mp2_batch_ints(const PairList &PA, const PairList &PB, MXParams q, int k0, 
         p.nbra = std::min(kb - c0, 65535 * kWarpsPerBlock);
         p.ket0 = PA.start[cb];
         p.nket = PA.count(cb);
-        p.mean_prims = pa[cb] * PB.prims(ck);
+        p.mean_prims = PA.prims[cb] * PB.prims[ck];
         jobs.push_back({launch_cost(cb, ck, (double)p.nbra * p.nket / 128), false,
                         [=](Queue &z) { return launch_mp2x(ck, cb, p, z); }});
       }
