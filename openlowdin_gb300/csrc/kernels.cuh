@@ -269,13 +269,14 @@ struct CPTask {
 // 18.4 ms (18.1 without the cap, 21.6 with one of 2^-12).
 enum class Tier { all, upper, lower };
 constexpr float kTierBound = 1.f / 4096, kTierCap = 1.f / 64;
-// Mixed builds, whose quartets below the split are evaluated in FP32 (error some
-// 2^-22 of a bound up to the split), take the tier up to 1/16 of the largest
-// bound, where its error stays below that of the FP32 quartets: up to 2^18
-// splits, and the tier of FP64 builds in any case.  A system held in FP64 for
-// its check keeps the tier of FP64 builds.  724-function chain, a later
-// iteration's density change, split 1e-5: 40.1 -> 34.3 ms.
-constexpr float kMixedTier = 256.f, kMixedCap = 0x1p18f;
+// Mixed builds, whose quartets below the split are evaluated in FP32, take the
+// tier up to 1/16 of the largest bound, where its error stays below theirs: up
+// to 2^20 splits (2^-21.3 splits at worst; 2^-24 of a bound up to the split,
+// amplified alike, is 2^-19.3), and the tier of FP64 builds in any case.  A system
+// held in FP64 for its check keeps the tier of FP64 builds.  Split 1e-5: 724-function
+// chain, a later iteration's density change, 40.1 -> 34.3 ms; four contracted
+// waters, whose tight cores it keeps out of FP64, 2.8 ms (3.1 with 2^18).
+constexpr float kMixedTier = 256.f, kMixedCap = 0x1p20f;
 // candidate quartets of a class below which one FP64 launch is shorter than two
 // launches (one water, 120 to 14,000 a class: 116 us in one, 163 us in two; four
 // waters with d: 1.09 ms with the line at 2e5, 1.00 at 5e4, 1.02 at 2e4)
