@@ -28,7 +28,7 @@ void set_error(const char *fmt, ...) {
 
 bool run_jobs(std::vector<LaunchJob> &jobs, cudaStream_t s) {
   std::stable_sort(jobs.begin(), jobs.end(), [](const LaunchJob &a, const LaunchJob &b) {
-    return a.in_order != b.in_order ? b.in_order : !a.in_order && a.cost > b.cost;
+    return a.in_order != b.in_order ? a.in_order : !a.in_order && a.cost > b.cost;
   });
   Queue q{s, true};
   q.sizing = true;
@@ -37,12 +37,10 @@ bool run_jobs(std::vector<LaunchJob> &jobs, cudaStream_t s) {
   if (q.need) CK(cudaMallocAsync((void **)&q.scratch, q.need * sizeof(double), s));
   q.need = 0;
   cudaError_t err = cudaSuccess;
-  bool ordered = false;
   for (const LaunchJob &j : jobs) {
-    if (ordered) q.beside = false;
+    if (j.in_order) q.beside = false;
     err = j.launch(q);
     if (err != cudaSuccess) break;
-    ordered = j.in_order;
   }
   if (q.scratch) {
     const cudaError_t e = cudaFreeAsync(q.scratch, s);

@@ -243,9 +243,9 @@ struct LaunchJob {
   bool in_order;
   std::function<cudaError_t(Queue &)> launch;
 };
-// Runs the jobs on s beside one another (launch_beside), costliest first, then
-// those in order one after another; what is queued on s afterwards is behind
-// them all.  Eight are in flight at most.  One after another -> so: one water (34
+// Runs the jobs in order one after another on s, then the others beside the last
+// of them and one another (launch_beside), costliest first; what is queued on s
+// afterwards is behind them all.  Eight are in flight at most.  One after another -> so: one water (34
 // functions, 6 launches of 6-170 blocks) 184 -> 114 us; two waters in a contracted
 // basis (21 launches) 1.78 -> 0.59 ms; four waters with d 1.71 -> 0.95 ms; a
 // 387-function chain, whose launches fill the GPU by themselves, 18.1 -> 18.0 ms.
