@@ -142,7 +142,9 @@ __device__ void ovl1d_dev(int li, int lj, double PA, double PB, double o2p, doub
     }
 }
 
-// S and T of every pair, and (WITHV) V of the pairs with an f shell
+// S and T of every pair, or (WITHV) V of the pairs with an f shell: apart, so that
+// the chains of the two run beside one another (three waters with an f shell on
+// O: 1.04 ms in one kernel, 0.81 so; one thread per pair for everything took 0.94)
 template <bool WITHV>
 __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
   if (beside_block()) return;
@@ -269,10 +271,17 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyParams P) {
 
 cudaError_t launch_one_body(const OneBodyParams &p, Queue &q) {
   const int npair = p.nsh * (p.nsh + 1) / 2;
-  const bool heavy = p.V && p.ncharge > 0 && p.lstart[kPotMaxL + 1] < p.nsh;
-  if (npair <= 0 || (!heavy && !p.S && !p.T)) return cudaSuccess;
+  if (npair <= 0 || (!p.S && !p.T)) return cudaSuccess;
   count_launches(q.sizing ? 0 : 1);
-  return launch_beside(q, heavy ? &one_body_kernel<true> : &one_body_kernel<false>, (npair + 127) / 128, 128, 0, p);
+  return launch_beside(q, &one_body_kernel<false>, (npair + 127) / 128, 128, 0, p);
+}
+
+cudaError_t launch_potential_f(OneBodyParams p, Queue &q) {
+  const int npair = p.nsh * (p.nsh + 1) / 2;
+  if (npair <= 0 || !p.V || p.ncharge <= 0 || p.lstart[kPotMaxL + 1] >= p.nsh) return cudaSuccess;
+  count_launches(q.sizing ? 0 : 1);
+  p.S = p.T = nullptr;
+  return launch_beside(q, &one_body_kernel<true>, (npair + 127) / 128, 128, 0, p);
 }
 
 cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, Queue &q) {

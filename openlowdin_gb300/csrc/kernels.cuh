@@ -648,8 +648,10 @@ struct OneBodyParams {
   double *S, *T, *V;          // n x n outputs (any may be null)
   BoysTables boys;
 };
-// S and T, and V of the pairs with an f shell
+// S and T of every pair
 cudaError_t launch_one_body(const OneBodyParams &p, Queue &q);
+// V of the pairs with an f shell
+cudaError_t launch_potential_f(OneBodyParams p, Queue &q);
 // V of the pairs with a later shell of angular momentum la and an earlier one of
 // lb (s, p and d), and the candidates of such a launch (0 for other classes)
 cudaError_t launch_potential(int la, int lb, const OneBodyParams &p, Queue &q);

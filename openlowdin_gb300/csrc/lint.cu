@@ -952,7 +952,8 @@ int LowdinGB300_one_body_device(LibintInterface *lint, int ncharge, const double
     if (cudaMemsetAsync(dV, 0, sizeof(double) * lint->nbasis * lint->nbasis, s) != cudaSuccess) return -1;
   }
   std::vector<LaunchJob> jobs;
-  // one thread per pair, so the longest: first, that the others run beside it
+  // one thread per pair, so the longest: first, that the others run beside them
+  jobs.push_back({HUGE_VAL, false, [=](Queue &q) { return launch_potential_f(p, q); }});
   jobs.push_back({HUGE_VAL, false, [=](Queue &q) { return launch_one_body(p, q); }});
   for (int la = 0; p.V && p.ncharge > 0 && la <= kMaxL; ++la)
     for (int lb = 0; lb <= kMaxL; ++lb)
