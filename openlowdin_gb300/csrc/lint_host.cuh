@@ -391,7 +391,7 @@ struct LibintInterface {
   DevShell *d_shells = nullptr;
   double *d_alpha = nullptr, *d_cn = nullptr;
   int *d_first = nullptr;
-  int *d_order = nullptr;      // shells by angular momentum, and where each begins
+  int *d_order = nullptr;      // shells by angular momentum (behind d_first), and where each begins
   int lstart[kMaxL + 2] = {0};
   DevBuf<double> dZR;          // point charges and positions of the last one-body call
   DevBuf<double> dGem;         // geminal parameters of the last G12 call {count, exponents, coefficients}
@@ -423,8 +423,7 @@ struct LibintInterface {
     all.release();
     if (d_norma) cudaFree(d_norma);
     if (d_shell_of) cudaFree(d_shell_of);
-    for (void *q : {(void *)d_shells, (void *)d_alpha, (void *)d_cn, (void *)d_first,
-                    (void *)d_order})
+    for (void *q : {(void *)d_shells, (void *)d_alpha, (void *)d_cn, (void *)d_first})
       if (q) cudaFree(q);
     d_norma = nullptr;
     d_shell_of = nullptr;
@@ -488,15 +487,16 @@ struct LibintInterface {
       al.insert(al.end(), h.alpha.begin(), h.alpha.end());
       cn.insert(cn.end(), h.cn.begin(), h.cn.end());
     }
-    if (!dev_upload(d_shells, ds) || !dev_upload(d_alpha, al) || !dev_upload(d_cn, cn) ||
-        !dev_upload(d_first, first))
-      return false;
-    std::vector<int> order(nshell());
-    for (int k = 0; k < nshell(); ++k) order[k] = k;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return shells[x].l < shells[y].l; });
+    // first functions, and behind them the shells by angular momentum
+    std::vector<int> fo(first.begin(), first.end());
+    const size_t nfirst = fo.size();
+    for (int k = 0; k < nshell(); ++k) fo.push_back(k);
+    std::stable_sort(fo.begin() + nfirst, fo.end(), [&](int x, int y) { return shells[x].l < shells[y].l; });
     for (int l = 0; l <= kMaxL + 1; ++l)
       lstart[l] = (int)std::count_if(shells.begin(), shells.end(), [&](const HostShell &h) { return h.l < l; });
-    if (!dev_upload(d_order, order)) return false;
+    if (!dev_upload(d_shells, ds) || !dev_upload(d_alpha, al) || !dev_upload(d_cn, cn) || !dev_upload(d_first, fo))
+      return false;
+    d_order = d_first + nfirst;
     have_sig = have_all = false;
     jk_ready = false;
     dirty = false;
