@@ -24,9 +24,10 @@ Sections of the JSON line:
                        the reference program's calling pattern, FP64), the
                        MP2 of MP2 requests through LowdinGB300_mp2_direct with
                        host-resident orbitals copied in.
-  roofline          -- the plain J/K kernels (one plain build of the stream's
-                       largest molecule, CUDA events) against the FP64 FMA
-                       peak measured in the run; the FP32 row kernels beside.
+  roofline          -- the FP64 J/K kernels alone (one allocation-free build,
+                       CUDA events) against the FP64 FMA peak measured in the
+                       run; beside them the plain build of the stream's largest
+                       molecule in its two tiers, and the FP32 row kernels.
   cpu_baseline      -- the oracle port (C/OpenMP, all host threads) on every
                        request of the stream: setup + one SCF iteration,
                        scaled by the request's plain iteration count.
@@ -578,12 +579,53 @@ def apmo_batch_section(args, dev):
 
 
 # --------------------------------------------------------------- roofline --
+def fp64_alone(target=480):
+    """The FP64 J/K kernels alone: the allocation-free build, which has no other
+    tier and holds up to 512 functions, of a chain at its core-guess density."""
+    import torch
+    from openlowdin_gb300 import flops as FL, lint, systems as S
+    from openlowdin_gb300.batch_scf import BatchSCF
+    sysd = S.chain_for_basis(10_000, target)
+    sp = sysd["species"][0]
+    s = BatchSCF([sysd])
+    g = list(s.groups.values())[0]
+    D = s._density(g, g.H)[0].contiguous()
+    s.close()
+    h = lint.Libint2Interface(sp, 1)
+    n, st = h.nbasis, torch.cuda.current_stream().cuda_stream
+    D = D[:n, :n].contiguous()
+    G = torch.empty_like(D)
+    factor = sp["kappa"] / sp["eta"]
+    h.twobody_device(D.data_ptr(), G.data_ptr(), factor, stream=st)
+    q = h.last_class_quartets()
+
+    def build():
+        if lint.lib().LowdinGB300_twobody_device_noalloc(h.h, D.data_ptr(), G.data_ptr(), factor, 0, 0.0, st) != 0:
+            raise RuntimeError(lint.last_error())
+
+    build()
+    build()
+    a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    reps = 3
+    a.record()
+    for _ in range(reps):
+        build()
+    b.record()
+    torch.cuda.synchronize()
+    ms = a.elapsed_time(b) / reps
+    h.close()
+    fl = FL.class_table_flops(q, "jk")
+    return {"system": f"chain molecule, {n} functions", "functions": n, "ms_per_build": ms, "quartets": int(q.sum()),
+            "flop_per_build": fl, "achieved_tflops": fl / (ms * 1e-3) / 1e12}
+
+
 def roofline_section(sysd):
-    """Plain J/K kernels (FP64 and double-float tiers): one plain Fock build of
-    `sysd` at its core-guess density (CUDA events on the launching stream, 3 builds), FLOPs from the
-    frozen per-class model over the quartets the build evaluated, against the
-    FP64 FMA throughput measured in this run.  Beside it the FP32 row kernels:
-    the same build with every quartet in FP32 (split above every bound)."""
+    """J/K kernels, each tier against its own peak where it has one: the FP64 kernels
+    alone against the FP64 FMA throughput measured in this run, the FP32 row kernels
+    (every quartet of `sysd` in FP32, split above every bound) against FP32's, and the
+    plain build of `sysd` in its two tiers, which mixes the pipes and has no
+    single peak.  CUDA events on the launching stream, 3 builds at the core-guess
+    density; FLOPs from the frozen per-class model over the quartets evaluated."""
     import torch
     from openlowdin_gb300 import flops as FL, lint, systems as S
     from openlowdin_gb300.batch_scf import BatchSCF
@@ -592,7 +634,7 @@ def roofline_section(sysd):
     g.Pin.copy_(s._density(g, g.H))
     st = torch.cuda.current_stream().cuda_stream
     out = {}
-    for name, prec, split in (("fp64", 0, 0.0), ("fp32_rows", 1, 1e30)):
+    for name, prec, split in (("plain", 0, 0.0), ("fp32_rows", 1, 1e30)):
         s.batch.fock(prec, split, st)
         s.batch.fock(prec, split, st)
         torch.cuda.synchronize()
@@ -610,33 +652,38 @@ def roofline_section(sysd):
         out[name] = {"ms_per_build": ms, "quartets": int(q.sum()), "flop_per_build": fl,
                      "achieved_tflops": fl / (ms * 1e-3) / 1e12}
     s.close()
+    f64 = fp64_alone()
     # the FMA-chain peaks, with the clocks seen while they ran
     clk = ClockSampler(torch.cuda.current_device())
     clk.start()
     peak64 = max(lint.measure_fma_tflops(True) for _ in range(3))
     peak32 = max(lint.measure_fma_tflops(False) for _ in range(3))
     peak_clocks = clk.stop()
-    f64, f32 = out["fp64"], out["fp32_rows"]
+    plain, f32 = out["plain"], out["fp32_rows"]
     traffic = None
     prof = os.path.join(ROOT, "profiles", "roofline_traffic.json")
     if os.path.exists(prof):
         try:
             with open(prof) as f:
                 tr = json.load(f)
-            traffic = tr.get("bytes_per_build_at", {}).get(str(S.nbasis(sysd["species"][0])))
+            traffic = tr.get("fp64_alone_bytes_per_build_at", {}).get(str(f64["functions"]))
         except (OSError, ValueError):
             traffic = None
     return {"bound": "fp64", "achieved": f64["achieved_tflops"], "peak": peak64, "unit": "TFLOP/s",
             "frac": f64["achieved_tflops"] / peak64 if peak64 > 0 else None, "traffic": traffic,
-            "kernel": "jk_tasks_kernel<double> for the quartets above 2^-12 of the largest bound and "
-                      "jk_tasks_kernel<dd32> (double-float, on the FP32 pipe) below it: every J/K class launch of "
-                      "one plain Fock build; the fraction of the FP64 peak can therefore exceed 1",
-            "system": f"chain molecule, {S.nbasis(sysd['species'][0])} functions (largest request of the stream)",
-            "ms_per_build": f64["ms_per_build"], "quartets": f64["quartets"], "flop_per_build": f64["flop_per_build"],
+            "kernel": "jk_tasks_kernel<double>: every J/K class launch of one Fock build of the allocation-free entry",
+            "system": f64["system"], "ms_per_build": f64["ms_per_build"], "quartets": f64["quartets"],
+            "flop_per_build": f64["flop_per_build"],
             "peak_source": "FP64 FMA throughput measured on this GPU in this run (LowdinGB300_measure_fma_tflops: "
                            "8 independent FMA chains per thread, 8 CTAs of 256 threads per SM, best of 3; "
                            "MEASURED_PEAKS.json has no FP64 entry)",
             "peak_clocks": peak_clocks,
+            "two_tiers": {"kernel": "jk_tasks_kernel<double> above the tier bound, jk_tasks_kernel<dd32> (double-float, "
+                                    "on the FP32 pipe) below it: one plain Fock build",
+                          "system": f"chain molecule, {S.nbasis(sysd['species'][0])} functions (largest request of "
+                                    "the stream)",
+                          "ms_per_build": plain["ms_per_build"], "quartets": plain["quartets"],
+                          "flop_per_build": plain["flop_per_build"], "fp64_equivalent_tflops": plain["achieved_tflops"]},
             "fp32_rows": {"kernel": "jk32_row_kernel (all quartets in FP32)", "ms_per_build": f32["ms_per_build"],
                           "achieved": f32["achieved_tflops"], "peak": peak32,
                           "frac": f32["achieved_tflops"] / peak32 if peak32 > 0 else None}}
