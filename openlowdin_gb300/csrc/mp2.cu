@@ -55,7 +55,9 @@ void mp2_columns(const PairList &P, long long colB, MP2Columns &mc) {
   for (int k = 0; k < npairs;) {
     mc.bfirst.push_back(k);
     const int c0 = mc.colbase[k];
-    while (k < npairs && mc.colbase[k] - c0 + ncart(P.h[k].la) * ncart(P.h[k].lb) <= colB) ++k;
+    // at least one pair, also when its columns (100 of two f shells) are more than colB
+    do ++k;
+    while (k < npairs && mc.colbase[k] - c0 + ncart(P.h[k].la) * ncart(P.h[k].lb) <= colB);
   }
   mc.bfirst.push_back(npairs);
 }
