@@ -181,9 +181,9 @@ int LowdinGB300_set_precision(LibintInterface *lint, int precision, double split
          in the reference), not the 52 bits of an element fed by small quartets
          alone.  LowdinGB300_twobody_device_noalloc uses FP64 alone, as do basis
          sets with norms of the contractions beyond 1e-8 .. 1e8;
-     1 = mixed: quartets with B below `split` run in FP32, those above as in 0
-         with the ends at 2^-4 of Q_max^2 max|D| and at the larger of 2^-6 and
-         2^20 split (their error stays below that of the FP32 quartets).
+     1 = mixed: quartets with B below `split` run in FP32, those above as in 0,
+         for electrons in double-float also up to 2^-4 of Q_max^2 max|D| while B is
+         below 2^20 split (their error stays below that of the FP32 quartets).
    Work is queued on `stream` (a cudaStream_t, 0 = legacy default); returns 0
    on success, -1 on error (see LowdinGB300_last_error). */
 int LowdinGB300_twobody_device(LibintInterface *lint, const double *dD, double *dG, double factor, int precision,

@@ -299,9 +299,8 @@ __global__ void __launch_bounds__(128, jk_min_blocks<R, LA, LB, LC, LD>()) jk_ta
   // largest norm of all), w >= tb in the FP64 launch, w < tb in the
   // double-float one
   const float dmax = T.Dnmax32 ? __ldg(T.Dnmax32) : -1.f;
-  const float tb = TL.tier == Tier::all ? 0.f
-                   : TL.mixed && !all64 ? tier_bound(kMixedTier * T.tier, dmax, TL.tier_cap)
-                                        : tier_bound(T.tier, dmax, kTierCap);
+  float tb = TL.tier == Tier::all ? 0.f : tier_bound(T.tier, dmax, kTierCap);
+  if (TL.tier != Tier::all && TL.mixed && !all64) tb = fmaxf(tb, tier_bound(kMixedTier * T.tier, dmax, TL.tier_cap));
   if (TL.tier == Tier::lower && (tb == 0.f || (T.screen && !(lo < tb)))) return;
   // Pairs are sorted by decreasing Schwarz factor inside a class and Dnmax32
   // bounds the six norms, so the first bra and the first ket of a range bound

@@ -307,7 +307,7 @@ inline void set_fp32_copies(TaskLaunch &tl) {
   tl.eps32 = (float)tl.eps;
   tl.split32 = (float)tl.split;
   tl.cut32 = (float)tl.cut;
-  tl.tier_cap = kMixedCap * tl.split32 > kTierCap ? kMixedCap * tl.split32 : kTierCap;
+  tl.tier_cap = kMixedCap * tl.split32;
 }
 
 // Kernel entry types of the class-templated launch tables (class_tables.cuh);

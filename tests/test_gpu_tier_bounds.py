@@ -90,6 +90,24 @@ def test_tier_ends(L, which, size, split):
     c.h.close()
 
 
+@pytest.mark.parametrize("split", [0.0, 1e-12])
+def test_tier_of_fp64_builds(L, oracle, split):
+    # Coulomb alone: an element is one integral, not above its quartet's bound, and in
+    # FP64 from 2^-12 of the largest bound on, also in mixed builds of a small split
+    pytest.importorskip("torch")
+    sp = _species("240")
+    c = _Case(L, sp)
+    tier = float(np.max(oracle.schwarz(oracle.Basis.from_shells(sp["shells"])))) ** 2 / 4096
+    seen = 0
+    for k in _functions(c.n):
+        G, R = c.one(k, 1.0, 0.0, precision=int(split > 0), split=split)
+        m = (np.abs(R) > 1.01 * tier) & (np.abs(R) < 2.0 ** -6)
+        seen += int(m.sum())
+        assert np.all(np.abs(G - R)[m] <= 2.0 ** -49 * np.abs(R[m]))
+    assert seen > 100
+    c.h.close()
+
+
 def test_mixed_tier_stays_below_the_fp32_quartets(L):
     # split 1e-5: an FP32 integral is within some 2^-17 of its bound
     pytest.importorskip("torch")
