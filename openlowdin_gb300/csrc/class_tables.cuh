@@ -74,13 +74,14 @@ static_assert(kNumPairClasses == 10, "launch-table rows list every pair class");
   const JKFn kJK32_##B[kNumPairClasses] = LGB_ROW(jk_entry, float, B);  \
   const JKFn kJKR_##B[kNumPairClasses] = LGB_ROW(jkr_entry, B);
 
-// Classes with double-float J/K kernels: those where they beat FP64.  ns per
+// Classes with double-float J/K kernels: those where they clearly beat FP64.  ns per
 // quartet on the whole GPU, FP64 / double-float (12 waters with d shells, 480
 // functions): (ss|ss) .121/.064, (ps|ss) .253/.109, (ps|ps) .429/.216, (pp|ss)
 // .479/.193, (pp|ps) .954/.580, (ds|ss) .400/.177, (ds|ps) .740/.500, (dp|ss)
 // .847/.567.  Above 27 integrals the code (some 27,000 instructions for (pp|pp))
-// outgrows the instruction cache and little is left: (pp|pp) 2.64/2.38, (ds|pp)
-// 1.86/1.52, (dp|ps) 1.78/1.57, (ds|ds) 1.87/1.78, (dd|ss) 1.85/2.05.
+// outgrows the instruction cache and 5 to 18 % are left, at two launches a class
+// instead of one and less of a quartet's precision: (pp|pp) 2.64/2.38, (ds|pp)
+// 1.86/1.52, (dp|ps) 1.78/1.57, (ds|ds) 1.87/1.78; (dd|ss) loses, 1.85/2.05.
 template <int B, int K>
 constexpr JKFn jkd_entry() {
   if constexpr (templated_class<B, K, kTemplatedMaxL4>() && B >= K &&

@@ -4,8 +4,9 @@
 //
 // In a cooperative kernel every warp is a worker with its own class-sized
 // shared work arrays (up to 4 warps per CTA, a persistent grid); a warp takes
-// work units -- a bra pair and 8 ket pairs of a task's 4 x 32 tile, or one
-// quartet -- and evaluates their quartets one after another, its 32 lanes
+// work units -- a bra pair, one to eight ket pairs (coop_tile) and a slice of
+// their primitive quartets, or one quartet -- and evaluates their quartets one
+// after another, its 32 lanes
 // together on each (eri_coop), then digests the quartet's integrals with the
 // lanes split over the output elements.  They compute in
 // FP64 (also when a mixed launch asks for the FP32 half: the split decides

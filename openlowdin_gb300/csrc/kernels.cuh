@@ -263,9 +263,10 @@ struct CPTask {
 // functions, 8 waters, 4 waters with d).  Species without screening keep FP64:
 // each of their elements has the relative precision of its own quartets.
 // Error of the matrix against an 80-bit evaluation of the same quartets (2-norm
-// over 2-norm), FP64 alone -> two tiers: 4 waters (136 functions) 3.0e-15 ->
-// 3.0e-15, 176-function chain 6.0e-15 -> 4.8e-15, 3 waters with d 3.9e-15 ->
-// 3.5e-15.  387-function chain (5 % of the quartets above the bound): 41.7 ->
+// over 2-norm), FP64 alone, one block a tile -> as it is: 4 waters (136 functions)
+// 3.0e-15 -> 2.8e-15, 176-function chain 6.0e-15 -> 4.9e-15, 3 waters with d
+// 3.9e-15 -> 3.5e-15, 2 contracted waters, whose quartets the tier leaves in FP64
+// but slices add in shares, 1.5e-15 -> 2.0e-15.  387-function chain (5 % of the quartets above the bound): 41.7 ->
 // 18.4 ms (18.1 without the cap, 21.6 with one of 2^-12).
 enum class Tier { all, upper, lower };
 constexpr float kTierBound = 1.f / 4096, kTierCap = 1.f / 64;
@@ -328,9 +329,11 @@ using CPFn = void (*)(const CPTask *, TaskLaunch);
 struct ITParams;
 using ITFn = void (*)(ITParams);
 __host__ __device__ constexpr int pc_L(int pc) { return pc_la(pc) + pc_lb(pc); }
-// classes above this total angular momentum use the cooperative kernels: the
-// fully unrolled one-thread-per-quartet kernels of total 5 keep up to 1.4 KB of
-// a thread in local memory, those of (dp|dp) and (dd|pp) 10 KB
+// classes above this total angular momentum use the cooperative kernels.  The
+// fully unrolled one-thread-per-quartet kernels of total 5 spill (frames of 2.4 KB
+// for (dp|pp), 1.7 KB for (dp|ds)) and still win, on launches that fill the GPU
+// too: J/K of 12 waters with d (480 functions) 17.7 ms with the line at 4, 13.7
+// here; those of (dp|dp) and (dd|pp) would keep 10 KB of a thread in local memory
 constexpr int kTemplatedMaxL = 5;
 // the same for the kernels that have no gain from it: FP32 (heavier classes
 // are evaluated in FP64 in the FP32 half of a mixed launch too) and first quarter
