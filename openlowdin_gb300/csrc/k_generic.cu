@@ -518,10 +518,12 @@ cudaError_t coop_launch(F f, const CoopShape &c, Queue &q, Args... args) {
     return launch_beside(q, f, c.grid, c.block, c.smem, args..., scr);
   }
   double *scr = nullptr;
+  q.beside = false;
   const cudaError_t e = cudaMallocAsync((void **)&scr, c.scratch * sizeof(double), q.s);
   if (e != cudaSuccess) return e;
   const cudaError_t e1 = launch_beside(q, f, c.grid, c.block, c.smem, args..., scr);
   const cudaError_t e2 = cudaFreeAsync(scr, q.s);
+  q.beside = false;
   return e1 == cudaSuccess ? e2 : e1;
 }
 

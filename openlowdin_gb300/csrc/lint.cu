@@ -34,7 +34,11 @@ bool run_jobs(std::vector<LaunchJob> &jobs, cudaStream_t s) {
   q.sizing = true;
   for (const LaunchJob &j : jobs) CK(j.launch(q));
   q.sizing = false;
-  if (q.need) CK(cudaMallocAsync((void **)&q.scratch, q.need * sizeof(double), s));
+  // no room for all of it at once: each launch then takes its own in turn
+  if (q.need && cudaMallocAsync((void **)&q.scratch, q.need * sizeof(double), s) != cudaSuccess) {
+    cudaGetLastError();
+    q.scratch = nullptr;
+  }
   q.need = 0;
   cudaError_t err = cudaSuccess;
   for (const LaunchJob &j : jobs) {
