@@ -956,14 +956,24 @@ int LowdinGB300_one_body_device(LibintInterface *lint, int ncharge, const double
     if (cudaMemsetAsync(dV, 0, sizeof(double) * lint->nbasis * lint->nbasis, s) != cudaSuccess) return -1;
   }
   std::vector<LaunchJob> jobs;
-  // one thread per pair, so the longest: first, that the others run beside them
-  jobs.push_back({HUGE_VAL, false, [=](Queue &q) { return launch_potential_f(p, q); }});
-  jobs.push_back({HUGE_VAL, false, [=](Queue &q) { return launch_one_body(p, q); }});
   for (int la = 0; p.V && p.ncharge > 0 && la <= kMaxL; ++la)
     for (int lb = 0; lb <= kMaxL; ++lb)
       if (potential_pairs(la, lb, p) > 0)
         jobs.push_back({(double)potential_pairs(la, lb, p) * p.ncharge * ncart(la) * ncart(lb), false,
                         [=](Queue &q) { return launch_potential(la, lb, p, q); }});
+  // S, T and V of f pairs, one thread per pair, are the longest: first, that the
+  // others run beside them.  With d shells there are more launches than the eight
+  // in flight, and the ninth waits for the first: then behind the two shortest, the
+  // shortest before the other (8 contracted waters 886 us with S and T first, 671
+  // so; a chain of s and p, five launches, 209 with them first and 244 so)
+  auto costlier = [](const LaunchJob &x, const LaunchJob &y) { return x.cost > y.cost; };
+  std::sort(jobs.begin(), jobs.end(), costlier);
+  const size_t ahead = jobs.size() + 2 > 8 ? 2 : 0;
+  std::rotate(jobs.begin(), jobs.end() - ahead, jobs.end());
+  std::reverse(jobs.begin(), jobs.begin() + ahead);
+  jobs.insert(jobs.begin() + ahead, {{0, false, [=](Queue &q) { return launch_potential_f(p, q); }},
+                                     {0, false, [=](Queue &q) { return launch_one_body(p, q); }}});
+  for (LaunchJob &j : jobs) j.cost = 0;   // run_jobs keeps this order
   return run_jobs(jobs, s) ? 0 : -1;
 }
 
