@@ -468,7 +468,7 @@ class BatchSCF:
         # mixed: incremental build from dP = P - P_ref on top of the previous
         # matrices, a full build (FP64 couplings) on the first and every
         # rebuild_every-th iteration; two-particle quartets whose Schwarz x
-        # |dP| bound is below the split run in FP32, the rest in FP64, and
+        # |dP| bound is below the split run in FP32, the rest above it, and
         # incremental couplings run in FP32 (their size scales with |dP|).
         full = (not mixed) or (it - 1) % self.rebuild_every == 0
         # systems in FP64 (an FP64 check, or after a failed one): full builds

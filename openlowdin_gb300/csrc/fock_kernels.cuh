@@ -241,7 +241,7 @@ __device__ __forceinline__ void jk_digest(const R (&I)[QClass<LA, LB, LC, LD>::N
 // blocks, 4.6 at 5, 5.3 at 6; (ss|ss) 2.2 -> 1.85 at 8; (ps|ps) 3.8 -> 3.6 and
 // (pp|ss) 2.1 -> 1.6 at 4.  FP64 and FP32: where one block is enough, the compiler
 // takes 1.6 to 2.5 times the registers that it did without a number.  FP64 alone
-// (the allocation-free entry), one block -> these: 150-function chain 2.50 -> 2.35
+// (the allocation-free entry), one block -> these: 156-function chain 2.50 -> 2.35
 // ms, 4 waters 0.87 -> 0.82, 387-function chain 39.9 -> 38.4; with more blocks
 // ((ss|ss) 8, (ps|ss) 6, (ps|ps) 5, (pp|ps) 3) 2.31, 0.81 and 37.9, but contracted
 // waters 2.5 -> 2.7.  FP32 (bra rows off), a mixed batch of 32 chains 38.4 -> 35.9.

@@ -259,7 +259,7 @@ struct CPTask {
 // that it stays near the screening threshold of 2^-52 whatever the largest bound
 // is: the quartets that screening drops leave 2e-11 in the matrix, and the
 // error against the unscreened 64-bit matrix is the same with and without the
-// tier in each power of ten of the elements' size (chains of 150 and 387
+// tier in each power of ten of the elements' size (chains of 156 and 387
 // functions, 8 waters, 4 waters with d).  Species without screening keep FP64:
 // each of their elements has the relative precision of its own quartets.
 // Error of the matrix against an 80-bit evaluation of the same quartets (2-norm
