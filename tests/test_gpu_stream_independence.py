@@ -92,7 +92,8 @@ def test_build_does_not_wait_for_a_transform(L):
 
     transform()
     torch.cuda.synchronize()
-    a.hold()
+    for _ in range(4):
+        a.hold()
     t = threading.Thread(target=transform)
     t.start()
     time.sleep(0.1)      # its launches are queued, and it waits for the result
